@@ -2688,11 +2688,26 @@ int motion_download(Context* ctx, int8_t* res, float* err, float* lvert, int32_t
 // term that is switched off leaves 0.
 __global__ void row_codes_kernel(GNArgs a, int slot, int8_t* __restrict__ out,
                                  float* __restrict__ out_err) {
+  // The problem's constants (all but the sums) in shared memory, copied by the
+  // whole CTA, and the inverse of the evaluated pose by one warp: with one
+  // thread copying and inverting, that prologue was 50 of the kernel's 57 us at
+  // 637x479.  The rows themselves are two gathers per pixel, latency-bound.
   __shared__ GNState S;
-  if (threadIdx.x == 0) {
-    S = a.st[slot];
-    S.Tf = S.evalTf;
-    S.invTf = inverse(S.evalTf);
+  {
+    const int* src = reinterpret_cast<const int*>(&a.st[slot]);
+    int* dst = reinterpret_cast<int*>(&S);
+    for (int i = threadIdx.x; i < (int)(offsetof(GNState, sums) / 4); i += blockDim.x)
+      dst[i] = src[i];
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    const float e = reinterpret_cast<const float*>(&S.evalTf)[lane & 15];
+    const float ie = inverse_warp(e, lane);
+    if (lane < 16) {
+      reinterpret_cast<float*>(&S.Tf)[lane] = e;
+      reinterpret_cast<float*>(&S.invTf)[lane] = ie;
+    }
   }
   __syncthreads();
   const int w = a.pyr.w[0], h = a.pyr.h[0], n = w * h;
