@@ -185,7 +185,9 @@ int mf_retrack_camera(mf_context* ctx, uint32_t moving_labels);
 int mf_track_objects(mf_context* ctx, const int* ids, int n);
 /* Diagnostics of a GN problem (slot 0: camera, slot i: object i): iterations
  * per level (int[4]), last normal-equation sums per level (double[4][32]),
- * FP64 pose (double[16]); any pointer may be NULL. */
+ * FP64 pose (double[16]); any pointer may be NULL.  Of an object's sums the
+ * three outlier counts (29..31) cover the pixels that its GN evaluates, which
+ * leave out what cannot hold a valid row. */
 int mf_track_info(mf_context* ctx, int slot, int* iterations, double* sums, double* pose);
 /* One evaluation of the normal equations (the 32 reduceKernel sums,
  * tracking.cpp:1191-1352) of a problem at `level` and at `pose` (NULL: its
@@ -530,14 +532,10 @@ int mf_frame_stats(mf_context* ctx, long long* out, int n);
 int mf_profile(mf_context* ctx, int reps, double* out, int n);
 /* Batched mode replays the frame as a CUDA graph once captured (default 1). */
 int mf_set_graphs(mf_context* ctx, int enable);
-/* No counterpart in the reference.  Batched GN runs every iteration of a
- * pyramid level in one cooperative launch per level and stage, with a grid
- * barrier between iterations and an early end once every problem has stopped
- * (1), or one launch per iteration, each chained to the previous one by
- * programmatic dependent launch (0, the default: faster on B200, where the
- * frame graph already removes the launch overhead and the grid barrier costs
- * more than a launch boundary).  Both give the same poses bit for bit.
- * Applies to frames captured after the call. */
+/* No counterpart in the reference.  Kept for callers: it used to choose
+ * between one launch per GN iteration (0) and one per pyramid level (1).
+ * Batched GN is now one launch for all levels and iterations of a stage in
+ * either setting, with the same poses bit for bit. */
 int mf_set_gn_persistent(mf_context* ctx, int enable);
 /* No counterpart in the reference.  Batched frames with objects: the
  * background's allocation and integration (which need only the camera pose)

@@ -36,7 +36,7 @@ MF_HD uchar4 u4(float x, float y, float z, float w) {
 MF_HD float sq(float r) { return r * r; }
 
 struct F3 { float x, y, z; };
-struct F4 { float x, y, z, w; };
+struct alignas(16) F4 { float x, y, z, w; };  // matrix rows move as one 16-byte access
 struct I3 { int x, y, z; };
 struct M4 { F4 r[4]; };  // Matrix4: r[i] is row i (utils/math_utils.h:47-49)
 

@@ -23,6 +23,17 @@ namespace mf {
 // kind: 0 none, 1 Huber (k 1.345), 2 Tukey (b 4.6851), 3 Cauchy (k 2.3849)
 // (tracking.h:19-24, :343-345).
 MF_ROBUST_HD void robust(float e, int kind, float& w, float& loss) {
+  // Within the quadratic part the double loss is 0.5 e^2 exactly, rounded once:
+  // 0.5f * (e * e), unless e * e leaves the normal range (the double path then).
+  // 0x1.5851eap+0f is the largest float at most 1.345.
+  if (kind <= 1) {
+    const float q = e * e;
+    if ((kind == 0 || fabsf(e) <= 0x1.5851eap+0f) && ((q >= 1e-30f && q <= 1e38f) || e == 0.f)) {
+      w = 1.f;
+      loss = 0.5f * q;
+      return;
+    }
+  }
   const double r = e;
   double wd = 1.0, l;
   switch (kind) {

@@ -1,19 +1,18 @@
 // ICP + photometric Gauss-Newton tracking on the device.
 //
 // Reference: apps/kfusion/src/cpp/tracking/tracking.cpp (Tracking) and
-// apps/kfusion/src/cpp/preprocessing/*.  Per GN iteration one kernel evaluates
-// the ICP row and the photometric row of every pixel of the level for every
-// problem of the stage (the camera, or all moving objects at once), weights
-// them (IRLS), and reduces the 29 sums of the normal equations plus the three
-// outlier counts:
+// apps/kfusion/src/cpp/preprocessing/*.  The whole coarse-to-fine GN of a
+// stage (the camera, or all moving objects at once) is one launch: per
+// iteration its CTAs evaluate the ICP row and the photometric row of every
+// pixel of the level, weight them (IRLS), and reduce the 29 sums of the normal
+// equations plus the three outlier counts:
 //   - per thread in FP32 over at most GN_PIX_MAX pixels (2 rows each), so no
 //     FP32 sum runs over more than 2 * GN_PIX_MAX terms,
-//   - per warp / block / grid in FP64 (block partials, fixed summation order,
-//     so results are bitwise reproducible run to run),
-// and the block that finishes last for a problem runs that problem's GN step
-// on the device (cost test, step back, FP64 6x6 solve, SE(3) update,
-// convergence test).  The host only launches: the whole coarse-to-fine loop is
-// a fixed sequence of launches, and problems that stopped skip their work.
+//   - per warp / block / grid in FP64 (fixed summation order, so results are
+//     bitwise reproducible run to run),
+// and every CTA of a problem then runs the same GN step on its own copy of the
+// problem (cost test, step back, FP64 6x6 solve, SE(3) update, convergence
+// test).  The host only launches.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -87,11 +86,16 @@ struct TrackState {
   F3* rV[MAX_INSTANCES][MAX_PYR] = {};
   GNState* d_state = nullptr;       // MAX_INSTANCES (slot 0: camera, slot i: object i)
   int slot_kind[MAX_INSTANCES];     // per slot: -1 never set up, else the GNState kind
-  unsigned* d_gnbar = nullptr;      // 2 x MAX_PYR grid-barrier counters (camera, objects)
-  int coop_blocks[2] = {0, 0};      // co-resident CTAs of gn_level_kernel<0> / <1>
-  double* d_partials = nullptr;     // MAX_INSTANCES x max_tiles x 32
+  unsigned* d_gnbar = nullptr;      // MAX_INSTANCES: each problem's barrier arrivals
+  double* d_gnrows = nullptr;       // 2 x GN_CAM_ROWS x 32 partial sums of the camera's GN
+  int coop_blocks = 0, obj_blocks = 0;  // co-resident CTAs of gn_camera_kernel, gn_objects_kernel
+  double* d_objrows = nullptr;      // 2 x max_instances x max_tiles x 32 tile sums of the objects
+  uint8_t* d_objlive = nullptr;     // 2 x max_instances x max_tiles
+  double* d_partials = nullptr;     // max_tiles x 32 (one evaluation at a time)
   int max_tiles = 0;
   float2* d_zr = nullptr;           // MAX_PYR x max_tiles live depth range per CTA tile
+  float2* d_zs = nullptr;           // MAX_PYR x max_segs, per 32-pixel segment
+  int max_segs = 0;
   float* d_Twc_prev = nullptr;      // camera pose of the previous frame
   uint8_t* d_mask0 = nullptr;       // full-resolution ICP outlier mask
   float gaussian[5];
@@ -334,7 +338,9 @@ __global__ void depth2vertex_slots_kernel(SlotLevels sl) {
 // retrack: the second trackLiveFrame of a frame (kfusion.cpp:370-373), from
 // the tracked pose against the same reference pose, which stays saved.
 __global__ void setup_camera_kernel(GNState* st, const float* __restrict__ Twc,
-                                    float* __restrict__ Twc_prev, F4 k, int retrack) {
+                                    float* __restrict__ Twc_prev, F4 k, int retrack,
+                                    unsigned* __restrict__ bar) {
+  *bar = 0;   // the grid barrier of this problem's GN launch
   GNState& S = st[0];
   const M4 T = load_m4(Twc);
   const M4 Tr = retrack ? load_m4(Twc_prev) : T;
@@ -381,21 +387,14 @@ __device__ void setup_object_post(GNState& S, const M4& T_w_c2) {
   S.evalTf = T0;
 }
 
-__global__ void setup_objects_kernel(GNState* st, IdList slots, const float* __restrict__ Twc2,
-                                     const float* __restrict__ Twc1, const float* __restrict__ Two,
-                                     const int* __restrict__ inst_label) {
-  const int t = threadIdx.x;
-  if (t >= slots.n) return;
-  const int s = slots.v[t];
-  setup_object_pre(st[s], s, load_m4(Twc1), load_m4(Two + 16 * s), inst_label[s]);
-  setup_object_post(st[s], load_m4(Twc2));
-}
-__global__ void setup_objects_pre_kernel(GNState* st, IdList slots, const float* __restrict__ Twc1,
+__global__ void setup_objects_pre_kernel(GNState* st, unsigned* __restrict__ bar, IdList slots,
+                                         const float* __restrict__ Twc1,
                                          const float* __restrict__ Two,
                                          const int* __restrict__ inst_label) {
   const int t = threadIdx.x;
   if (t >= slots.n) return;
   const int s = slots.v[t];
+  bar[s] = 0;   // the barrier of this problem's CTAs
   setup_object_pre(st[s], s, load_m4(Twc1), load_m4(Two + 16 * s), inst_label[s]);
 }
 __global__ void setup_objects_post_kernel(GNState* st, IdList slots, const float* __restrict__ Twc2) {
@@ -486,6 +485,83 @@ __device__ __forceinline__ double jtj_at(const double* v21, int i, int j) {
   return v21[a * 6 - a * (a - 1) / 2 + (b - a)];
 }
 
+// solve6_eigen by one warp, the same operations on the same values (so the same
+// bits): the rotation's coefficients on every lane, its three loops over k on
+// lanes (columns of A and V at once, then the rows of A), the projections and
+// the result's components on lanes.  x on all lanes.  On one lane with the
+// matrices in local memory an iteration that needed it took some 250 us longer
+// (frames with such an object: 1.95 ms of object GN against 0.93).
+__device__ __noinline__ void solve6_eigen_warp(const double* s, int lane, double condition,
+                                               double x[6]) {
+  __shared__ double A[6][6], V[6][6], coef[6], xs[6];
+  for (int e = lane; e < 36; e += 32) {
+    const int i = e / 6, j = e % 6;
+    A[i][j] = jtj_at(s + 7, i, j);
+    V[i][j] = i == j ? 1.0 : 0.0;
+  }
+  __syncwarp();
+  for (int sweep = 0; sweep < 60; ++sweep) {
+    double off = 0;
+    for (int p = 0; p < 6; ++p)
+      for (int q = p + 1; q < 6; ++q) off += A[p][q] * A[p][q];
+    if (off < 1e-300) break;
+    for (int p = 0; p < 6; ++p)
+      for (int q = p + 1; q < 6; ++q) {
+        const double apq = A[p][q];
+        if (apq == 0) continue;
+        const double theta = (A[q][q] - A[p][p]) / (2 * apq);
+        const double ta = fabs(theta);
+        double t, c;
+        if (ta > 0x1p28) {
+          // theta^2 + 1 rounds to theta^2 and t^2 + 1 to 1, so both square
+          // roots are exact: t = 1 / (2 |theta|) (0 once theta^2 overflows)
+          t = ta > 0x1.fffffffffffffp511 ? 0.0 : 1.0 / (ta + ta);
+          t = theta >= 0 ? t : -t;
+          c = 1.0;
+        } else {
+          t = (theta >= 0 ? 1.0 : -1.0) / (ta + sqrt(theta * theta + 1));
+          c = 1 / sqrt(t * t + 1);
+        }
+        const double sn = t * c;
+        __syncwarp();
+        if (lane < 12) {
+          double(*M)[6] = lane < 6 ? A : V;
+          const int k = lane < 6 ? lane : lane - 6;
+          const double mp = M[k][p], mq = M[k][q];
+          M[k][p] = c * mp - sn * mq;
+          M[k][q] = sn * mp + c * mq;
+        }
+        __syncwarp();
+        if (lane < 6) {
+          const double ap = A[p][lane], aq = A[q][lane];
+          A[p][lane] = c * ap - sn * aq;
+          A[q][lane] = sn * ap + c * aq;
+        }
+        __syncwarp();
+      }
+  }
+  double smax = 0;
+#pragma unroll
+  for (int i = 0; i < 6; ++i) smax = fmax(smax, fabs(A[i][i]));
+  const int k = lane < 6 ? lane : 5;
+  const double sk = fabs(A[k][k]);
+  const bool use = sk > smax / condition && sk != 0;
+  double vb = 0;
+#pragma unroll
+  for (int i = 0; i < 6; ++i) vb += V[i][k] * s[1 + i];
+  if (lane < 6) coef[lane] = vb / A[lane][lane];
+  const unsigned used = __ballot_sync(FULL_MASK, use);
+  __syncwarp();
+  double xi = 0;
+  for (int j = 0; j < 6; ++j)
+    if ((used >> j) & 1u) xi += coef[j] * V[k][j];
+  if (lane < 6) xs[lane] = xi;
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 6; ++i) x[i] = xs[i];
+  __syncwarp();
+}
+
 // solve6 with row i of the eliminated system on lane i < 6 (lanes 6..31
 // repeat row 5): the pivot row reaches every lane by shuffles; x (all lanes)
 // and the fallback flag as solve6 gives them.
@@ -515,15 +591,8 @@ __device__ __forceinline__ bool solve6_warp(const double* s, int lane, double x[
   }
 #pragma unroll
   for (int j = 0; j < 6; ++j) ok = ok && (piv[j] > 1e-5 * pmax);
-  if (!ok) {  // the rare truncated eigen solve, serially on lane 0
-    if (lane == 0) {
-      double A[6][6], b[6];
-      make_jtj(v21, A);
-      for (int i = 0; i < 6; ++i) b[i] = s[1 + i];
-      solve6_eigen(A, b, 1e6, x);
-    }
-#pragma unroll
-    for (int i = 0; i < 6; ++i) x[i] = __shfl_sync(FULL_MASK, x[i], 0);
+  if (!ok) {  // the truncated eigen solve
+    solve6_eigen_warp(s, lane, 1e6, x);
     return true;
   }
   const double xr = c / a[r];
@@ -532,66 +601,56 @@ __device__ __forceinline__ bool solve6_warp(const double* s, int lane, double x[
   return false;
 }
 
-// inverse(M4) by the lanes of one warp, the same operations on the same values
-// (so the same bits): lane j < 8 holds column j of [A | I] and the elimination
-// updates every column at once; the pivot column is broadcast by shuffles.
-// m_e: element (lane & 15) of A, row-major; returns element (lane & 15) of the
-// inverse.
-__device__ __forceinline__ float inverse_warp(float m_e, int lane) {
-  const int col = lane & 7;
-  float c[4];
+// inverse(M4) by one warp, the same operations on the same values (so the
+// same bits): every lane eliminates A on its own registers (the row swaps are
+// uniform branches, rarely taken) and carries one column of the identity,
+// lane & 3.  A is read from memory by all lanes: `A` is its 16 floats, row-
+// major.  Returns element (lane & 15) of the inverse.  (One column of [A | I]
+// per lane, its pivots and factors moved by 40 shuffles, took 2.8 k cycles of
+// the GN step's 7.5 k; this form 2.1 k.)
+__device__ __forceinline__ float inverse_warp(const float* A, int lane) {
+  float a[4][4], b[4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    const float v = __shfl_sync(FULL_MASK, m_e, 4 * r + (col & 3));
-    c[r] = col < 4 ? v : (r == col - 4 ? 1.f : 0.f);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) a[r][k] = A[4 * r + k];
+    b[r] = r == (lane & 3) ? 1.f : 0.f;
   }
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    float ac[4];
+  for (int c = 0; c < 4; ++c) {
+    int p = c;
+    float best = fabsf(a[c][c]);
 #pragma unroll
-    for (int r = k; r < 4; ++r) ac[r] = __shfl_sync(FULL_MASK, c[r], k);
-    int p = k;
-    float best = fabsf(ac[k]);
+    for (int r = c + 1; r < 4; ++r)
+      if (fabsf(a[r][c]) > best) { best = fabsf(a[r][c]); p = r; }
 #pragma unroll
-    for (int r = k + 1; r < 4; ++r)
-      if (fabsf(ac[r]) > best) { best = fabsf(ac[r]); p = r; }
-#pragma unroll
-    for (int r = k + 1; r < 4; ++r) {
+    for (int r = c + 1; r < 4; ++r) {
       if (p == r) {
-        float t = c[k]; c[k] = c[r]; c[r] = t;
-        t = ac[k]; ac[k] = ac[r]; ac[r] = t;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float t = a[c][k]; a[c][k] = a[r][k]; a[r][k] = t;
+        }
+        const float t = b[c]; b[c] = b[r]; b[r] = t;
       }
     }
-    // the columns of A left of k are not updated (inverse() starts at j = k)
 #pragma unroll
-    for (int r = k + 1; r < 4; ++r) {
-      const float f = ac[r] / ac[k];
-      if (col >= k) c[r] -= f * c[k];
+    for (int r = c + 1; r < 4; ++r) {
+      const float f = a[r][c] / a[c][c];
+#pragma unroll
+      for (int k = c + 1; k < 4; ++k) a[r][k] -= f * a[c][k];  // column c is not read again
+      b[r] -= f * b[c];
     }
   }
-  // back substitution on the identity's columns (lanes 4..7), with the upper
-  // triangle of the eliminated A from lanes 0..3
-  float U[4][4];
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int k = r; k < 4; ++k) U[r][k] = __shfl_sync(FULL_MASK, c[r], k);
   float R[4];
 #pragma unroll
   for (int r = 3; r >= 0; --r) {
-    float s = c[r];
+    float s = b[r];
 #pragma unroll
-    for (int k = r + 1; k < 4; ++k) s -= U[r][k] * R[k];
-    R[r] = s / U[r][r];
+    for (int k = r + 1; k < 4; ++k) s -= a[r][k] * R[k];
+    R[r] = s / a[r][r];
   }
-  const int i = (lane >> 2) & 3;
-  float out = 0.f;
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const float v = __shfl_sync(FULL_MASK, R[r], 4 + (lane & 3));
-    if (r == i) out = v;
-  }
-  return out;
+  const int i = (lane >> 2) & 3;   // lane's own column is lane & 3, its element's row i
+  return i == 0 ? R[0] : i == 1 ? R[1] : i == 2 ? R[2] : R[3];
 }
 
 __device__ __noinline__ void gn_step_warp(GNState* Sp, const double* s, int level, int first) {
@@ -668,14 +727,14 @@ __device__ __noinline__ void gn_step_warp(GNState* Sp, const double* s, int leve
       Tl = R;
     }
   }
-  const float tf = (float)Tl;
-  const float itf = inverse_warp(tf, lane);
   if (lane < 16) {
     S.T[e] = Tl;
     S.prevT[e] = Pl;
-    reinterpret_cast<float*>(&S.Tf)[e] = tf;
-    reinterpret_cast<float*>(&S.invTf)[e] = itf;
+    reinterpret_cast<float*>(&S.Tf)[e] = (float)Tl;
   }
+  __syncwarp();
+  const float itf = inverse_warp(reinterpret_cast<const float*>(&S.Tf), lane);
+  if (lane < 16) reinterpret_cast<float*>(&S.invTf)[e] = itf;
   if (lane == 0) {
     S.prev_err = new_err;
     S.done = done;
@@ -691,173 +750,317 @@ struct GNArgs {
   int cur;              // live set index
   int W, H;             // full-resolution model maps
   const F3* mvertex; const F3* mnormal; const int* mlabel;  // composite model maps
-  F3* rV[MAX_INSTANCES];   // rendered reference vertex of each slot at this level
+  F3* rV[MAX_PYR][MAX_INSTANCES];  // rendered reference vertex of each slot, by level
   GNState* st;
   double* partials;
   int max_tiles;
   const float2* zr;     // live depth range of each CTA tile, [level][tile]
-  F4 kL;                // intrinsics at this level
+  const float2* zs;     // and of each 32-pixel segment, [level][segment]
+  int max_segs;
+  F4 kL[MAX_PYR];       // intrinsics by level
   F4 k0;                // full resolution
   float inv_cov_rgb;
   int robust;
   int use_icp, use_rgb;
-  int device_step;      // 1: the last block runs gn_step; 0: only the sums
-  int first_iter;       // 1: the first iteration of a level in the batched loop:
-                        // a stopped problem runs again and the step starts
-                        // from prev_err = infinity (trackLiveFrame's per-level
-                        // reset, tracking.cpp:247-249, 624-627)
 };
+
+// The planes of one level.  Selected by comparing the level with constants:
+// indexing the parameter arrays with it would copy them to local memory.
+struct GNView {
+  int w, h;
+  const F3* V; const F3* Vref; const F3* N; const F3* COV;
+  const float* I; const float* Iref; const float* GX; const float* GY;
+  const uint8_t* MASK;
+  F4 kL;
+};
+__device__ __forceinline__ GNView gn_view(const GNArgs& a, int L) {
+  GNView v;
+#pragma unroll
+  for (int l = 0; l < MAX_PYR; ++l) {
+    if (l != L) continue;
+    v.w = a.pyr.w[l]; v.h = a.pyr.h[l];
+    v.V = a.cur ? a.pyr.V[1][l] : a.pyr.V[0][l];
+    v.Vref = a.cur ? a.pyr.V[0][l] : a.pyr.V[1][l];
+    v.I = a.cur ? a.pyr.I[1][l] : a.pyr.I[0][l];
+    v.Iref = a.cur ? a.pyr.I[0][l] : a.pyr.I[1][l];
+    v.N = a.pyr.N[l]; v.COV = a.pyr.COV[l];
+    v.GX = a.pyr.GX[l]; v.GY = a.pyr.GY[l];
+    v.MASK = a.pyr.MASK[l];
+    v.kL = a.kL[l];
+  }
+  return v;
+}
+__device__ __forceinline__ const F3* gn_ref_vertex(const GNArgs& a, int L, int s) {
+  const F3* r = nullptr;
+#pragma unroll
+  for (int l = 0; l < MAX_PYR; ++l)
+    if (l == L) r = a.rV[l][s];
+  return r;
+}
 
 struct Row { int result; float e; float J[6]; };
 
+// length(v) > 0.1f without the square root: the square root is monotone, so
+// the test holds exactly when dot(v, v) exceeds the largest float whose square
+// root is at most 0.1f (NaN fails both).
+__device__ __forceinline__ bool longer_than_10cm(F3 v) { return dot(v, v) > 0x1.47ae16p-7f; }
+
+// sqrtf((float)(1.0 / (double)sig)): a quotient of floats rounded to double and
+// then to float equals the float quotient (53 >= 2 * 24 + 2 bits; Figueroa,
+// "When is double rounding innocuous?", 1995).
+__device__ __forceinline__ float inv_sigma(float sig) { return sqrtf(1.0f / sig); }
+
+// rotate(camera_matrix(k), v): the products with the matrix's zeros only add
+// +-0, or turn a coordinate that is out of the image anyway into NaN, which is
+// out of the image too.
+__device__ __forceinline__ F3 project(const F4& k, F3 v) {
+  return mk3(k.x * v.x + k.z * v.z, k.y * v.y + k.w * v.z, v.z);
+}
+__device__ __forceinline__ bool in_image(float px, float py, int w, int h) {
+  return !(px < 1 || px > (float)(unsigned)(w - 2) || py < 1 || py > (float)(unsigned)(h - 2) ||
+           isnan(px) || isnan(py));
+}
+
+// The four taps and fractions of a bilinear lookup; without a lookup (`in`
+// false) every tap is element 0.
+struct Cell { int b, dx, dy; float fx, fy; };
+__device__ __forceinline__ Cell cell_at(bool in, float px, float py, int w) {
+  Cell c;
+  const float fx0 = floorf(px), fy0 = floorf(py);
+  c.b = in ? (int)fx0 + (int)fy0 * w : 0;
+  c.dx = in ? 1 : 0;
+  c.dy = in ? w : 0;
+  c.fx = px - fx0;
+  c.fy = py - fy0;
+  return c;
+}
+__device__ __forceinline__ float bil4(float t00, float t10, float t01, float t11, float fx,
+                                      float fy) {
+  return t00 * (1.f - fx) * (1.f - fy) + t10 * (1.f - fy) * fx + t01 * (1.f - fx) * fy +
+         t11 * fx * fy;
+}
 __device__ __forceinline__ float bil(const float* img, int w, float px, float py) {
-  const float fx0 = floorf(px), fy0 = floorf(py);
-  const int bx = (int)fx0, by = (int)fy0;
-  const float fx = px - fx0, fy = py - fy0;
-  return img[bx + by * w] * (1.f - fx) * (1.f - fy) + img[bx + 1 + by * w] * (1.f - fy) * fx +
-         img[bx + (by + 1) * w] * (1.f - fx) * fy + img[bx + 1 + (by + 1) * w] * fx * fy;
+  const Cell c = cell_at(true, px, py, w);
+  return bil4(img[c.b], img[c.b + 1], img[c.b + w], img[c.b + w + 1], c.fx, c.fy);
 }
 
-// Object model maps derived from the composite maps and labels.
-__device__ __forceinline__ void obj_maps(const GNArgs& a, int idx, int label, F3& v, F3& n) {
-  if (a.mlabel[idx] == label) { v = a.mvertex[idx]; n = a.mnormal[idx]; }
-  else { v = mk3(0.f); n = mk3(INVALIDF, 0.f, 0.f); }
-}
-// A 2x2 cell outside the object's label box holds only other labels: its four
-// taps are (0, INVALID normal) without reading the maps (same arithmetic).
-__device__ __forceinline__ void bil_obj(const GNArgs& a, const GNState& S, float px, float py,
-                                        F3& v, F3& n) {
-  const float fx0 = floorf(px), fy0 = floorf(py);
-  const int bx = (int)fx0, by = (int)fy0;
-  const float fx = px - fx0, fy = py - fy0;
-  F3 v0, v1, v2, v3, n0, n1, n2, n3;
-  if (bx + 1 < S.box[0] || bx > S.box[2] || by + 1 < S.box[1] || by > S.box[3]) {
-    v0 = v1 = v2 = v3 = mk3(0.f);
-    n0 = n1 = n2 = n3 = mk3(INVALIDF, 0.f, 0.f);
-  } else {
-    obj_maps(a, bx + by * a.W, S.label, v0, n0);
-    obj_maps(a, bx + 1 + by * a.W, S.label, v1, n1);
-    obj_maps(a, bx + (by + 1) * a.W, S.label, v2, n2);
-    obj_maps(a, bx + 1 + (by + 1) * a.W, S.label, v3, n3);
-  }
-  const float A = 1.f - fx, B = 1.f - fy;
-  v = mk3(v0.x * A * B + v1.x * B * fx + v2.x * A * fy + v3.x * fx * fy,
-          v0.y * A * B + v1.y * B * fx + v2.y * A * fy + v3.y * fx * fy,
-          v0.z * A * B + v1.z * B * fx + v2.z * A * fy + v3.z * fx * fy);
-  n = mk3(n0.x * A * B + n1.x * B * fx + n2.x * A * fy + n3.x * fx * fy,
-          n0.y * A * B + n1.y * B * fx + n2.y * A * fy + n3.y * fx * fy,
-          n0.z * A * B + n1.z * B * fx + n2.z * A * fy + n3.z * fx * fy);
-}
+// The rows of one pixel.  Both rows are written as one straight line: the
+// loads that do not depend on the pose, both projections, every gather (at a
+// harmless address where a test failed), then both rows.  A pixel then waits
+// for memory twice, and the two rows' arithmetic overlaps; as two functions
+// with early returns a pixel's chain was 6.7 k cycles long and a level-0
+// evaluation at 640x480 12.6 us; now 3.6 k, and 12.0 us (1280x720: 45 against
+// 46, 160x120: 5.7 against 10.4).
+// A term that is off leaves result 0.
 
-// track_ICP_Kernel, tracking.cpp:923-1020.
-__device__ void icp_camera(const GNArgs& a, const GNState& S, int L, int p, Row& r) {
-  if (a.pyr.MASK[L][p]) { r.result = -6; return; }
-  const F3 n = a.pyr.N[L][p];
-  if (n.x == INVALIDF) { r.result = -1; return; }
-  const F3 pv = xform(S.Tf, a.pyr.V[a.cur][L][p]);
-  const F3 pp = xform(S.view, pv);
-  const float px = pp.x / pp.z, py = pp.y / pp.z;
-  if (px < 1 || px > (float)(unsigned)(a.W - 2) || py < 1 || py > (float)(unsigned)(a.H - 2) ||
-      isnan(px) || isnan(py)) { r.result = -2; return; }
-  const unsigned rx = (unsigned)px, ry = (unsigned)py;
-  const F3 rn = a.mnormal[rx + ry * a.W];
-  if (rn.x == INVALIDF) { r.result = -3; return; }
-  const F3 diff = a.mvertex[rx + ry * a.W] - pv;
-  const F3 pn = rotate(S.Tf, n);
-  if (length(diff) > 0.1f) { r.result = -4; return; }
-  if (dot(pn, rn) < 0.8f) { r.result = -5; return; }
-  r.result = 1;
-  const F3 P = a.pyr.COV[L][p];
-  const float sig = rn.x * rn.x * P.x + rn.y * rn.y * P.y + rn.z * rn.z * P.z;
-  const float ic = sqrtf((float)(1.0 / (double)sig));
-  r.e = ic * dot(rn, diff);
-  const F3 j1 = ic * cross(pv, rn);
-  r.J[0] = ic * rn.x; r.J[1] = ic * rn.y; r.J[2] = ic * rn.z;
-  r.J[3] = j1.x; r.J[4] = j1.y; r.J[5] = j1.z;
-}
-
-// track_Obj_ICP_Kernel, tracking.cpp:392-486 (object outlier mask is all zero).
-__device__ void icp_object(const GNArgs& a, const GNState& S, int L, int p, Row& r) {
-  const F3 cn = a.pyr.N[L][p];
-  if (cn.x == INVALIDF) { r.result = -1; return; }
-  const F3 cv = a.pyr.V[a.cur][L][p];
-  if (cv.x == 0 && cv.y == 0 && cv.z == 0) { r.result = -1; return; }
-  const F3 o2v = xform(S.invTf, cv);
-  const F3 c1v = xform(S.T_c1_o1, o2v);
-  const F3 pr = rotate(camera_matrix(a.k0), c1v);
-  const float px = pr.x / pr.z, py = pr.y / pr.z;
-  if (px < 1 || px > (float)(unsigned)(a.W - 2) || py < 1 || py > (float)(unsigned)(a.H - 2) ||
-      isnan(px) || isnan(py)) { r.result = -2; return; }
-  const F3 o2n = rotate(S.invTf, cn);
-  F3 wrv, wrn;
-  bil_obj(a, S, px, py, wrv, wrn);
-  if (wrn.x == INVALIDF) { r.result = -3; return; }
-  const F3 o1rv = xform(S.inv_T_w_o1, wrv);
-  const F3 o1rn = rotate(S.inv_T_w_o1, wrn);
-  const F3 diff = o2v - o1rv;
-  const float residual = dot(o1rn, diff);
-  if (length(diff) > 0.1f) { r.result = -4; return; }
-  if (dot(o2n, o1rn) < 0.8f) { r.result = -5; return; }
-  const F3 P = a.pyr.COV[L][p];
-  const float sig = o1rn.x * o1rn.x * P.x + o1rn.y * o1rn.y * P.y + o1rn.z * o1rn.z * P.z;
-  const float ic = sqrtf((float)(1.0 / (double)sig));
-  r.e = ic * residual;
-  const F3 Jt = rotate(S.Tf, o1rn);
-  const float c0 = -1.0f * ic * -1.0f;
-  const F3 j1 = ic * cross(cv, Jt);
-  r.J[0] = c0 * Jt.x; r.J[1] = c0 * Jt.y; r.J[2] = c0 * Jt.z;
-  r.J[3] = j1.x; r.J[4] = j1.y; r.J[5] = j1.z;
-  r.result = 1;
-}
-
-// trackRGB (tracking.cpp:1023-1111, warp :1114-1121, rgb_jacobian :1123-1150)
-// and track_obj_RGB_kernel (:491-578, obj_warp :359-367, obj_rgb_jacobian
-// :1152-1178).  The photometric outlier mask of the reference is all zero.
-__device__ void rgb_row(const GNArgs& a, const GNState& S, const F3* rV, int L, int p, int w,
-                        int h, Row& r) {
-  if (S.kind == 1) {
-    // an object's rendered reference is valid only inside its label box,
-    // halved per pyramid level (half-sampling never widens it)
-    const int x = p % w, y = p / w;
-    if (x < (S.box[0] >> L) || x > (S.box[2] >> L) || y < (S.box[1] >> L) ||
-        y > (S.box[3] >> L)) {
-      r.result = -1;
-      return;
-    }
-  }
-  const F3 rv = rV[p];
-  const F3 rl = a.pyr.V[1 - a.cur][L][p];
-  if (rv.z <= 0.f || rv.z == INVALIDF) { r.result = -1; return; }
-  if (length(rv - rl) > 0.1f && rl.z > 0.f) { r.result = -3; return; }
-  const M4 KL = camera_matrix(a.kL);
-  F3 lv, wv;
-  if (S.kind == 0) {
-    wv = xform(S.T_w_r, rv);
-    lv = xform(S.invTf, wv);
-  } else {
-    const F3 o1v = xform(S.inv_T_c1_o1, rv);
-    lv = xform(S.Tf, o1v);
-  }
-  const F3 pr = rotate(KL, lv);
-  const float px = pr.x / pr.z, py = pr.y / pr.z;
-  if (px < 1 || px > (float)(unsigned)(w - 2) || py < 1 || py > (float)(unsigned)(h - 2) ||
-      isnan(px) || isnan(py)) { r.result = -2; return; }
-  const float residual = a.pyr.I[1 - a.cur][L][p] - bil(a.pyr.I[a.cur][L], w, px, py);
-  const float gx = bil(a.pyr.GX[L], w, px, py), gy = bil(a.pyr.GY[L], w, px, py);
-  const float fx = KL.r[0].x, fy = KL.r[1].y;
-  F3 Jt = (1.f / lv.z) * mk3(gx * fx, gy * fy, -(gx * lv.x * fx + gy * lv.y * fy) / lv.z);
+// The photometric row once its taps are there: trackRGB (tracking.cpp:
+// 1023-1111, warp :1114-1121, rgb_jacobian :1123-1150) and
+// track_obj_RGB_kernel (:491-578, obj_rgb_jacobian :1152-1178).
+template <int KIND>
+__device__ __forceinline__ void rgb_finish(const GNState& S, const F4& k, float ic, float residual,
+                                           float gx, float gy, F3 wv, F3 live, Row& r) {
+  F3 Jt = (1.f / live.z) * mk3(gx * k.x, gy * k.y,
+                               -(gx * live.x * k.x + gy * live.y * k.y) / live.z);
   F3 Jr;
-  if (S.kind == 0) {
+  if (KIND == 0) {
     Jt = -1.f * rotate(S.Tf, Jt);  // rotate(Jtrans, transpose(T_w_l))
     Jr = cross(wv, Jt);
   } else {
-    Jr = cross(lv, Jt);
+    Jr = cross(live, Jt);
   }
-  const float ic = a.inv_cov_rgb;
   r.J[0] = ic * Jt.x; r.J[1] = ic * Jt.y; r.J[2] = ic * Jt.z;
   r.J[3] = ic * Jr.x; r.J[4] = ic * Jr.y; r.J[5] = ic * Jr.z;
   r.e = ic * residual;
-  r.result = 1;
+}
+
+// track_ICP_Kernel (tracking.cpp:923-1020) and trackRGB.  The photometric
+// outlier mask of the reference is all zero.
+template <bool ICP, bool RGB>
+__device__ __forceinline__ void camera_rows(const GNArgs& a, const GNView& lv, const GNState& S,
+                                            const F3* rV, int p, Row& ri, Row& rr) {
+  uint8_t mask;
+  F3 n, vl, P, rv, rl;
+  float i_ref;
+  if (ICP) { mask = lv.MASK[p]; n = lv.N[p]; vl = lv.V[p]; P = lv.COV[p]; }
+  if (RGB) { rv = rV[p]; rl = lv.Vref[p]; i_ref = lv.Iref[p]; }
+  // projections
+  F3 pv, wv, live;
+  bool in_i, in_r;
+  int q = 0;
+  Cell c;
+  if (ICP) {
+    pv = xform(S.Tf, vl);
+    const F3 pp = xform(S.view, pv);
+    const float px = pp.x / pp.z, py = pp.y / pp.z;
+    in_i = in_image(px, py, a.W, a.H);
+    ri.result = mask ? -6 : n.x == INVALIDF ? -1 : in_i ? 0 : -2;
+    q = ri.result == 0 ? (int)px + (int)py * a.W : 0;
+  }
+  if (RGB) {
+    wv = xform(S.T_w_r, rv);
+    live = xform(S.invTf, wv);
+    const F3 pr = project(lv.kL, live);
+    const float px = pr.x / pr.z, py = pr.y / pr.z;
+    in_r = in_image(px, py, lv.w, lv.h);
+    rr.result = (rv.z <= 0.f || rv.z == INVALIDF) ? -1
+                : (longer_than_10cm(rv - rl) && rl.z > 0.f) ? -3 : in_r ? 0 : -2;
+    c = cell_at(rr.result == 0, px, py, lv.w);
+  }
+  // gathers
+  F3 rn, rm;
+  float t[12];
+  if (ICP) { rn = a.mnormal[q]; rm = a.mvertex[q]; }
+  if (RGB) {
+    const int b1 = c.b + c.dx, b2 = c.b + c.dy, b3 = b2 + c.dx;
+    t[0] = lv.I[c.b]; t[1] = lv.I[b1]; t[2] = lv.I[b2]; t[3] = lv.I[b3];
+    t[4] = lv.GX[c.b]; t[5] = lv.GX[b1]; t[6] = lv.GX[b2]; t[7] = lv.GX[b3];
+    t[8] = lv.GY[c.b]; t[9] = lv.GY[b1]; t[10] = lv.GY[b2]; t[11] = lv.GY[b3];
+  }
+  if (ICP) {
+    const F3 diff = rm - pv;
+    const F3 pn = rotate(S.Tf, n);
+    if (ri.result == 0)
+      ri.result = rn.x == INVALIDF ? -3 : longer_than_10cm(diff) ? -4 : dot(pn, rn) < 0.8f ? -5 : 1;
+    const float sig = rn.x * rn.x * P.x + rn.y * rn.y * P.y + rn.z * rn.z * P.z;
+    const float ic = inv_sigma(sig);
+    ri.e = ic * dot(rn, diff);
+    const F3 j1 = ic * cross(pv, rn);
+    ri.J[0] = ic * rn.x; ri.J[1] = ic * rn.y; ri.J[2] = ic * rn.z;
+    ri.J[3] = j1.x; ri.J[4] = j1.y; ri.J[5] = j1.z;
+  } else {
+    ri.result = 0;
+  }
+  if (RGB) {
+    const float residual = i_ref - bil4(t[0], t[1], t[2], t[3], c.fx, c.fy);
+    const float gx = bil4(t[4], t[5], t[6], t[7], c.fx, c.fy);
+    const float gy = bil4(t[8], t[9], t[10], t[11], c.fx, c.fy);
+    rgb_finish<0>(S, lv.kL, a.inv_cov_rgb, residual, gx, gy, wv, live, rr);
+    if (rr.result == 0) rr.result = 1;
+  } else {
+    rr.result = 0;
+  }
+}
+
+// Object model maps derived from the composite maps and labels: the composite
+// where label == object, (0, INVALID normal) elsewhere.
+__device__ __forceinline__ void obj_maps(const GNArgs& a, int idx, bool in, int label, F3& v,
+                                         F3& n) {
+  // all three loaded before the label is looked at
+  const int l = a.mlabel[idx];
+  const F3 mv = a.mvertex[idx], mn = a.mnormal[idx];
+  const bool mine = in && l == label;
+  v = mk3(mine ? mv.x : 0.f, mine ? mv.y : 0.f, mine ? mv.z : 0.f);
+  n = mk3(mine ? mn.x : INVALIDF, mine ? mn.y : 0.f, mine ? mn.z : 0.f);
+}
+__device__ __forceinline__ F3 bil4(F3 t0, F3 t1, F3 t2, F3 t3, float fx, float fy) {
+  const float A = 1.f - fx, B = 1.f - fy;
+  return mk3(t0.x * A * B + t1.x * B * fx + t2.x * A * fy + t3.x * fx * fy,
+             t0.y * A * B + t1.y * B * fx + t2.y * A * fy + t3.y * fx * fy,
+             t0.z * A * B + t1.z * B * fx + t2.z * A * fy + t3.z * fx * fy);
+}
+
+// track_Obj_ICP_Kernel (tracking.cpp:392-486, object outlier mask all zero) and
+// track_obj_RGB_kernel.
+template <bool ICP, bool RGB>
+__device__ __forceinline__ void object_rows(const GNArgs& a, const GNView& lv, const GNState& S,
+                                            const F3* rV, int L, int p, Row& ri, Row& rr) {
+  F3 cn, cv, P, rv, rl;
+  float i_ref;
+  if (ICP) { cn = lv.N[p]; cv = lv.V[p]; P = lv.COV[p]; }
+  if (RGB) { rv = rV[p]; rl = lv.Vref[p]; i_ref = lv.Iref[p]; }
+  F3 o2v, live;
+  Cell ci, c;
+  bool cell_in = false;
+  if (ICP) {
+    o2v = xform(S.invTf, cv);
+    const F3 c1v = xform(S.T_c1_o1, o2v);
+    const F3 pr = project(a.k0, c1v);
+    const float px = pr.x / pr.z, py = pr.y / pr.z;
+    ri.result = cn.x == INVALIDF || (cv.x == 0 && cv.y == 0 && cv.z == 0) ? -1
+                : in_image(px, py, a.W, a.H) ? 0 : -2;
+    ci = cell_at(ri.result == 0, px, py, a.W);
+    // a 2x2 cell outside the object's label box holds only other labels: its
+    // taps are (0, INVALID normal) without reading the maps
+    const int bx = (int)floorf(px), by = (int)floorf(py);
+    cell_in = ri.result == 0 && !(bx + 1 < S.box[0] || bx > S.box[2] || by + 1 < S.box[1] ||
+                                  by > S.box[3]);
+    if (!cell_in) ci.b = ci.dx = ci.dy = 0;
+  }
+  if (RGB) {
+    const F3 o1v = xform(S.inv_T_c1_o1, rv);
+    live = xform(S.Tf, o1v);
+    const F3 pr = project(lv.kL, live);
+    const float px = pr.x / pr.z, py = pr.y / pr.z;
+    // an object's rendered reference is valid only inside its label box,
+    // halved per pyramid level (half-sampling never widens it)
+    const int x = p % lv.w, y = p / lv.w;
+    const bool boxed = !(x < (S.box[0] >> L) || x > (S.box[2] >> L) || y < (S.box[1] >> L) ||
+                         y > (S.box[3] >> L));
+    rr.result = !boxed || rv.z <= 0.f || rv.z == INVALIDF ? -1
+                : (longer_than_10cm(rv - rl) && rl.z > 0.f) ? -3
+                : in_image(px, py, lv.w, lv.h) ? 0 : -2;
+    c = cell_at(rr.result == 0, px, py, lv.w);
+  }
+  F3 v0, v1, v2, v3, n0, n1, n2, n3;
+  float t[12];
+  if (ICP) {
+    obj_maps(a, ci.b, cell_in, S.label, v0, n0);
+    obj_maps(a, ci.b + ci.dx, cell_in, S.label, v1, n1);
+    obj_maps(a, ci.b + ci.dy, cell_in, S.label, v2, n2);
+    obj_maps(a, ci.b + ci.dx + ci.dy, cell_in, S.label, v3, n3);
+  }
+  if (RGB) {
+    const int b1 = c.b + c.dx, b2 = c.b + c.dy, b3 = b2 + c.dx;
+    t[0] = lv.I[c.b]; t[1] = lv.I[b1]; t[2] = lv.I[b2]; t[3] = lv.I[b3];
+    t[4] = lv.GX[c.b]; t[5] = lv.GX[b1]; t[6] = lv.GX[b2]; t[7] = lv.GX[b3];
+    t[8] = lv.GY[c.b]; t[9] = lv.GY[b1]; t[10] = lv.GY[b2]; t[11] = lv.GY[b3];
+  }
+  if (ICP) {
+    const F3 wrv = bil4(v0, v1, v2, v3, ci.fx, ci.fy), wrn = bil4(n0, n1, n2, n3, ci.fx, ci.fy);
+    const F3 o2n = rotate(S.invTf, cn);
+    const F3 o1rv = xform(S.inv_T_w_o1, wrv);
+    const F3 o1rn = rotate(S.inv_T_w_o1, wrn);
+    const F3 diff = o2v - o1rv;
+    const float residual = dot(o1rn, diff);
+    if (ri.result == 0)
+      ri.result = wrn.x == INVALIDF ? -3 : longer_than_10cm(diff) ? -4
+                  : dot(o2n, o1rn) < 0.8f ? -5 : 1;
+    const float sig = o1rn.x * o1rn.x * P.x + o1rn.y * o1rn.y * P.y + o1rn.z * o1rn.z * P.z;
+    const float ic = inv_sigma(sig);
+    ri.e = ic * residual;
+    const F3 Jt = rotate(S.Tf, o1rn);
+    const float c0 = -1.0f * ic * -1.0f;
+    const F3 j1 = ic * cross(cv, Jt);
+    ri.J[0] = c0 * Jt.x; ri.J[1] = c0 * Jt.y; ri.J[2] = c0 * Jt.z;
+    ri.J[3] = j1.x; ri.J[4] = j1.y; ri.J[5] = j1.z;
+  } else {
+    ri.result = 0;
+  }
+  if (RGB) {
+    const float residual = i_ref - bil4(t[0], t[1], t[2], t[3], c.fx, c.fy);
+    const float gx = bil4(t[4], t[5], t[6], t[7], c.fx, c.fy);
+    const float gy = bil4(t[8], t[9], t[10], t[11], c.fx, c.fy);
+    rgb_finish<1>(S, lv.kL, a.inv_cov_rgb, residual, gx, gy, mk3(0.f), live, rr);
+    if (rr.result == 0) rr.result = 1;
+  } else {
+    rr.result = 0;
+  }
+}
+
+// Both rows of a pixel with the terms that the context uses (at least one).
+template <int KIND>
+__device__ __forceinline__ void gn_rows(const GNArgs& a, const GNView& lv, const GNState& S,
+                                        const F3* rV, int L, int p, Row& ri, Row& rr) {
+  if (a.use_icp && a.use_rgb) {
+    if (KIND == 0) camera_rows<true, true>(a, lv, S, rV, p, ri, rr);
+    else object_rows<true, true>(a, lv, S, rV, L, p, ri, rr);
+  } else if (a.use_icp) {
+    if (KIND == 0) camera_rows<true, false>(a, lv, S, rV, p, ri, rr);
+    else object_rows<true, false>(a, lv, S, rV, L, p, ri, rr);
+  } else {
+    if (KIND == 0) camera_rows<false, true>(a, lv, S, rV, p, ri, rr);
+    else object_rows<false, true>(a, lv, S, rV, L, p, ri, rr);
+  }
 }
 
 // Index of J_i J_j (i <= j) among the 21 upper-triangle terms, row-major
@@ -886,10 +1089,12 @@ __device__ __forceinline__ void accumulate(float* acc, int* cnt, const Row& r, i
   acc[28] += 1.f;
 }
 
-// Range of live depths over the pixels of each GN tile (CTA) and level whose
-// ICP row gets past the validity checks (valid normal, nonzero vertex).
-__global__ void tile_depth_range_kernel(PyrPtrs pyr, int cur, float2* __restrict__ zr,
-                                        int max_tiles) {
+// Range of live depths over the pixels of each GN tile and of each 32-pixel
+// segment (a warp's pixels of one step through its tile) whose ICP row gets
+// past the validity checks (valid normal, nonzero vertex), by level.
+__global__ void __launch_bounds__(GN_THREADS)
+tile_depth_range_kernel(PyrPtrs pyr, int cur, float2* __restrict__ zr, int max_tiles,
+                        float2* __restrict__ zs, int max_segs) {
   const int L = blockIdx.y;
   const int w = pyr.w[L], n = w * pyr.h[L];
   const int ppt = gn_pix(L);
@@ -898,14 +1103,18 @@ __global__ void tile_depth_range_kernel(PyrPtrs pyr, int cur, float2* __restrict
   float lo = INFINITY, hi = -INFINITY;
   for (int k = 0; k < ppt; ++k) {
     const int p = p0 + k * GN_THREADS + threadIdx.x;
+    float l = INFINITY, h = -INFINITY;
     if (p < n && pyr.N[L][p].x != INVALIDF) {
       const F3 v = pyr.V[cur][L][p];
-      if (!(v.x == 0 && v.y == 0 && v.z == 0)) { lo = fminf(lo, v.z); hi = fmaxf(hi, v.z); }
+      if (!(v.x == 0 && v.y == 0 && v.z == 0)) { l = fminf(l, v.z); h = fmaxf(h, v.z); }
     }
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    for (int o = 16; o > 0; o >>= 1) {
+      l = fminf(l, __shfl_xor_sync(0xffffffffu, l, o));
+      h = fmaxf(h, __shfl_xor_sync(0xffffffffu, h, o));
+    }
+    if ((threadIdx.x & 31) == 0 && p < n) zs[(size_t)L * max_segs + (p >> 5)] = make_float2(l, h);
+    lo = fminf(lo, l);
+    hi = fmaxf(hi, h);
   }
   __shared__ float2 sw[GN_THREADS / 32];
   if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = make_float2(lo, hi);
@@ -934,8 +1143,8 @@ __global__ void tile_depth_range_kernel(PyrPtrs pyr, int cur, float2* __restrict
 // behind camera 1 or a NaN projection makes the answer true, as the first such
 // corner did in a sequential loop; otherwise no NaN reaches the minima and
 // maxima, so their order does not matter.
-__device__ bool object_tile_live(const GNArgs& a, const GNState& S, int L, int tile, int w,
-                                 int n) {
+__device__ bool object_tile_live(const GNArgs& a, const F4& kL, const GNState& S, int L,
+                                 int tile, int w, int n) {
   const int ppt = gn_pix(L);
   const int p0 = tile * GN_THREADS * ppt, p1 = min(n, p0 + GN_THREADS * ppt);
   const int ya = p0 / w, yb = (p1 - 1) / w;
@@ -948,7 +1157,7 @@ __device__ bool object_tile_live(const GNArgs& a, const GNState& S, int L, int t
   if (!a.use_icp) return false;
   const float2 zr = a.zr[L * a.max_tiles + tile];
   if (!(zr.x <= zr.y)) return false;  // no pixel of the tile reaches the projection
-  const M4 iK = inverse_camera_matrix(a.kL), K0 = camera_matrix(a.k0);
+  const M4 iK = inverse_camera_matrix(kL), K0 = camera_matrix(a.k0);
   const int c = threadIdx.x & 7;
   const float x = (float)((c & 1) ? xb : xa), y = (float)((c & 2) ? yb : ya);
   const float z = (c & 4) ? zr.y : zr.x;
@@ -1016,14 +1225,14 @@ template <int KIND>
 __device__ __forceinline__ double gn_tile_sums(const GNArgs& a, const GNState& S, int s, int L,
                                                int tile, double (*sh)[32],
                                                float (*red)[32][33]) {
-  const int w = a.pyr.w[L], h = a.pyr.h[L];
-  const int n = w * h;
+  const GNView lv = gn_view(a, L);
+  const int w = lv.w, n = w * lv.h;
   bool live = true;
   if (KIND == 1) {
     __shared__ int s_live;
     if (threadIdx.x < 32) {
-      const bool lv = object_tile_live(a, S, L, tile, w, n);
-      if (threadIdx.x == 0) s_live = lv ? 1 : 0;
+      const bool tl = object_tile_live(a, lv.kL, S, L, tile, w, n);
+      if (threadIdx.x == 0) s_live = tl ? 1 : 0;
     }
     __syncthreads();
     live = s_live != 0;
@@ -1034,24 +1243,16 @@ __device__ __forceinline__ double gn_tile_sums(const GNArgs& a, const GNState& S
 #pragma unroll
     for (int i = 0; i < 29; ++i) acc[i] = 0.f;
     int cnt[3] = {0, 0, 0};
-    const F3* rV = a.rV[s];
+    const F3* rV = gn_ref_vertex(a, L, s);
     const int ppt = gn_pix(L);
 #pragma unroll 1
     for (int k = 0; k < ppt; ++k) {
       const int p = tile * (GN_THREADS * ppt) + k * GN_THREADS + threadIdx.x;
       if (p >= n) break;
-      Row r;
-      if (a.use_icp) {
-        r.result = 0;
-        if (KIND == 0) icp_camera(a, S, L, p, r);
-        else icp_object(a, S, L, p, r);
-        accumulate(acc, cnt, r, a.robust);
-      }
-      if (a.use_rgb) {
-        r.result = 0;
-        rgb_row(a, S, rV, L, p, w, h, r);
-        accumulate(acc, cnt, r, a.robust);
-      }
+      Row ri, rr;
+      gn_rows<KIND>(a, lv, S, rV, L, p, ri, rr);
+      if (a.use_icp) accumulate(acc, cnt, ri, a.robust);
+      if (a.use_rgb) accumulate(acc, cnt, rr, a.robust);
     }
     sh[warp][lane] = warp_sum_fp64(acc, cnt, red[warp], lane);
   } else {
@@ -1070,12 +1271,12 @@ __device__ __forceinline__ double gn_tile_sums(const GNArgs& a, const GNState& S
 // by the whole CTA (the last CTA of the problem): tot[i] = sum i.  The loads
 // of 16 tiles are issued before their in-order additions, so the tail waits on
 // about ntiles / 128 L2 round trips instead of ntiles / 64.
-__device__ __forceinline__ void gn_tail_sums(const GNArgs& a, int s, int ntiles,
+__device__ __forceinline__ void gn_tail_sums(const GNArgs& a, int ntiles,
                                              double (*sh)[32], double* tot) {
   constexpr int G = GN_THREADS / 32, U = 16;
   {
     const int i = threadIdx.x & 31, g = threadIdx.x >> 5;  // 8 groups of tiles
-    const double* col = a.partials + (size_t)s * a.max_tiles * 32 + i;
+    const double* col = a.partials + i;
     double v = 0;
     int b = g;
     for (; b + (U - 1) * G < ntiles; b += U * G) {
@@ -1098,66 +1299,19 @@ __device__ __forceinline__ void gn_tail_sums(const GNArgs& a, int s, int ntiles,
   __syncthreads();
 }
 
-// One GN iteration of every problem in `slots` (grid.y = problem): the rows of
-// every tile, the tile partials, and in the CTA that finishes last for a
-// problem (ticket counter) the sum over the tiles and, with device_step, the
-// problem's GN step on the device.
-// KIND 0: the camera problem; KIND 1: object problems (one instantiation each
-// keeps the kernel's code small).
-// Programmatic dependent launch: the iterations of a level are chained so that
-// the next launch's CTAs start while the previous one finishes (its tail and
-// step), issue the prefetch of their pose-independent pixel data, and wait
-// (griddepcontrol.wait) before they read anything the previous launch writes
-// (the problem states, the partials).  Without the launch attribute the wait
-// returns at once.
-__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void griddep_launch_dependents() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void prefetch_l1(const void* p) {
-  asm volatile("prefetch.L1 [%0];" :: "l"(p));
-}
-
-// The pixel data of a tile that does not depend on the pose (live vertex,
-// normal, covariance and mask; rendered and live reference vertex, reference
-// intensity) into L1.  Written before the GN launches of a frame start.
-__device__ __forceinline__ void gn_prefetch(const GNArgs& a, int s, int L, int tile) {
-  const int n = a.pyr.w[L] * a.pyr.h[L];
-  const int ppt = gn_pix(L);
-#pragma unroll 1
-  for (int k = 0; k < ppt; ++k) {
-    const int p = tile * (GN_THREADS * ppt) + k * GN_THREADS + threadIdx.x;
-    if (p >= n) break;
-    if (a.use_icp) {
-      prefetch_l1(a.pyr.N[L] + p);
-      prefetch_l1(a.pyr.V[a.cur][L] + p);
-      prefetch_l1(a.pyr.COV[L] + p);
-      prefetch_l1(a.pyr.MASK[L] + p);
-    }
-    if (a.use_rgb) {
-      prefetch_l1(a.rV[s] + p);
-      prefetch_l1(a.pyr.V[1 - a.cur][L] + p);
-      prefetch_l1(a.pyr.I[1 - a.cur][L] + p);
-    }
-  }
-}
-
+// One evaluation of the normal equations of the problem in slot s: the rows of
+// every tile, the tile partials, and in the CTA that finishes last (ticket
+// counter) the sum over the tiles.
 template <int KIND>
 __global__ void __launch_bounds__(GN_THREADS, MF_GN_MINB)
-gn_iter_kernel(GNArgs a, IdList slots, int L) {
-  const int s = slots.v[blockIdx.y];
-  gn_prefetch(a, s, L, blockIdx.x);
-  griddep_wait();
+gn_eval_kernel(GNArgs a, int s, int L) {
   GNState& S = a.st[s];
-  if (S.done && !a.first_iter) return;
-  // every CTA of this launch is resident: the next iteration may start
-  griddep_launch_dependents();
   __shared__ double sh[GN_THREADS / 32][32];
   __shared__ float red[GN_THREADS / 32][32][33];
   const double v = gn_tile_sums<KIND>(a, S, s, L, blockIdx.x, sh, red);
   __shared__ bool last;
   if (threadIdx.x < 32) {
-    a.partials[((size_t)s * a.max_tiles + blockIdx.x) * 32 + threadIdx.x] = v;
+    a.partials[(size_t)blockIdx.x * 32 + threadIdx.x] = v;
     __threadfence();
   }
   __syncthreads();
@@ -1169,27 +1323,133 @@ gn_iter_kernel(GNArgs a, IdList slots, int L) {
   if (!last) return;
   __threadfence();
   __shared__ double tot[32];
-  gn_tail_sums(a, s, (int)gridDim.x, sh, tot);
+  gn_tail_sums(a, (int)gridDim.x, sh, tot);
   if (threadIdx.x < 32) {
     S.sums[L][threadIdx.x] = tot[threadIdx.x];
     if (threadIdx.x == 0) S.ticket = 0;
-    if (a.device_step) gn_step_warp(&S, tot, L, a.first_iter);
   }
 }
 
-// ------------------------------------------------------------------ persistent level
-// All GN iterations of one pyramid level for every problem in `slots`, in one
-// cooperative launch (every CTA resident): the (problem, tile) items of an
-// iteration are spread over the grid, the CTA that finishes a problem's last
-// tile sums its partials and runs its step (as gn_iter_kernel does), and a
-// grid barrier separates the iterations.  After each barrier the CTAs read the
-// problems' `done` flags; when every problem has stopped, the level ends
-// without launching the remaining iterations.  The per-pixel rows, the tile
-// partials, their sum and the step are gn_iter_kernel's, so the poses equal
-// the per-iteration launches' bit for bit.
-// Every wait is bounded: a barrier that does not complete within
-// GN_BAR_SPINS polls sets MF_STATUS_GN_TIMEOUT and the CTA returns.
-constexpr unsigned GN_BAR_SPINS = 1u << 22;   // x >= 64 ns sleeps: about 0.3 s
+// ------------------------------------------------------------------ whole GN loops
+// The coarse-to-fine GN of a stage in one launch.  The pixels of a level stay
+// with the same CTA over all its iterations, so the rows' inputs stay in that
+// SM's L1; an iteration is the rows of the CTA's tiles, one exchange of the
+// CTAs' partial sums, and then every CTA adds the same partials in the same
+// order and runs the same step on its own copy of the problem in shared
+// memory.  No CTA waits for another one's step, no state travels between
+// them, and a problem that stopped ends its level at once.
+//
+// Sums: FP32 per thread over the rows of its 1 (level > 0) or 3 pixels of a
+// tile, FP64 from there on in a fixed order: the warp's lanes, each warp's
+// tiles (row, row + R, ...: "row" is a virtual CTA, R a constant), the 16
+// warps of the row, the rows.  The order does not depend on the grid or on
+// the device, and the plain mode evaluates through the same kernels, so poses
+// are the same bit for bit in every mode.
+// Tiles in flight per CTA: two teams of 8 warps at 128 registers each.  Three
+// at 80 registers spill, and a pixel's chain then takes 5.2 k instead of 3.6 k
+// cycles: 160x120 29.2 k against 23.5 k cycles per level-0 iteration, 640x480
+// 37.4 k against 36.4 k; only 1280x720, with eight tiles per SM, gains 2 % by
+// the third.
+constexpr int GN_TEAMS = 2;
+constexpr int GN_BLOCK = GN_TEAMS * GN_THREADS;
+constexpr int GN_WARPS = GN_BLOCK / 32;
+constexpr int GN_CAM_ROWS = 148;                     // one virtual CTA per SM
+
+struct GNShared {
+  GNState S;
+  GNView lv;         // the level being evaluated
+  double sh[GN_WARPS][32];
+  double tot[32];
+  int flag;
+  float red[GN_WARPS][32][17];   // a warp's transposition: 16 values of 32 lanes at a time
+};
+
+struct GNLoop {
+  int levels;
+  int iters[MAX_PYR];
+  int only;          // >= 0: one evaluation of this level without a step (sums only)
+  double* rows;      // partial sums, alternating by iteration: camera 2 x GN_CAM_ROWS x 32,
+                     // objects 2 x slots x max_tiles x 32
+  uint8_t* lives;    // objects: the tiles with a sum, 2 x slots x max_tiles
+  unsigned* bar;     // barrier arrivals by problem slot
+  int slots;         // problem slots (the context's instance capacity)
+  int* status;
+  float* poses;      // camera: T_w_c; objects: the volume poses
+};
+
+// The warp's FP64 sum of value `lane` (29 sums, then the 3 counts).  The lanes'
+// FP32 values are transposed through shared memory 16 at a time; the two
+// halves of the warp add 16 lanes' values each, in two chains.
+__device__ __forceinline__ double gn_warp_sum(const float* acc, const int* cnt, float (*red)[17],
+                                              int lane) {
+  const int col = lane & 15, half = lane >> 4;
+  double out = 0;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      red[lane][i] = 16 * h + i < 29 ? acc[16 * h + i < 29 ? 16 * h + i : 0]
+                                     : (float)cnt[16 * h + i < 29 ? 0 : 16 * h + i - 29];  // exact
+    __syncwarp();
+    double v0 = 0, v1 = 0;
+#pragma unroll
+    for (int j = 0; j < 16; j += 2) {
+      v0 += (double)red[16 * half + j][col];
+      v1 += (double)red[16 * half + j + 1][col];
+    }
+    double v = v0 + v1;
+    v += __shfl_xor_sync(FULL_MASK, v, 16);
+    if (half == h) out = v;
+    __syncwarp();
+  }
+  return out;
+}
+
+// The sum over the CTA's 16 warps of sh[warp][lane], by one warp, in four chains.
+__device__ __forceinline__ double gn_sum_warps(const double (*sh)[32], int lane) {
+  double c[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int k = 0; k < GN_WARPS; k += 4)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) c[q] += sh[k + q][lane];
+  return (c[0] + c[1]) + (c[2] + c[3]);
+}
+
+// The 32 sums of a row (its tiles row, row + nrows, ...) of level L, by the
+// whole CTA: team j of 8 warps takes every second of them.  Returned by lane i
+// of warp 0.  Every thread reaches the barrier inside.
+template <int KIND>
+__device__ __forceinline__ double gn_row_sums(const GNArgs& a, GNShared& sm, int s, int L,
+                                              int row, int nrows) {
+  const GNView& lv = sm.lv;
+  const int n = lv.w * lv.h, ppt = gn_pix(L);
+  const int ntiles = (n + GN_THREADS * ppt - 1) / (GN_THREADS * ppt);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int team = warp / (GN_THREADS / 32), wi = warp % (GN_THREADS / 32);
+  const GNState& S = sm.S;
+  const F3* rV = gn_ref_vertex(a, L, s);
+  double v = 0;
+#pragma unroll 1
+  for (int t = row + nrows * team; t < ntiles; t += GN_TEAMS * nrows) {
+    float acc[29];
+#pragma unroll
+    for (int i = 0; i < 29; ++i) acc[i] = 0.f;
+    int cnt[3] = {0, 0, 0};
+#pragma unroll 1
+    for (int k = 0; k < ppt; ++k) {
+      const int p = (t * ppt + k) * GN_THREADS + wi * 32 + lane;
+      if (p >= n) break;
+      Row ri, rr;
+      gn_rows<KIND>(a, lv, S, rV, L, p, ri, rr);
+      if (a.use_icp) accumulate(acc, cnt, ri, a.robust);
+      if (a.use_rgb) accumulate(acc, cnt, rr, a.robust);
+    }
+    v += gn_warp_sum(acc, cnt, sm.red[warp], lane);
+  }
+  sm.sh[warp][lane] = v;
+  __syncthreads();
+  return warp == 0 ? gn_sum_warps(sm.sh, lane) : 0.0;
+}
 
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   unsigned v;
@@ -1197,89 +1457,450 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   return v;
 }
 
-// GNState copied between global memory (through L2: other SMs write it within
-// the launch) and shared memory, by the whole CTA.
-__device__ __forceinline__ void state_load(const GNState* g, GNState* sm) {
-  static_assert(sizeof(GNState) % 4 == 0, "GNState is copied as words");
-  const int* src = reinterpret_cast<const int*>(g);
-  int* dst = reinterpret_cast<int*>(sm);
-  for (int i = threadIdx.x; i < (int)(sizeof(GNState) / 4); i += blockDim.x) dst[i] = __ldcg(src + i);
-  __syncthreads();
-}
-__device__ __forceinline__ void state_store(const GNState* sm, GNState* g) {
-  const int* src = reinterpret_cast<const int*>(sm);
-  int* dst = reinterpret_cast<int*>(g);
-  for (int i = threadIdx.x; i < (int)(sizeof(GNState) / 4); i += blockDim.x) __stcg(dst + i, src[i]);
-  __threadfence();
-  __syncthreads();
+// Waits until `target` CTAs have arrived at `bar`.  Bounded: after GN_BAR_SPINS
+// polls it sets MF_STATUS_GN_TIMEOUT and returns 1, and the CTA returns.
+constexpr unsigned GN_BAR_SPINS = 1u << 21;   // polls, 32 ns apart after the first 64: about 1 s
+__device__ __forceinline__ int gn_wait(const unsigned* bar, unsigned target, int* status) {
+  for (unsigned spins = 0; ld_acquire_u32(bar) < target; ++spins) {
+    if (spins >= GN_BAR_SPINS) {
+      atomicOr(status, MF_STATUS_GN_TIMEOUT);
+      return 1;
+    }
+    if (spins > 64) __nanosleep(32);
+  }
+  return 0;
 }
 
-template <int KIND>
-__global__ void __launch_bounds__(GN_THREADS, MF_GN_MINB)
-gn_level_kernel(GNArgs a, IdList slots, int L, int iters, int ntiles, unsigned* __restrict__ bar,
-                int* __restrict__ status) {
-  __shared__ GNState sS;
-  __shared__ double sh[GN_THREADS / 32][32];
-  __shared__ float red[GN_THREADS / 32][32][33];
-  __shared__ double tot[32];
-  __shared__ int s_flag, s_done;
-  const int items = slots.n * ntiles;
-  for (int it = 0; it < iters; ++it) {
-    for (int item = blockIdx.x; item < items; item += gridDim.x) {
-      const int pi = item / ntiles, tile = item - pi * ntiles;
-      const int s = slots.v[pi];
-      state_load(a.st + s, &sS);
-      // a stopped problem runs again in the level's first iteration (the
-      // level's reset, tracking.cpp:247-249, 624-627)
-      if (sS.done && it > 0) continue;
-      const double v = gn_tile_sums<KIND>(a, sS, s, L, tile, sh, red);
-      if (threadIdx.x < 32) {
-        a.partials[((size_t)s * a.max_tiles + tile) * 32 + threadIdx.x] = v;
+__device__ __forceinline__ void gn_copy_state(const GNState* from, GNState* to) {
+  static_assert(sizeof(GNState) % 4 == 0, "GNState is copied as words");
+  const int* src = reinterpret_cast<const int*>(from);
+  int* dst = reinterpret_cast<int*>(to);
+  for (int i = threadIdx.x; i < (int)(sizeof(GNState) / 4); i += blockDim.x) dst[i] = src[i];
+}
+
+// The camera's GN (trackLiveFrame :240-335): a cooperative launch of one CTA
+// per SM (fewer for small frames).  The partial rows are exchanged through L2
+// with one grid barrier per iteration.
+// What bounds it at 640x480: the evaluation of the rows (instruction issue,
+// the FP64 of the weights included), then the serial tail of an iteration
+// (barrier, row sums, step).  One launch per iteration, chained by
+// programmatic dependent launch, with the step in the CTA that finished last,
+// took 260 us for a frame's iterations (ncu, their sum); this launch takes 130.
+__global__ void __launch_bounds__(GN_BLOCK, 1)
+gn_camera_kernel(GNArgs a, GNLoop g) {
+  extern __shared__ __align__(16) unsigned char gn_smem[];
+  GNShared& sm = *reinterpret_cast<GNShared*>(gn_smem);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  gn_copy_state(a.st, &sm.S);
+  __syncthreads();
+  unsigned target = 0;
+  int par = 0;
+  for (int L = g.only >= 0 ? g.only : g.levels - 1; L >= (g.only >= 0 ? g.only : 0); --L) {
+    if (threadIdx.x == 0) sm.lv = gn_view(a, L);
+    __syncthreads();
+    const int n = sm.lv.w * sm.lv.h, tp = GN_THREADS * gn_pix(L);
+    const int nrows = min((n + tp - 1) / tp, GN_CAM_ROWS);
+    int iters = 1;
+    if (g.only < 0) {
+#pragma unroll
+      for (int l = 0; l < MAX_PYR; ++l)
+        if (l == L) iters = g.iters[l];
+    }
+    for (int it = 0; it < iters; ++it) {
+      double* rows = g.rows + (size_t)par * GN_CAM_ROWS * 32;
+      for (int row = blockIdx.x; row < nrows; row += gridDim.x) {
+        const double v = gn_row_sums<0>(a, sm, 0, L, row, nrows);
+        if (warp == 0) __stcg(rows + row * 32 + lane, v);
+        if (row + (int)gridDim.x < nrows) __syncthreads();  // sh is written again
+      }
+      if (warp == 0) {
         __threadfence();
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) s_flag = atomicAdd(&a.st[s].ticket, 1) == ntiles - 1;
-      __syncthreads();
-      if (!s_flag) continue;
-      __threadfence();
-      gn_tail_sums(a, s, ntiles, sh, tot);
-      if (threadIdx.x < 32) sS.sums[L][threadIdx.x] = tot[threadIdx.x];
-      __syncthreads();
-      if (threadIdx.x < 32) {
-        if (threadIdx.x == 0) sS.ticket = 0;
-        gn_step_warp(&sS, tot, L, it == 0);
-      }
-      __syncthreads();
-      state_store(&sS, a.st + s);
-    }
-    // grid barrier; then every CTA reads the same `done` flags
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      atomicAdd(bar, 1u);
-      const unsigned target = (unsigned)(it + 1) * gridDim.x;
-      int flag = 0;
-      for (unsigned spins = 0; ld_acquire_u32(bar) < target; ++spins) {
-        if (spins >= GN_BAR_SPINS) {
-          atomicOr(status, MF_STATUS_GN_TIMEOUT);
-          flag = -1;
-          break;
+        __syncwarp();
+        if (lane == 0) {
+          atomicAdd(g.bar, 1u);
+          target += gridDim.x;
+          sm.flag = gn_wait(g.bar, target, g.status);
         }
-        __nanosleep(64);
       }
-      s_flag = flag;
+      __syncthreads();
+      if (sm.flag) return;
+      // every load in flight before the first addition
+      constexpr int U = (GN_CAM_ROWS + GN_WARPS - 1) / GN_WARPS;
+      double part[U], v = 0;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        part[u] = warp + u * GN_WARPS < nrows ? __ldcg(rows + (warp + u * GN_WARPS) * 32 + lane)
+                                              : 0.0;
+#pragma unroll
+      for (int u = 0; u < U; ++u) v += part[u];
+      sm.sh[warp][lane] = v;
+      __syncthreads();
+      if (warp == 0) {
+        const double t = gn_sum_warps(sm.sh, lane);
+        sm.tot[lane] = t;
+        sm.S.sums[L][lane] = t;
+        __syncwarp();
+        if (g.only < 0) gn_step_warp(&sm.S, sm.tot, L, it == 0);
+      }
+      __syncthreads();
+      par ^= 1;
+      if (sm.S.done && g.only < 0) break;
+    }
+  }
+  if (blockIdx.x != 0) return;
+  gn_copy_state(&sm.S, a.st);
+  if (g.only < 0 && threadIdx.x < 16) g.poses[threadIdx.x] = (float)sm.S.T[threadIdx.x];
+}
+
+// ------------------------------------------------------------------ objects
+// The objects' GN (trackEachObject :629-694): one cooperative launch whose
+// CTAs are shared out among the objects, one or more each in proportion to
+// the objects' label boxes.  The CTAs of an object run its whole loop and
+// wait for each other only (one barrier per object and iteration), so a small
+// object never waits for a large one.
+//
+// An object covers a few percent of the frame.  Each iteration first lists
+// the CTA's tasks -- (tile, warp of the tile) pairs with a 32-pixel segment
+// that can hold a valid row (object_segment_live) -- one thread per pair, and
+// the warps then take the listed tasks in turn.  A tile is 768 consecutive
+// pixels, more than one image row of a 640-pixel frame: with whole tiles as
+// the unit, six of seven evaluated pixels lay beside the object.
+//
+// The object problems can be so poorly conditioned that the last bit of a sum
+// shows in the pose, so the order of the FP64 sums is fixed whatever the
+// number of CTAs: the lanes of a warp in order, the 8 warps of a tile, the
+// tiles g, g + 8, ... of column g in order, the 8 columns.  Warps and tiles
+// without a live segment would add exact zeros and are left out.
+//
+// Measured on one B200 (ncu, a frame's launches of 19 iterations against this
+// one): three objects at 640x480 383 -> 258 us, six at 1280x720 869 -> 450,
+// twelve of uneven size at 640x480 1178 -> 734.
+constexpr int GO_WARPS = 16, GO_BLOCK = 32 * GO_WARPS;
+constexpr int GO_CHUNK = 32;               // tiles listed at a time
+constexpr int GO_TASKS = 8 * GO_CHUNK;
+
+struct GOShared {
+  GNState S;
+  GNView lv;
+  double sh[8][32];              // the columns' sums
+  double tot[32];
+  double ws[GO_TASKS][32];       // warp sums of the listed tasks
+  float red[GO_WARPS][32][33];
+  int list[GO_TASKS];            // task | live segments << 16
+  int live[GO_TASKS];            // task -> its live segments
+  short slot[GO_TASKS];          // task -> its place in the list, or -1
+  int pick[GO_WARPS][32];        // the live ones of 32 tiles of a column
+  int ntask, flag;
+  int obj, rank, size;           // this CTA's place: list position, rank among its CTAs, their number
+  M4 M;                          // T_c1_o1 inverse(T): live camera -> reference camera, its x
+                                 // and y rows taken through the intrinsics
+  float ifx, ify;                // 1 / focal lengths of the level
+  F3 origin;                     // the world origin's image in the live camera
+};
+
+// object_tile_live for one 32-pixel segment, by one thread.  The bounds only
+// have to hold up to its slack (2 pixels, 1 mm), so the frustum's corners are
+// taken through one product matrix (its rows scaled by the intrinsics), the
+// quotients are approximate ones, and the distance to the world origin is
+// taken in the live camera's frame.
+__device__ __forceinline__ bool object_segment_live(const GNArgs& a, const GOShared& sm, int L,
+                                                    int p0, int n) {
+  const GNState& S = sm.S;
+  const int w = sm.lv.w, p1 = min(n, p0 + 32) - 1;
+  const int ya = p0 / w, xe = p0 - ya * w + (p1 - p0);   // xe: the last pixel's x in row ya
+  const bool one_row = xe < w;
+  const int yb = one_row ? ya : p1 / w;
+  const int xa = one_row ? p0 - ya * w : 0, xb = one_row ? xe : w - 1;
+  const bool has_box = S.box[2] >= S.box[0];
+  if (a.use_rgb && has_box &&
+      !(xb < (S.box[0] >> L) || xa > (S.box[2] >> L) || yb < (S.box[1] >> L) ||
+        ya > (S.box[3] >> L)))
+    return true;
+  if (!a.use_icp) return false;
+  const float2 zr = a.zs[(size_t)L * a.max_segs + (p0 >> 5)];
+  if (!(zr.x <= zr.y)) return false;  // no pixel of the segment reaches the projection
+  float qx0 = INFINITY, qx1 = -INFINITY, qy0 = INFINITY, qy1 = -INFINITY;
+  bool unbounded = false;   // behind camera 1, or NaN
+  const float xs[2] = {((float)xa - sm.lv.kL.z) * sm.ifx, ((float)xb - sm.lv.kL.z) * sm.ifx};
+  const float ys[2] = {((float)ya - sm.lv.kL.w) * sm.ify, ((float)yb - sm.lv.kL.w) * sm.ify};
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    if (c >= 2 && one_row) continue;   // one image row: its two ends
+    const float dx = xs[c & 1], dy = ys[c >> 1];
+    const F3 D = rotate(sm.M, mk3(dx, dy, 1.f));
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float z = e ? zr.y : zr.x;
+      const F3 q = z * D + get_translation(sm.M);
+      const float px = __fdividef(q.x, q.z), py = __fdividef(q.y, q.z);
+      unbounded |= !(q.z > 0.f) || isnan(px) || isnan(py);
+      qx0 = fminf(qx0, px); qx1 = fmaxf(qx1, px);
+      qy0 = fminf(qy0, py); qy1 = fmaxf(qy1, py);
+    }
+  }
+  if (unbounded) return true;
+  if (has_box && floorf(qx1) + 3.f >= (float)S.box[0] && floorf(qx0) - 2.f <= (float)S.box[2] &&
+      floorf(qy1) + 3.f >= (float)S.box[1] && floorf(qy0) - 2.f <= (float)S.box[3])
+    return true;
+  // the frustum's box in the live camera: x and y reach z times the directions
+  const float x0 = fminf(zr.x * xs[0], zr.y * xs[0]), x1 = fmaxf(zr.x * xs[1], zr.y * xs[1]);
+  const float ylo = fminf(ys[0], ys[1]), yhi = fmaxf(ys[0], ys[1]);
+  const float y0 = fminf(zr.x * ylo, zr.y * ylo), y1 = fmaxf(zr.x * yhi, zr.y * yhi);
+  const float ox = fmaxf(fmaxf(x0 - sm.origin.x, sm.origin.x - x1), 0.f);
+  const float oy = fmaxf(fmaxf(y0 - sm.origin.y, sm.origin.y - y1), 0.f);
+  const float oz = fmaxf(fmaxf(zr.x - sm.origin.z, sm.origin.z - zr.y), 0.f);
+  // a NaN origin bounds nothing
+  return !(ox * ox + oy * oy + oz * oz > 0.101f * 0.101f);
+}
+
+// mul(A, B) by the lanes of one warp, element (lane & 15), A and B row-major.
+__device__ __forceinline__ float mul_warp(const float* A, const float* B, int lane) {
+  const int i = (lane >> 2) & 3, j = lane & 3;
+  float s = A[4 * i] * B[j];
+#pragma unroll
+  for (int k = 1; k < 4; ++k) s += A[4 * i + k] * B[4 * k + j];
+  return s;
+}
+
+// The share of CTA `b` of `nb`: every object one CTA, the others in proportion
+// to the 32-pixel segments that their label boxes meet (in pixels).  With
+// fewer CTAs than objects CTA b takes objects b, b + nb, ...
+__device__ void gn_share(const GNState* __restrict__ st, const IdList& slots, int b, int nb,
+                         GOShared& sm) {
+  long long area[MAX_INSTANCES], total = 0;
+  for (int i = 0; i < slots.n; ++i) {
+    const GNState& S = st[slots.v[i]];
+    const long long w = S.box[2] - S.box[0] + 1, h = S.box[3] - S.box[1] + 1;
+    area[i] = (S.box[2] >= S.box[0] ? (w + 48) * h : 0) + GN_THREADS * GN_PIX_MAX;
+    total += area[i];
+  }
+  const int spare = nb - slots.n;
+  sm.obj = b;
+  sm.rank = 0;
+  sm.size = 1;
+  if (spare <= 0) return;
+  long long sum = 0;
+  int first = 0;
+  for (int i = 0; i < slots.n; ++i) {
+    // the cumulative share rounded down, so that the shares add up to nb
+    sum += area[i];
+    const int next = (int)(spare * sum / total) + i + 1;
+    if (b < next) {
+      sm.obj = i;
+      sm.rank = b - first;
+      sm.size = next - first;
+      return;
+    }
+    first = next;
+  }
+}
+
+__global__ void __launch_bounds__(GO_BLOCK, 1)
+gn_objects_kernel(GNArgs a, GNLoop g, IdList slots, const float* __restrict__ Twc2) {
+  extern __shared__ __align__(16) unsigned char gn_smem[];
+  GOShared& sm = *reinterpret_cast<GOShared*>(gn_smem);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) gn_share(a.st, slots, blockIdx.x, gridDim.x, sm);
+  __syncthreads();
+  const int rank = sm.rank, size = sm.size;
+  GNState& S = sm.S;
+  for (int obj = sm.obj; obj < slots.n; obj += size == 1 ? (int)gridDim.x : slots.n) {
+    const int s = slots.v[obj];
+    __syncthreads();
+    gn_copy_state(a.st + s, &S);
+    __syncthreads();
+    if (g.only < 0 && warp == 0) {
+      // setup_object_post: the start pose inverse(T_w_c2) T_w_o1
+      float* c2 = reinterpret_cast<float*>(&S.T_w_c2);
+      float* tmp = reinterpret_cast<float*>(&sm.M);
+      if (lane < 16) c2[lane] = Twc2[lane];
+      __syncwarp();
+      const float ie = inverse_warp(c2, lane);
+      if (lane < 16) tmp[lane] = ie;
+      __syncwarp();
+      const float t0 = mul_warp(tmp, reinterpret_cast<const float*>(&S.T_w_o1), lane);
+      float* Tf = reinterpret_cast<float*>(&S.Tf);
+      if (lane < 16) {
+        Tf[lane] = t0;
+        reinterpret_cast<float*>(&S.evalTf)[lane] = t0;
+        S.T[lane] = S.prevT[lane] = (double)t0;
+      }
+      __syncwarp();
+      const float it0 = inverse_warp(Tf, lane);
+      if (lane < 16) reinterpret_cast<float*>(&S.invTf)[lane] = it0;
+    }
+    unsigned* bar = g.bar + s;
+    unsigned target = 0;
+    int par = 0;
+    for (int L = g.only >= 0 ? g.only : g.levels - 1; L >= (g.only >= 0 ? g.only : 0); --L) {
+      if (threadIdx.x == 0) sm.lv = gn_view(a, L);
+      __syncthreads();
+      const GNView& lv = sm.lv;
+      const int n = lv.w * lv.h, ppt = gn_pix(L);
+      const int ntiles = (n + GN_THREADS * ppt - 1) / (GN_THREADS * ppt);
+      const int U = (ntiles - rank + size - 1) / size;   // this CTA's tiles: rank, rank + size, ...
+      const F3* rV = gn_ref_vertex(a, L, s);
+      int iters = 1;
+      if (g.only < 0) {
+#pragma unroll
+        for (int l = 0; l < MAX_PYR; ++l)
+          if (l == L) iters = g.iters[l];
+      }
+      for (int it = 0; it < iters; ++it) {
+        if (warp == 0) {
+          const float m = mul_warp(reinterpret_cast<const float*>(&S.T_c1_o1),
+                                   reinterpret_cast<const float*>(&S.invTf), lane);
+          // row i < 2: f_i times itself plus c_i times row 2
+          const float m2 = __shfl_sync(FULL_MASK, m, 8 + (lane & 3));
+          const int i = (lane >> 2) & 3;
+          const float mk = i == 0 ? a.k0.x * m + a.k0.z * m2
+                           : i == 1 ? a.k0.y * m + a.k0.w * m2 : m;
+          if (lane < 16) reinterpret_cast<float*>(&sm.M)[lane] = mk;
+          if (lane == 0) {
+            sm.origin = xform(S.Tf, get_translation(S.inv_T_w_o1));
+            sm.ifx = 1.f / lv.kL.x;
+            sm.ify = 1.f / lv.kL.y;
+          }
+        }
+        // this iteration's tile sums and live flags (alternating, so that a
+        // slow CTA still reads the last ones)
+        const size_t base = ((size_t)par * g.slots + s) * a.max_tiles;
+        double* rows = g.rows + base * 32;
+        uint8_t* lives = g.lives + base;
+        for (int u0 = 0; u0 < U; u0 += GO_CHUNK) {
+          const int nt = min(GO_CHUNK, U - u0);
+          if (threadIdx.x == 0) sm.ntask = 0;
+          __syncthreads();
+          if (threadIdx.x < nt * 8) sm.live[threadIdx.x] = 0;
+          __syncthreads();
+          for (int i = threadIdx.x; i < nt * 8 * ppt; i += GO_BLOCK) {
+            // segment k of task i / ppt
+            const int task = ppt == 1 ? i : i / GN_PIX_MAX, k = ppt == 1 ? 0 : i % GN_PIX_MAX;
+            const int t = rank + size * (u0 + (task >> 3));
+            const int p0 = (t * ppt + k) * GN_THREADS + (task & 7) * 32;
+            if (p0 < n && object_segment_live(a, sm, L, p0, n)) atomicOr(&sm.live[task], 1 << k);
+          }
+          __syncthreads();
+          if (threadIdx.x < nt * 8) {
+            const int live = sm.live[threadIdx.x];
+            int q = -1;
+            if (live) {
+              q = atomicAdd(&sm.ntask, 1);
+              sm.list[q] = threadIdx.x | live << 16;
+            }
+            sm.slot[threadIdx.x] = (short)q;
+          }
+          __syncthreads();
+          for (int q = warp; q < sm.ntask; q += GO_WARPS) {
+            const int task = sm.list[q] & 0xffff, live = sm.list[q] >> 16;
+            const int t = rank + size * (u0 + (task >> 3));
+            float acc[29];
+#pragma unroll
+            for (int i = 0; i < 29; ++i) acc[i] = 0.f;
+            int cnt[3] = {0, 0, 0};
+#pragma unroll 1
+            for (int k = 0; k < ppt; ++k) {
+              const int p = (t * ppt + k) * GN_THREADS + (task & 7) * 32 + lane;
+              if (!((live >> k) & 1) || p >= n) continue;
+              Row ri, rr;
+              gn_rows<1>(a, lv, S, rV, L, p, ri, rr);
+              if (a.use_icp) accumulate(acc, cnt, ri, a.robust);
+              if (a.use_rgb) accumulate(acc, cnt, rr, a.robust);
+            }
+            __syncwarp();
+            sm.ws[q][lane] = warp_sum_fp64(acc, cnt, sm.red[warp], lane);
+            __syncwarp();
+          }
+          __syncthreads();
+          for (int u = warp; u < nt; u += GO_WARPS) {
+            const int t = rank + size * (u0 + u);
+            double sum = 0;
+            int any = 0;
+#pragma unroll
+            for (int wi = 0; wi < 8; ++wi) {
+              const int q = sm.slot[8 * u + wi];
+              any |= q >= 0;
+              sum += q >= 0 ? sm.ws[q][lane] : 0.0;
+            }
+            if (any) __stcg(rows + (size_t)t * 32 + lane, sum);
+            if (lane == 0) __stcg(lives + t, (uint8_t)any);
+          }
+          __syncthreads();
+        }
+        if (threadIdx.x == 0) {
+          __threadfence();
+          atomicAdd(bar, 1u);
+          target += size;
+          sm.flag = gn_wait(bar, target, g.status);
+        }
+        __syncthreads();
+        if (sm.flag) return;
+        // column g by warps g and g + 8: 32 tiles of the column at a time, the
+        // live ones' sums fetched into ws, half of them by each warp, then
+        // added in order by warp g
+        {
+          const int g8 = warp & 7;
+          double v = 0;
+          for (int b0 = g8; b0 - g8 < ntiles; b0 += 8 * 32) {
+            const int t = b0 + 8 * lane;
+            const bool on = t < ntiles && __ldcg(lives + t) != 0;
+            const unsigned m = __ballot_sync(FULL_MASK, on);
+            const int cnt = __popc(m), mid = (cnt + 1) / 2;
+            const int q0 = warp < 8 ? 0 : mid, q1 = warp < 8 ? mid : cnt;
+            if (on) sm.pick[warp][__popc(m & ((1u << lane) - 1))] = t;
+            __syncwarp();
+            double c[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q)
+              if (q0 + q < q1)
+                c[q] = __ldcg(rows + (size_t)sm.pick[warp][q0 + q] * 32 + lane);
+#pragma unroll
+            for (int q = 0; q < 16; ++q)
+              if (q0 + q < q1) sm.ws[g8 * 32 + q0 + q][lane] = c[q];
+            __syncthreads();
+            if (warp < 8) {
+#pragma unroll 8
+              for (int q = 0; q < cnt; ++q) v += sm.ws[g8 * 32 + q][lane];
+            }
+            __syncthreads();
+          }
+          if (warp < 8) sm.sh[warp][lane] = v;
+        }
+        __syncthreads();
+        if (warp == 0) {
+          double t = 0;
+#pragma unroll
+          for (int q = 0; q < 8; ++q) t += sm.sh[q][lane];
+          sm.tot[lane] = t;
+          S.sums[L][lane] = t;
+          __syncwarp();
+          if (g.only < 0) gn_step_warp(&S, sm.tot, L, it == 0);
+        }
+        __syncthreads();
+        par ^= 1;
+        if (S.done && g.only < 0) break;
+      }
+    }
+    if (rank != 0) return;
+    if (g.only < 0 && warp == 0) {
+      // finalize_objects: the volume pose and the virtual camera pose
+      // (tracking.cpp:695-696); (float)T is the last Tf
+      float* Tco = reinterpret_cast<float*>(&S.Tf);
+      float* Tv = reinterpret_cast<float*>(&S.T_virtual);
+      float* tmp = reinterpret_cast<float*>(&sm.M);
+      float* pose = g.poses + 16 * s;
+      const float two = mul_warp(reinterpret_cast<const float*>(&S.T_w_c2), Tco, lane);
+      const float it = inverse_warp(Tco, lane);
+      if (lane < 16) {
+        pose[lane] = two;
+        tmp[lane] = it;
+      }
+      __syncwarp();
+      const float tv = mul_warp(reinterpret_cast<const float*>(&S.T_w_o1), tmp, lane);
+      if (lane < 16) Tv[lane] = tv;
     }
     __syncthreads();
-    if (s_flag != 0) return;
-    // the problems' done flags, one lane per problem
-    if (threadIdx.x < 32) {
-      int all = 1;
-      for (int i = threadIdx.x; i < slots.n; i += 32) all &= __ldcg(&a.st[slots.v[i]].done) != 0;
-      all = __all_sync(FULL_MASK, all);
-      if (threadIdx.x == 0) s_done = all;
-    }
-    __syncthreads();
-    if (s_done) return;
+    gn_copy_state(&S, a.st + s);
   }
 }
 
@@ -1329,20 +1950,31 @@ int track_init(Context* ctx) {
   for (int l = 0; l < ts->levels; ++l)
     ts->max_tiles = std::max(ts->max_tiles, div_up((long long)P.w[l] * P.h[l], GN_THREADS * gn_pix(l)));
   if (talloc(ctx, &ts->d_state, MAX_INSTANCES)) return MF_E_CUDA;
-  if (talloc(ctx, &ts->d_partials, (size_t)MAX_INSTANCES * ts->max_tiles * 32)) return MF_E_CUDA;
+  if (talloc(ctx, &ts->d_partials, (size_t)ts->max_tiles * 32)) return MF_E_CUDA;
   if (talloc(ctx, &ts->d_zr, (size_t)MAX_PYR * ts->max_tiles)) return MF_E_CUDA;
+  ts->max_segs = div_up((long long)ctx->W * ctx->H, 32);
+  if (talloc(ctx, &ts->d_zs, (size_t)MAX_PYR * ts->max_segs)) return MF_E_CUDA;
   if (talloc(ctx, &ts->d_Twc_prev, 16)) return MF_E_CUDA;
   if (talloc(ctx, &ts->d_mask0, (size_t)ctx->W * ctx->H)) return MF_E_CUDA;
-  if (talloc(ctx, &ts->d_gnbar, 2 * MAX_PYR)) return MF_E_CUDA;
-  // the persistent GN launch needs every CTA resident: its grid is at most
-  // the SM count times the CTAs one SM holds
+  if (talloc(ctx, &ts->d_gnbar, MAX_INSTANCES)) return MF_E_CUDA;
+  if (talloc(ctx, &ts->d_gnrows, 2 * GN_CAM_ROWS * 32)) return MF_E_CUDA;
+  if (talloc(ctx, &ts->d_objrows, (size_t)2 * ctx->cfg.max_instances * ts->max_tiles * 32)) return MF_E_CUDA;
+  if (talloc(ctx, &ts->d_objlive, (size_t)2 * ctx->cfg.max_instances * ts->max_tiles)) return MF_E_CUDA;
+  // the GN launches need every CTA resident: a grid is at most the SM count
+  // times the CTAs one SM holds
   {
-    int sms = 0, b0 = 0, b1 = 0;
+    int sms = 0, b = 0;
     MF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    MF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b0, gn_level_kernel<0>, GN_THREADS, 0));
-    MF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, gn_level_kernel<1>, GN_THREADS, 0));
-    ts->coop_blocks[0] = sms * b0;
-    ts->coop_blocks[1] = sms * b1;
+    MF_CUDA(cudaFuncSetAttribute(gn_camera_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(GNShared)));
+    MF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, gn_camera_kernel, GN_BLOCK,
+                                                          sizeof(GNShared)));
+    ts->coop_blocks = sms * b;
+    MF_CUDA(cudaFuncSetAttribute(gn_objects_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(GOShared)));
+    MF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, gn_objects_kernel, GO_BLOCK,
+                                                          sizeof(GOShared)));
+    ts->obj_blocks = sms * b;
   }
   // Tracking::Tracking, tracking.cpp:77-84: gaussian[i] = expf(-(x*x) / (2 delta^2)),
   // x = i - 2, delta = 4 (computed on the host exactly as the reference does).
@@ -1513,7 +2145,7 @@ static const void* sums_ptr(const TrackState& T, int slot, int L) {
   return (const char*)(T.d_state + slot) + offsetof(GNState, sums) + sizeof(double) * 32 * L;
 }
 
-static GNArgs make_args(Context* ctx, int L, int device_step) {
+static GNArgs make_args(Context* ctx) {
   TrackState& T = *ctx->track;
   GNArgs a;
   std::memset(&a, 0, sizeof(a));
@@ -1521,12 +2153,16 @@ static GNArgs make_args(Context* ctx, int L, int device_step) {
   a.cur = T.cur;
   a.W = ctx->W; a.H = ctx->H;
   a.mvertex = ctx->d_vertex; a.mnormal = ctx->d_normal; a.mlabel = ctx->d_label;
-  for (int s = 0; s < ctx->cfg.max_instances; ++s) a.rV[s] = T.rV[s][L];
+  for (int l = 0; l < T.levels; ++l) {
+    for (int s = 0; s < ctx->cfg.max_instances; ++s) a.rV[l][s] = T.rV[s][l];
+    a.kL[l] = kdiv(ctx->cfg, l);
+  }
   a.st = T.d_state;
   a.partials = T.d_partials;
   a.max_tiles = T.max_tiles;
   a.zr = T.d_zr;
-  a.kL = kdiv(ctx->cfg, L);
+  a.zs = T.d_zs;
+  a.max_segs = T.max_segs;
   a.k0 = kdiv(ctx->cfg, 0);
   // obtainErrorParameters (TUM branch, tracking.cpp:766-772) keeps sigma_bright
   // in a float member; trackRGB uses 1.0 / sigma_bright (double) as a float.
@@ -1535,7 +2171,6 @@ static GNArgs make_args(Context* ctx, int L, int device_step) {
   a.robust = ctx->cfg.robust_kernel;
   a.use_icp = ctx->cfg.use_icp;
   a.use_rgb = ctx->cfg.use_rgb;
-  a.device_step = device_step;
   return a;
 }
 
@@ -1546,86 +2181,80 @@ static int tile_depth_range(Context* ctx) {
   TrackState& T = *ctx->track;
   const int tiles = div_up((long long)T.pyr.w[0] * T.pyr.h[0], GN_THREADS * gn_pix(0));
   tile_depth_range_kernel<<<dim3(tiles, T.levels), GN_THREADS, 0, ctx->stream>>>(
-      T.pyr, T.cur, T.d_zr, T.max_tiles);
+      T.pyr, T.cur, T.d_zr, T.max_tiles, T.d_zs, T.max_segs);
   MF_CUDA(cudaGetLastError());
   return MF_OK;
 }
 
-// Coarse-to-fine GN of every problem in `slots`, all on the device
-// (trackLiveFrame :240-335 / trackEachObject :629-694): one cooperative
-// launch per level (gn_level_kernel), or, with gn_persistent off, one launch
-// per iteration (gn_iter_kernel); both give the same poses bit for bit.
-template <int KIND>
-static cudaError_t launch_gn_level(const GNArgs& a, const IdList& slots, int L, int iters,
-                                   int ntiles, unsigned* bar, int* status, int grid,
-                                   cudaStream_t stream) {
+// The camera's GN launch: the whole loop, or with `only` >= 0 one evaluation
+// of that level whose sums land in the problem's state (plain mode).
+static int launch_gn_camera(Context* ctx, const GNArgs& a, int only) {
+  TrackState& T = *ctx->track;
+  GNLoop g{};
+  g.levels = T.levels;
+  g.only = only;
+  g.rows = T.d_gnrows;
+  g.bar = T.d_gnbar;
+  g.status = ctx->d_status;
+  g.poses = ctx->d_Twc;
+  int rows = 1;
+  for (int L = 0; L < T.levels; ++L) {
+    g.iters[L] = ctx->cfg.gn_iterations[L];
+    rows = std::max(rows, std::min(div_up((long long)T.pyr.w[L] * T.pyr.h[L],
+                                          GN_THREADS * gn_pix(L)), GN_CAM_ROWS));
+  }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(GN_THREADS);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = stream;
+  cfg.gridDim = dim3(std::min(rows, T.coop_blocks));
+  cfg.blockDim = dim3(GN_BLOCK);
+  cfg.dynamicSmemBytes = sizeof(GNShared);
+  cfg.stream = ctx->stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, gn_level_kernel<KIND>, a, slots, L, iters, ntiles, bar,
-                            status);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, gn_camera_kernel, a, g);
+  if (e != cudaSuccess) {
+    ctx->last_error = std::string("camera GN launch: ") + cudaGetErrorString(e);
+    return MF_E_CUDA;
+  }
+  return MF_OK;
 }
 
-template <int KIND>
-static cudaError_t launch_gn_iter(const GNArgs& a, const IdList& slots, int L, int tiles,
-                                  bool overlap, cudaStream_t stream) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(tiles, slots.n);
-  cfg.blockDim = dim3(GN_THREADS);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = overlap ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, gn_iter_kernel<KIND>, a, slots, L);
-}
-
-static int gn_device(Context* ctx, const IdList& slots, int kind) {
+// The objects' GN launch, as launch_gn_camera: GO_CTAS CTAs per object while
+// the device has them, so that in a frame with few objects the background's
+// allocation and integration find SMs beside it.  Frame with three objects at
+// 640x480: 8 per object 1119 us, 16 1017, 24 980, 32 975, every SM 980; with
+// six at 1280x720: 3097, 2651, 2518, 2522, 2527.
+constexpr int GO_CTAS = 32;
+static int launch_gn_objects(Context* ctx, const GNArgs& a, const IdList& slots, int only) {
   TrackState& T = *ctx->track;
-  bool chained = false;
-  const bool persistent = ctx->gn_persistent && T.coop_blocks[kind] > 0;
-  unsigned* bar = T.d_gnbar + kind * MAX_PYR;
-  if (persistent) MF_CUDA(cudaMemsetAsync(bar, 0, sizeof(unsigned) * MAX_PYR, ctx->stream));
-  for (int L = T.levels - 1; L >= 0; --L) {
-    GNArgs a = make_args(ctx, L, 1);
-    const int tiles = div_up((long long)T.pyr.w[L] * T.pyr.h[L], GN_THREADS * gn_pix(L));
-    const int iters = ctx->cfg.gn_iterations[L];
-    if (persistent) {
-      if (iters <= 0) continue;
-      const int grid = std::min(tiles * slots.n, T.coop_blocks[kind]);
-      const cudaError_t e =
-          kind == 0 ? launch_gn_level<0>(a, slots, L, iters, tiles, bar + L, ctx->d_status, grid,
-                                         ctx->stream)
-                    : launch_gn_level<1>(a, slots, L, iters, tiles, bar + L, ctx->d_status, grid,
-                                         ctx->stream);
-      if (e != cudaSuccess) {
-        ctx->last_error = std::string("persistent GN launch: ") + cudaGetErrorString(e);
-        return MF_E_CUDA;
-      }
-      continue;
-    }
-    for (int it = 0; it < iters; ++it) {
-      a.first_iter = it == 0;  // the level's reset happens in its first iteration
-      // every launch but the first of the chain overlaps its predecessor, a
-      // GN launch (which writes only problem states and partials)
-      const bool overlap = chained;
-      chained = true;
-      const cudaError_t e = kind == 0 ? launch_gn_iter<0>(a, slots, L, tiles, overlap, ctx->stream)
-                                      : launch_gn_iter<1>(a, slots, L, tiles, overlap, ctx->stream);
-      if (e != cudaSuccess) {
-        ctx->last_error = std::string("GN launch: ") + cudaGetErrorString(e);
-        return MF_E_CUDA;
-      }
-    }
+  GNLoop g{};
+  g.levels = T.levels;
+  g.only = only;
+  g.rows = T.d_objrows;
+  g.lives = T.d_objlive;
+  g.slots = ctx->cfg.max_instances;
+  g.bar = T.d_gnbar;
+  g.status = ctx->d_status;
+  g.poses = ctx->d_Two;
+  for (int L = 0; L < T.levels; ++L) g.iters[L] = ctx->cfg.gn_iterations[L];
+  const int ctas = std::min(T.obj_blocks, GO_CTAS * slots.n);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(GO_BLOCK);
+  cfg.dynamicSmemBytes = sizeof(GOShared);
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e =
+      cudaLaunchKernelEx(&cfg, gn_objects_kernel, a, g, slots, (const float*)ctx->d_Twc);
+  if (e != cudaSuccess) {
+    ctx->last_error = std::string("object GN launch: ") + cudaGetErrorString(e);
+    return MF_E_CUDA;
   }
   return MF_OK;
 }
@@ -1645,14 +2274,16 @@ static int gn_host(Context* ctx, int slot) {
     S.prev_err = INFINITY;
     S.done = 0;
     S.ticket = 0;
-    const GNArgs a = make_args(ctx, L, 0);
-    const int tiles = div_up((long long)T.pyr.w[L] * T.pyr.h[L], GN_THREADS * gn_pix(L));
+    const GNArgs a = make_args(ctx);
     for (int it = 0; it < ctx->cfg.gn_iterations[L] && !S.done; ++it) {
       MF_CUDA(cudaMemcpyAsync(T.d_state + slot, &S, sizeof(GNState), cudaMemcpyHostToDevice,
                               ctx->stream));
-      if (S.kind == 0) gn_iter_kernel<0><<<dim3(tiles, 1), GN_THREADS, 0, ctx->stream>>>(a, one, L);
-      else gn_iter_kernel<1><<<dim3(tiles, 1), GN_THREADS, 0, ctx->stream>>>(a, one, L);
-      MF_CUDA(cudaGetLastError());
+      MF_CUDA(cudaMemsetAsync(T.d_gnbar + slot, 0, sizeof(unsigned), ctx->stream));
+      if (S.kind == 0) {
+        if (int rc = launch_gn_camera(ctx, a, L)) return rc;
+      } else {
+        if (int rc = launch_gn_objects(ctx, a, one, L)) return rc;
+      }
       MF_CUDA(cudaMemcpyAsync(S.sums[L], sums_ptr(T, slot, L), sizeof(double) * 32,
                               cudaMemcpyDeviceToHost, ctx->stream));
       MF_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1681,7 +2312,8 @@ int track_camera_pre(Context* ctx, int retrack) {
   T.tracked = true;
   T.slot_kind[0] = 0;
   setup_camera_kernel<<<1, 1, 0, ctx->stream>>>(T.d_state, ctx->d_Twc, T.d_Twc_prev,
-                                                F4{c.k[0], c.k[1], c.k[2], c.k[3]}, retrack);
+                                                F4{c.k[0], c.k[1], c.k[2], c.k[3]}, retrack,
+                                                T.d_gnbar);
   MF_CUDA(cudaGetLastError());
   IdList cam;
   cam.n = 1;
@@ -1701,14 +2333,8 @@ int track_camera_mask(Context* ctx, uint32_t moving) {
 
 int track_camera_gn(Context* ctx) {
   TrackState& T = *ctx->track;
-  IdList cam;
-  cam.n = 1;
-  cam.v[0] = 0;
-  if (ctx->cfg.batched) {
-    if (int rc = gn_device(ctx, cam, 0)) return rc;
-  } else {
-    if (int rc = gn_host(ctx, 0)) return rc;
-  }
+  if (ctx->cfg.batched) return launch_gn_camera(ctx, make_args(ctx), -1);
+  if (int rc = gn_host(ctx, 0)) return rc;
   finalize_camera_kernel<<<1, 1, 0, ctx->stream>>>(T.d_state, ctx->d_Twc);
   MF_CUDA(cudaGetLastError());
   return MF_OK;
@@ -1723,7 +2349,6 @@ int track_camera(Context* ctx, uint32_t moving, int retrack) {
 // Tracking::trackEachObject for every id (instance ids >= 1), against the
 // model maps of the last raycast, from the previous camera pose (saved by
 // track_camera) to the current one.
-static int track_objects_run(Context* ctx, const IdList& ids);
 
 // The parts of trackEachObject before its GN that need neither the freshly
 // tracked camera pose nor the live pyramid: the problems' setup from the
@@ -1734,47 +2359,31 @@ int track_objects_pre(Context* ctx, const IdList& ids) {
   if (ids.n == 0) return MF_OK;
   TrackState& T = *ctx->track;
   for (int i = 0; i < ids.n; ++i) T.slot_kind[ids.v[i]] = 1;
-  setup_objects_pre_kernel<<<1, 32, 0, ctx->stream>>>(T.d_state, ids, T.d_Twc_prev, ctx->d_Two,
-                                                      ctx->d_inst_label);
+  setup_objects_pre_kernel<<<1, 32, 0, ctx->stream>>>(T.d_state, T.d_gnbar, ids, T.d_Twc_prev,
+                                                      ctx->d_Two, ctx->d_inst_label);
   MF_CUDA(cudaGetLastError());
   return render_reference(ctx, ids);
 }
 
 // After track_objects_pre: the rest of the setup with the tracked camera pose,
-// then the GN.
+// the GN and its results (all three in the batched mode's one launch).
 int track_objects_gn(Context* ctx, const IdList& ids) {
   if (ids.n == 0) return MF_OK;
+  if (int rc = tile_depth_range(ctx)) return rc;
+  if (ctx->cfg.batched) return launch_gn_objects(ctx, make_args(ctx), ids, -1);
   TrackState& T = *ctx->track;
   setup_objects_post_kernel<<<1, 32, 0, ctx->stream>>>(T.d_state, ids, ctx->d_Twc);
   MF_CUDA(cudaGetLastError());
-  return track_objects_run(ctx, ids);
-}
-
-int track_objects(Context* ctx, const IdList& ids) {
-  if (int rc = track_init(ctx)) return rc;
-  if (ids.n == 0) return MF_OK;
-  TrackState& T = *ctx->track;
-  for (int i = 0; i < ids.n; ++i) T.slot_kind[ids.v[i]] = 1;
-  setup_objects_kernel<<<1, 32, 0, ctx->stream>>>(T.d_state, ids, ctx->d_Twc, T.d_Twc_prev,
-                                                  ctx->d_Two, ctx->d_inst_label);
-  MF_CUDA(cudaGetLastError());
-  if (int rc = render_reference(ctx, ids)) return rc;
-  return track_objects_run(ctx, ids);
-}
-
-// The objects' GN once their problems are set up and their references rendered.
-static int track_objects_run(Context* ctx, const IdList& ids) {
-  TrackState& T = *ctx->track;
-  if (int rc = tile_depth_range(ctx)) return rc;
-  if (ctx->cfg.batched) {
-    if (int rc = gn_device(ctx, ids, 1)) return rc;
-  } else {
-    for (int i = 0; i < ids.n; ++i)
-      if (int rc = gn_host(ctx, ids.v[i])) return rc;
-  }
+  for (int i = 0; i < ids.n; ++i)
+    if (int rc = gn_host(ctx, ids.v[i])) return rc;
   finalize_objects_kernel<<<1, 32, 0, ctx->stream>>>(T.d_state, ids, ctx->d_Two);
   MF_CUDA(cudaGetLastError());
   return MF_OK;
+}
+
+int track_objects(Context* ctx, const IdList& ids) {
+  if (int rc = track_objects_pre(ctx, ids)) return rc;
+  return track_objects_gn(ctx, ids);
 }
 
 bool track_has_ref(Context* ctx) { return ctx->track && ctx->track->have_ref; }
@@ -1824,12 +2433,12 @@ int track_eval(Context* ctx, int slot, int L, const float* pose16, double* sums)
   IdList one;
   one.n = 1;
   one.v[0] = slot;
-  const GNArgs a = make_args(ctx, L, 0);
+  const GNArgs a = make_args(ctx);
   const int tiles = div_up((long long)T.pyr.w[L] * T.pyr.h[L], GN_THREADS * gn_pix(L));
   if (S.kind == 1)
     if (int rc = tile_depth_range(ctx)) return rc;
-  if (S.kind == 0) gn_iter_kernel<0><<<dim3(tiles, 1), GN_THREADS, 0, ctx->stream>>>(a, one, L);
-  else gn_iter_kernel<1><<<dim3(tiles, 1), GN_THREADS, 0, ctx->stream>>>(a, one, L);
+  if (S.kind == 0) gn_eval_kernel<0><<<tiles, GN_THREADS, 0, ctx->stream>>>(a, slot, L);
+  else gn_eval_kernel<1><<<tiles, GN_THREADS, 0, ctx->stream>>>(a, slot, L);
   MF_CUDA(cudaGetLastError());
   MF_CUDA(cudaMemcpyAsync(sums, sums_ptr(T, slot, L), sizeof(double) * 32,
                           cudaMemcpyDeviceToHost, ctx->stream));
@@ -1854,15 +2463,19 @@ int profile_gn(Context* ctx, int reps, double* us, double* bytes) {
   S.done = 0;
   S.ticket = 0;
   MF_CUDA(cudaMemcpyAsync(T.d_state, &S, sizeof(GNState), cudaMemcpyHostToDevice, ctx->stream));
-  const GNArgs a = make_args(ctx, 0, 0);
+  const GNArgs a = make_args(ctx);
   const int tiles = div_up((long long)T.pyr.w[0] * T.pyr.h[0], GN_THREADS * gn_pix(0));
-  gn_iter_kernel<0><<<dim3(tiles, 1), GN_THREADS, 0, ctx->stream>>>(a, one, 0);  // warm
+  auto launch = [&]() -> int {
+    MF_CUDA(cudaMemsetAsync(T.d_gnbar, 0, sizeof(unsigned), ctx->stream));
+    return launch_gn_camera(ctx, a, 0);
+  };
+  if (int rc = launch()) return rc;  // warm
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   cudaEventRecord(e0, ctx->stream);
   for (int r = 0; r < reps; ++r)
-    gn_iter_kernel<0><<<dim3(tiles, 1), GN_THREADS, 0, ctx->stream>>>(a, one, 0);
+    if (int rc = launch()) return rc;
   cudaEventRecord(e1, ctx->stream);
   MF_CUDA(cudaEventSynchronize(e1));
   float ms = 0;
@@ -1941,15 +2554,15 @@ gn_eval_static_kernel(GNArgs a, int s, int L, int set_pose, M4 Tf, M4 invTf,
   double* out = reinterpret_cast<double*>(scratch + EVAL_SUMS_OFF);
   unsigned* ticket = reinterpret_cast<unsigned*>(scratch + EVAL_TICKET_OFF);
 
-  const int w = a.pyr.w[L], h = a.pyr.h[L];
-  const int n = w * h;
+  const GNView lv = gn_view(a, L);
+  const int w = lv.w, n = w * lv.h;
   // object problems: a tile that cannot hold a valid row skips its pixels
   bool live = true;
   if (KIND == 1) {
     __shared__ int s_live;
     if (threadIdx.x < 32) {
-      const bool lv = object_tile_live(a, S, L, blockIdx.x, w, n);
-      if (threadIdx.x == 0) s_live = lv ? 1 : 0;
+      const bool tl = object_tile_live(a, lv.kL, S, L, blockIdx.x, w, n);
+      if (threadIdx.x == 0) s_live = tl ? 1 : 0;
     }
     __syncthreads();
     live = s_live != 0;
@@ -1963,24 +2576,16 @@ gn_eval_static_kernel(GNArgs a, int s, int L, int set_pose, M4 Tf, M4 invTf,
 #pragma unroll
     for (int i = 0; i < 29; ++i) acc[i] = 0.f;
     int cnt[3] = {0, 0, 0};
-    const F3* rV = a.rV[s];
+    const F3* rV = gn_ref_vertex(a, L, s);
     const int ppt = gn_pix(L);
 #pragma unroll 1
     for (int k = 0; k < ppt; ++k) {
       const int p = blockIdx.x * (GN_THREADS * ppt) + k * GN_THREADS + threadIdx.x;
       if (p >= n) break;
-      Row r;
-      if (a.use_icp) {
-        r.result = 0;
-        if (KIND == 0) icp_camera(a, S, L, p, r);
-        else icp_object(a, S, L, p, r);
-        accumulate(acc, cnt, r, a.robust);
-      }
-      if (a.use_rgb) {
-        r.result = 0;
-        rgb_row(a, S, rV, L, p, w, h, r);
-        accumulate(acc, cnt, r, a.robust);
-      }
+      Row ri, rr;
+      gn_rows<KIND>(a, lv, S, rV, L, p, ri, rr);
+      if (a.use_icp) accumulate(acc, cnt, ri, a.robust);
+      if (a.use_rgb) accumulate(acc, cnt, rr, a.robust);
     }
     sh[warp][lane] = warp_sum_fp64(acc, cnt, red[warp], lane);
   } else {
@@ -2072,7 +2677,7 @@ int track_eval_static(Context* ctx, int slot, int L, const float* pose16, double
     std::memcpy(&Tf, pose16, 64);
     invTf = inverse(Tf);
   }
-  const GNArgs a = make_args(ctx, L, 0);
+  const GNArgs a = make_args(ctx);
   if (kind == 1)
     if (int rc = tile_depth_range(ctx)) return rc;
   // the ticket must be zero when the launch starts (the last CTA also resets it)
@@ -2250,10 +2855,10 @@ camera_cost_kernel(GNArgs a, CostOut c) {
     }
     // ---- photometric (rgb_row, camera, level 0)
     if (a.use_rgb) {
-      const F3 rv = a.rV[0][p];
+      const F3 rv = a.rV[0][0][p];
       const F3 rl = a.pyr.V[1 - a.cur][0][p];
       if (!(rv.z <= 0.f || rv.z == INVALIDF) && !(length(rv - rl) > 0.1f && rl.z > 0.f)) {
-        const M4 KL = camera_matrix(a.kL);
+        const M4 KL = camera_matrix(a.kL[0]);
         const F3 wv = xform(S.T_w_r, rv);
         const F3 lv = xform(S.invTf, wv);
         const F3 pr = rotate(KL, lv);
@@ -2289,7 +2894,7 @@ camera_cost_kernel(GNArgs a, CostOut c) {
           if (c.want_grad) {
             // rv = d K^-1 (x, y, 1), d = (T_w_r^-1 v_m).z
             const int x = p % w, y = p / w;
-            const F3 ray = rotate(inverse_camera_matrix(a.kL), mk3((float)x, (float)y, 1.f));
+            const F3 ray = rotate(inverse_camera_matrix(a.kL[0]), mk3((float)x, (float)y, 1.f));
             const float g_d = dot(rotate_t(g3, S.T_w_r), ray);
             atomic_add3(c.gV + 3 * (size_t)p, (de * g_d) * xyz(S.inv_T_w_r.r[2]));
           }
@@ -2390,7 +2995,7 @@ int camera_cost(Context* ctx, const float* T_live16, int want_grad, double* out8
   double* gV = want_grad ? T.d_gmodel : nullptr;
   double* gN = want_grad ? T.d_gmodel + 3 * WH : nullptr;
   if (want_grad) MF_CUDA(cudaMemsetAsync(T.d_gmodel, 0, sizeof(double) * 6 * WH, ctx->stream));
-  const GNArgs a = make_args(ctx, 0, 0);
+  const GNArgs a = make_args(ctx);
   camera_cost_kernel<<<nb, 256, 0, ctx->stream>>>(a, CostOut{T.d_cost_part, gV, gN, want_grad});
   cost_sum_kernel<<<1, 8 * COST_GROUPS, 0, ctx->stream>>>(T.d_cost_part, nb, T.d_cost);
   MF_CUDA(cudaGetLastError());
@@ -2715,33 +3320,23 @@ __global__ void row_codes_kernel(GNArgs a, int slot, int8_t* __restrict__ out,
   __syncthreads();
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
-    const float e = reinterpret_cast<const float*>(&S.evalTf)[lane & 15];
-    const float ie = inverse_warp(e, lane);
+    const float* eval = reinterpret_cast<const float*>(&S.evalTf);
+    const float ie = inverse_warp(eval, lane);
     if (lane < 16) {
-      reinterpret_cast<float*>(&S.Tf)[lane] = e;
+      reinterpret_cast<float*>(&S.Tf)[lane] = eval[lane];
       reinterpret_cast<float*>(&S.invTf)[lane] = ie;
     }
   }
   __syncthreads();
-  const int w = a.pyr.w[0], h = a.pyr.h[0], n = w * h;
+  const GNView lv = gn_view(a, 0);
+  const int n = lv.w * lv.h;
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
-  Row r;
-  int8_t ci = 0, cr = 0;
-  float ei = 0.f, er = 0.f;  // TrackData::error of rows with result 1
-  if (a.use_icp) {
-    r.result = 0;
-    if (S.kind == 0) icp_camera(a, S, 0, p, r);
-    else icp_object(a, S, 0, p, r);
-    ci = (int8_t)r.result;
-    if (ci == 1) ei = r.e;
-  }
-  if (a.use_rgb) {
-    r.result = 0;
-    rgb_row(a, S, a.rV[slot], 0, p, w, h, r);
-    cr = (int8_t)r.result;
-    if (cr == 1) er = r.e;
-  }
+  Row ri, rr;
+  if (S.kind == 0) gn_rows<0>(a, lv, S, a.rV[0][slot], 0, p, ri, rr);
+  else gn_rows<1>(a, lv, S, a.rV[0][slot], 0, p, ri, rr);
+  const int8_t ci = a.use_icp ? (int8_t)ri.result : 0, cr = a.use_rgb ? (int8_t)rr.result : 0;
+  const float ei = ci == 1 ? ri.e : 0.f, er = cr == 1 ? rr.e : 0.f;  // TrackData::error
   out[p] = ci;
   out[n + p] = cr;
   if (out_err) {
@@ -2756,7 +3351,7 @@ int track_results(Context* ctx, int slot, int8_t* d_out, float* d_err, float* po
     return MF_E_STATE;
   }
   const int n = ctx->W * ctx->H;
-  GNArgs a = make_args(ctx, 0, 0);
+  GNArgs a = make_args(ctx);
   row_codes_kernel<<<div_up(n, 256), 256, 0, ctx->stream>>>(a, slot, d_out, d_err);
   MF_CUDA(cudaGetLastError());
   if (pose_eval) {
