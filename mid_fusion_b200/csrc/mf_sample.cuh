@@ -20,7 +20,7 @@ __device__ __forceinline__ int memo_slot(const Volume& V, BlockMemo& m, int x, i
   const int key = (x >> 3) | ((y >> 3) << 10) | ((z >> 3) << 20);
   if (key != m.key) {
     m.key = key;
-    m.slot = V.block_tab[morton3(x >> 3, y >> 3, z >> 3)];
+    m.slot = V.block_tab[block_index(x >> 3, y >> 3, z >> 3)];
   }
   return m.slot;
 }
@@ -134,7 +134,7 @@ static __device__ __noinline__ F3 volume_grad_generic(const Pool& P, const Volum
     if ((tx == bx0 || tx == bx1) && (ty == by0 || ty == by1) && (tz == bz0 || tz == bz1))
       sl = slot8[(tx != bx0 ? 1 : 0) | (ty != by0 ? 2 : 0) | (tz != bz0 ? 4 : 0)];
     else  // only when the sample position itself lies outside the volume
-      sl = V.block_tab[morton3(tx, ty, tz)];
+      sl = V.block_tab[block_index(tx, ty, tz)];
     return sl < 0 ? 1.f : __ldg(P.tsdf + (size_t)sl * 512 + voxel_index(x, y, z));
   };
 #define G(X, Y, Z) g(X, Y, Z)
@@ -194,7 +194,7 @@ static __device__ __noinline__ F3 volume_grad(const Pool& P, const Volume& V, F3
   const int bx1 = cx[3] >> 3, by1 = cy[3] >> 3, bz1 = cz[3] >> 3;
 #pragma unroll
   for (int c = 0; c < 8; ++c)
-    st[c * stride] = V.block_tab[morton3((c & 1) ? bx1 : bx0, (c & 2) ? by1 : by0,
+    st[c * stride] = V.block_tab[block_index((c & 1) ? bx1 : bx0, (c & 2) ? by1 : by0,
                                          (c & 4) ? bz1 : bz0)];
   int sx[4], sy[4], sz[4], ox[4], oy[4], oz[4];
 #pragma unroll
