@@ -391,7 +391,7 @@ int mf_integrate(mf_context* ctx, const int* ids, int n) {
     IdList l;
     l.n = n;
     for (int i = 0; i < n; ++i) l.v[i] = ids[i];
-    if (int rc = stage_prepare(ctx, l)) return rc;
+    if (int rc = stage_prepare(ctx, l, true)) return rc;
     if (int rc = stage_alloc(ctx, l)) return rc;
     if (int rc = stage_integrate(ctx, l)) return rc;
   } else {
@@ -399,7 +399,7 @@ int mf_integrate(mf_context* ctx, const int* ids, int n) {
       IdList l;
       l.n = 1;
       l.v[0] = ids[i];
-      if (int rc = stage_prepare(ctx, l)) return rc;
+      if (int rc = stage_prepare(ctx, l, true)) return rc;
       if (int rc = stage_alloc(ctx, l)) return rc;
       if (int rc = stage_integrate(ctx, l)) return rc;
     }

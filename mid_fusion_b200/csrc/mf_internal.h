@@ -158,7 +158,8 @@ struct Context {
   } while (0)
 
 // kernels / stages implemented in the .cu files
-int stage_prepare(Context* ctx, const IdList& ids);
+// reset: zero the counters of an allocation and a visit list that follow
+int stage_prepare(Context* ctx, const IdList& ids, bool reset = false);
 int stage_alloc(Context* ctx, const IdList& ids);
 int stage_integrate(Context* ctx, const IdList& ids, int ctas = 0);
 int stage_raycast(Context* ctx, const IdList& ids, float epsilon);
@@ -256,7 +257,7 @@ void int_variant_describe(int v, char* buf, int cap);
 // integrate_blocks_kernel alone, on `pool` (the live pool or a scratch copy),
 // over the visit list of the last stage_integrate / visit_list
 int launch_integrate_blocks(Context* ctx, const Pool& pool, int variant, int ctas = 0);
-int build_visit_list(Context* ctx, uint32_t inst_mask);
+int build_visit_list(Context* ctx, uint32_t inst_mask, bool zeroed = false);
 // the autotuner (mf_tune.cu)
 int tune_variant_count(int stage);
 int autotune(Context* ctx, int reps, float* ray_us, float* int_us);

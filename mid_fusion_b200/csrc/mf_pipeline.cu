@@ -90,7 +90,7 @@ static int frame_overlapped(Context* ctx, bool gen, const IdList& all, const IdL
   ctx->stream = side;
   std::swap(ctx->d_visit, ctx->d_visit_side);
   std::swap(ctx->d_visit_count, ctx->d_visit_count_side);
-  if (!rc) rc = stage_prepare(ctx, bg);
+  if (!rc) rc = stage_prepare(ctx, bg, true);
   if (!rc) rc = stage_alloc(ctx, bg);
   if (!rc) rc = stage_integrate(ctx, bg, ctx->overlap_ctas > 0 ? ctx->overlap_ctas : 0);
   if (!rc && phased) rc = stage_raycast_hits(ctx, bg, 0, ctx->ray_epsilon);
@@ -102,7 +102,7 @@ static int frame_overlapped(Context* ctx, bool gen, const IdList& all, const IdL
   ok(cudaStreamWaitEvent(main, ctx->ev_obj, 0));
   if (!rc) rc = track_objects_gn(ctx, objs);
   ok(cudaStreamWaitEvent(main, ctx->ev_gen, 0));
-  if (!rc) rc = stage_prepare(ctx, objs);
+  if (!rc) rc = stage_prepare(ctx, objs, true);
   if (!rc) rc = stage_alloc(ctx, objs);
   if (!rc) rc = stage_integrate(ctx, objs);
   if (!rc && phased) rc = stage_raycast_hits(ctx, objs, 1, ctx->ray_epsilon);
@@ -145,7 +145,7 @@ static int frame_body(Context* ctx, bool track, bool labels) {
       if (int rc = track_objects(ctx, objs)) return rc;
   }
   if (ctx->cfg.batched) {
-    if (int rc = stage_prepare(ctx, all)) return rc;
+    if (int rc = stage_prepare(ctx, all, true)) return rc;
     if (int rc = stage_alloc(ctx, all)) return rc;
     if (int rc = stage_integrate(ctx, all)) return rc;
   } else {
@@ -153,7 +153,7 @@ static int frame_body(Context* ctx, bool track, bool labels) {
       IdList one;
       one.n = 1;
       one.v[0] = i;
-      if (int rc = stage_prepare(ctx, one)) return rc;
+      if (int rc = stage_prepare(ctx, one, true)) return rc;
       if (int rc = stage_alloc(ctx, one)) return rc;
       if (int rc = stage_integrate(ctx, one)) return rc;
     }
@@ -285,7 +285,7 @@ int process_frame_motion(Context* ctx, float thr, float moved, uint32_t* moving_
   all.n = n;
   for (int i = 0; i < n; ++i) all.v[i] = i;
   if (ctx->cfg.batched) {
-    if (int rc = stage_prepare(ctx, all)) return rc;
+    if (int rc = stage_prepare(ctx, all, true)) return rc;
     if (int rc = stage_alloc(ctx, all)) return rc;
     if (int rc = stage_integrate(ctx, all)) return rc;
   } else {
@@ -293,7 +293,7 @@ int process_frame_motion(Context* ctx, float thr, float moved, uint32_t* moving_
       IdList one;
       one.n = 1;
       one.v[0] = i;
-      if (int rc = stage_prepare(ctx, one)) return rc;
+      if (int rc = stage_prepare(ctx, one, true)) return rc;
       if (int rc = stage_alloc(ctx, one)) return rc;
       if (int rc = stage_integrate(ctx, one)) return rc;
     }

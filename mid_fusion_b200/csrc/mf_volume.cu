@@ -14,42 +14,79 @@
 #include <cstring>
 #include "mf_internal.h"
 #include "mf_sample.cuh"
+#include "mf_warp.cuh"
 
 namespace mf {
 
 // ------------------------------------------------------------------ prepare
 // Per-instance matrices every stage needs, computed from the device-resident
 // camera and volume poses with the reference's float operation order.
-__global__ void prepare_kernel(const float* __restrict__ Twc_p, const float* __restrict__ Two_p,
-                               const Volume* __restrict__ vols, InstFrame* __restrict__ out,
-                               F4 k, float mu, IdList ids,
-                               const unsigned long long* __restrict__ reserved,
-                               const int* __restrict__ labels) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ids.n) return;
-  const int i = ids.v[t];
-  const M4 T_w_c = load_m4(Twc_p), T_w_o = load_m4(Two_p + 16 * i);
-  const Volume V = vols[i];
-  InstFrame f;
-  f.T_w_o = T_w_o;
-  f.inv_T_w_o = inverse(T_w_o);
-  const M4 K = camera_matrix(k);
-  f.kPose = mul(T_w_c, inverse(K));
-  f.o_cam = xform(f.inv_T_w_o, get_translation(T_w_c));
+// One block per instance, one warp per inverse: the three 4x4 eliminations and
+// the products run on lanes, side by side (one thread per instance took 10 us
+// for them, on the frame's critical path; now 3).  `reset`: the allocation and
+// the visit list that follow start from zeroed counters (each memset node of a
+// frame's graph cost 4 us, two per instance).
+__global__ void __launch_bounds__(96)
+prepare_kernel(const float* __restrict__ Twc_p, const float* __restrict__ Two_p,
+               const Volume* __restrict__ vols, InstFrame* __restrict__ out, F4 k, float mu,
+               IdList ids, const unsigned long long* __restrict__ reserved,
+               const int* __restrict__ labels, int reset, int* __restrict__ visit_count) {
+  __shared__ InstFrame f;
+  __shared__ M4 A[3], I[3], iK;   // T_w_o, K, T_w_c; their inverses; K's closed-form inverse
+  const int i = ids.v[blockIdx.x];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const Volume& V = vols[i];
   const float vs = V.dim / V.size;
-  f.inv_voxel = 1 / vs;
-  f.band = 2 * mu;
-  f.num_steps = (int)ceilf(f.band * f.inv_voxel);
-  f.reserved = reserved[i];
-  f.Tcw = mul(inverse(T_w_c), T_w_o);
-  f.KTcw = mul(K, f.Tcw);
-  f.delta = rotate(f.Tcw, mk3(vs, 0, 0));
-  f.cam_delta = rotate(K, f.delta);
-  const M4 view = mul(T_w_c, inverse_camera_matrix(k));
-  f.view = view;
-  f.o_origin = xform(f.inv_T_w_o, get_translation(view));
-  f.label = labels[i];
-  out[i] = f;
+  auto at = [](M4& m) { return reinterpret_cast<float*>(&m); };
+  if (warp == 0 && lane < 16) at(A[0])[lane] = Two_p[16 * i + lane];
+  if (warp == 2 && lane < 16) at(A[2])[lane] = Twc_p[lane];
+  if (warp == 1 && lane == 0) {
+    A[1] = camera_matrix(k);
+    iK = inverse_camera_matrix(k);
+    f.inv_voxel = 1 / vs;
+    f.band = 2 * mu;
+    f.num_steps = (int)ceilf(f.band * f.inv_voxel);
+    f.reserved = reserved[i];
+    f.label = labels[i];
+    if (reset) {
+      *V.last_emit = 0;
+      *V.emit_total = 0;
+      if (blockIdx.x == 0) *visit_count = 0;
+    }
+  }
+  __syncthreads();
+  {
+    const float e = inverse_warp(at(A[warp]), lane);
+    if (lane < 16) at(I[warp])[lane] = e;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const float kp = mul_warp(at(A[2]), at(I[1]), lane);
+    if (lane < 16) {
+      at(f.T_w_o)[lane] = at(A[0])[lane];
+      at(f.inv_T_w_o)[lane] = at(I[0])[lane];
+      at(f.kPose)[lane] = kp;
+    }
+    if (lane == 0) f.o_cam = xform(I[0], get_translation(A[2]));
+  } else if (warp == 1) {
+    const float c = mul_warp(at(I[2]), at(A[0]), lane);
+    if (lane < 16) at(f.Tcw)[lane] = c;
+    __syncwarp();
+    const float kc = mul_warp(at(A[1]), at(f.Tcw), lane);
+    if (lane < 16) at(f.KTcw)[lane] = kc;
+    if (lane == 0) {
+      f.delta = rotate(f.Tcw, mk3(vs, 0, 0));
+      f.cam_delta = rotate(A[1], f.delta);
+    }
+  } else {
+    const float w = mul_warp(at(A[2]), at(iK), lane);
+    if (lane < 16) at(f.view)[lane] = w;
+    __syncwarp();
+    if (lane == 0) f.o_origin = xform(I[0], get_translation(f.view));
+  }
+  __syncthreads();
+  for (int w = threadIdx.x; w < (int)(sizeof(InstFrame) / 4); w += 96)
+    reinterpret_cast<int*>(out + i)[w] = reinterpret_cast<const int*>(&f)[w];
 }
 
 // ------------------------------------------------------------------ allocation
@@ -59,11 +96,22 @@ __global__ void prepare_kernel(const float* __restrict__ Twc_p, const float* __r
 // request count (runs of equal blocks along a ray are added at once).  The
 // emission order of the single-threaded reference (row, column, step) of the
 // thread's last emitted sample is folded into last_emit with atomicMax.
+// Bound by instruction issue.  Background 512^3 and three objects 256^3 at
+// 640x480, all four in one launch: 116 us with 64-bit indices and the slot
+// waited for on entry, 71 us with 32-bit ones and the slot looked at when the
+// block is left, now 46 (the objects' long rays launched first).
+constexpr int RUN_SHIFT = 27;                          // table indices are below 2^27
+constexpr uint32_t RUN_INDEX = (1u << RUN_SHIFT) - 1;
+// A step is half a voxel to a voxel long, so a run through a block (8 sqrt 3
+// voxels) has at most 29 samples, and 24 samples leave at most 3 * (24 / 8 + 1)
+// blocks, one more at the ray's end.
+constexpr int MARK_STEPS = 24, RUN_LIST = 14;
 __global__ void __launch_bounds__(256)
 alloc_mark_kernel(const float* __restrict__ depth, const float* __restrict__ masks, int W,
                   int H, const Volume* __restrict__ vols, const InstFrame* __restrict__ frames,
                   IdList ids, Pool pool) {
-  const int inst = ids.v[blockIdx.y];
+  // the objects' long rays first: the background's short ones fill the tail
+  const int inst = ids.v[gridDim.y - 1 - blockIdx.y];
   const Volume& V = vols[inst];
   const InstFrame& F = frames[inst];
   unsigned count = 0, last_order = 0, last_idx = 0;
@@ -75,7 +123,10 @@ alloc_mark_kernel(const float* __restrict__ depth, const float* __restrict__ mas
   __shared__ int s_pix[256];
   __shared__ float s_d[256];
   __shared__ int s_wn[8];
+  __shared__ uint32_t s_spread[512];   // spread3_10 of a block coordinate
+  __shared__ uint32_t s_list[RUN_LIST][256];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < (V.size >> 3); i += 256) s_spread[i] = spread3_10(i);
   {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const float dq = q < W * H ? depth[q] : 0.f;
@@ -97,50 +148,103 @@ alloc_mark_kernel(const float* __restrict__ depth, const float* __restrict__ mas
   const bool has_ray = (int)threadIdx.x < n_rays;
   const int p = has_ray ? s_pix[threadIdx.x] : 0;
   const float d = has_ray ? s_d[threadIdx.x] : 0.f;
-  // no early return: every lane reaches the warp reduction below
+  // no early return: every lane reaches the warp-wide steps below
+  const int32_t* __restrict__ tab = V.block_tab;   // not written by this kernel
+  uint32_t* __restrict__ req = V.req;
+  uint8_t* __restrict__ active = pool.active;
+  const float inv_voxel = F.inv_voxel, size_f = (float)(unsigned)V.size;
+  const int num_steps = F.num_steps;
+  F3 pos = mk3(0.f), step = mk3(0.f);
+  bool all_in = false;
   if (has_ray) {
     const unsigned x = p % W, y = p / W;
-    const float size_f = (float)(unsigned)V.size;
     const F3 w_vertex = xform(F.kPose, mk3((x + 0.5f) * d, (y + 0.5f) * d, d));
     const F3 o_vertex = xform(F.inv_T_w_o, w_vertex);
     const F3 direction = normalize(F.o_cam - o_vertex);
-    const F3 origin = o_vertex - (F.band * 0.5f) * direction;
-    const F3 step = (direction * F.band) / (float)F.num_steps;
-    F3 pos = origin;
-    int run_idx = -1, run_len = 0;
-    int cur_key = -1, cur_slot = -1;
-    uint32_t cur_bidx = 0;
-    for (int i = 0; i < F.num_steps; i++) {
-      // the reference floors pos / voxel and tests 0 <= floor < size; with an
-      // integer size that holds exactly when 0 <= pos / voxel < size, and there
-      // the truncating conversion is the floor (one conversion per axis
-      // instead of a floor and a conversion; NaN fails the test either way)
-      const float fx = pos.x * F.inv_voxel, fy = pos.y * F.inv_voxel, fz = pos.z * F.inv_voxel;
-      if (fx < size_f && fy < size_f && fz < size_f && fx >= 0 && fy >= 0 && fz >= 0) {
-        const I3 v{(int)fx, (int)fy, (int)fz};
-        const int key = (v.x >> 3) | ((v.y >> 3) << 10) | ((v.z >> 3) << 20);
-        if (key != cur_key) {  // a new block along the ray: look it up once
-          cur_key = key;
-          cur_bidx = (uint32_t)morton3(v.x >> 3, v.y >> 3, v.z >> 3);
-          cur_slot = V.block_tab[cur_bidx];
-          if (cur_slot >= 0) pool.active[cur_slot] = 1;
+    pos = o_vertex - (F.band * 0.5f) * direction;
+    step = (direction * F.band) / (float)num_steps;
+    // both ends at least two voxels inside: so is every sample (the sums'
+    // rounding stays far below a voxel over 4096 steps)
+    const F3 end = pos + (float)num_steps * step;
+    const float lo = 2.f, hi = size_f - 2.f;
+    auto inside = [&](F3 q) {
+      const float fx = q.x * inv_voxel, fy = q.y * inv_voxel, fz = q.z * inv_voxel;
+      return fx > lo && fx < hi && fy > lo && fy < hi && fz > lo && fz < hi;
+    };
+    all_in = num_steps <= 4096 && inside(pos) && inside(end);
+  }
+  // The march lists the blocks it leaves (samples << 27 | table index, in shared
+  // memory), MARK_STEPS samples at a time; the warp then looks the listed blocks
+  // up together.  A lookup inside the march made the warp wait for it at nearly
+  // every step, because some lane enters a block there.
+  uint32_t key = 0, bidx = 0;   // keys start at BIG_BITS
+  int run = 0, n_list = 0, order = 0;   // order: step of the next listed sample
+  // floor(f / 8) of 0 <= f < 4096 in the low bits: with rounding towards minus
+  // infinity the sum's last place is 8 (a truncating conversion runs at a
+  // quarter of the rate)
+  constexpr float BIG = 100663296.f;   // 2^26 + 2^25
+  constexpr uint32_t BIG_BITS = 0x4cc00000u;
+  auto sample = [&](int i, float fx, float fy, float fz) {
+    const uint32_t kx = __float_as_uint(__fadd_rd(fx, BIG)), ky = __float_as_uint(__fadd_rd(fy, BIG)),
+                   kz = __float_as_uint(__fadd_rd(fz, BIG));
+    const uint32_t k = kx + (ky << 10) + (kz << 20);
+    if (k != key) {
+      if (run) s_list[n_list++][threadIdx.x] = ((uint32_t)run << RUN_SHIFT) | bidx;
+      else order = i;
+      key = k;
+      bidx = s_spread[kx - BIG_BITS] | (s_spread[ky - BIG_BITS] << 1) |
+             (s_spread[kz - BIG_BITS] << 2);
+      run = 0;
+    }
+    ++run;
+  };
+  const int steps = __any_sync(0xffffffffu, has_ray) ? num_steps : 0;
+  for (int i0 = 0; i0 < steps; i0 += MARK_STEPS) {
+    const int i1 = min(i0 + MARK_STEPS, steps);
+    if (has_ray) {
+      if (all_in) {
+        for (int i = i0; i < i1; i++) {
+          sample(i, pos.x * inv_voxel, pos.y * inv_voxel, pos.z * inv_voxel);
+          pos = pos + step;
         }
-        if (cur_slot < 0) {
-          if ((int)cur_bidx == run_idx) {
-            ++run_len;
-          } else {
-            if (run_len) atomicAdd(&V.req[run_idx], (uint32_t)run_len);
-            run_idx = (int)cur_bidx;
-            run_len = 1;
-          }
-          ++count;
-          last_order = (unsigned)p * (unsigned)F.num_steps + (unsigned)i;
-          last_idx = cur_bidx;
+      } else {
+        for (int i = i0; i < i1; i++) {
+          // the reference floors pos / voxel and tests 0 <= floor < size; with an
+          // integer size that holds exactly when 0 <= pos / voxel < size (NaN
+          // fails the test either way).  The samples inside are consecutive:
+          // the positions are monotone along every axis.
+          const float fx = pos.x * inv_voxel, fy = pos.y * inv_voxel, fz = pos.z * inv_voxel;
+          if (fx < size_f && fy < size_f && fz < size_f && fx >= 0 && fy >= 0 && fz >= 0)
+            sample(i, fx, fy, fz);
+          pos = pos + step;
         }
       }
-      pos = pos + step;
+      if (i1 == steps && run)
+        s_list[n_list++][threadIdx.x] = ((uint32_t)run << RUN_SHIFT) | bidx;
     }
-    if (run_len) atomicAdd(&V.req[run_idx], (uint32_t)run_len);
+    const int n_max = __reduce_max_sync(0xffffffffu, n_list);
+    for (int e = 0; e < n_max; e += 4) {
+      uint32_t ent[4];
+      int slot[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        ent[u] = e + u < n_list ? s_list[e + u][threadIdx.x] : 0;   // 0: no samples
+        slot[u] = ent[u] ? __ldg(tab + (ent[u] & RUN_INDEX)) : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const uint32_t n = ent[u] >> RUN_SHIFT;
+        order += n;
+        if (ent[u] && slot[u] >= 0) active[slot[u]] = 1;
+        if (slot[u] < 0) {
+          last_idx = ent[u] & RUN_INDEX;
+          last_order = (unsigned)p * (unsigned)num_steps + (unsigned)(order - 1);
+          atomicAdd(&req[last_idx], n);
+          count += n;
+        }
+      }
+    }
+    n_list = 0;
   }
   // one emission-count and one last-emission atomic per warp
   unsigned long long last = count ? (((unsigned long long)last_order << 32) | last_idx) : 0ULL;
@@ -613,24 +717,24 @@ void volume_free(Instance& in) {
 }
 
 
-int stage_prepare(Context* ctx, const IdList& ids) {
+int stage_prepare(Context* ctx, const IdList& ids, bool reset) {
   if (ids.n == 0) return MF_OK;
   const mf_config& c = ctx->cfg;
-  prepare_kernel<<<1, 32, 0, ctx->stream>>>(ctx->d_Twc, ctx->d_Two, ctx->d_vols, ctx->d_frames,
-                                             F4{c.k[0], c.k[1], c.k[2], c.k[3]}, c.mu, ids,
-                                             ctx->d_reserved, ctx->d_inst_label);
+  prepare_kernel<<<ids.n, 96, 0, ctx->stream>>>(ctx->d_Twc, ctx->d_Two, ctx->d_vols, ctx->d_frames,
+                                                F4{c.k[0], c.k[1], c.k[2], c.k[3]}, c.mu, ids,
+                                                ctx->d_reserved, ctx->d_inst_label, reset,
+                                                ctx->d_visit_count);
   MF_CUDA(cudaGetLastError());
   return MF_OK;
 }
 
+// After stage_prepare(ids, reset = true).
 int stage_alloc(Context* ctx, const IdList& ids) {
   if (ids.n == 0) return MF_OK;
   const int WH = ctx->W * ctx->H;
   int max_tab = 0;
   for (int i = 0; i < ids.n; ++i) {
     const Volume& V = ctx->inst[ids.v[i]].vol;
-    MF_CUDA(cudaMemsetAsync(V.last_emit, 0, sizeof(unsigned long long), ctx->stream));
-    MF_CUDA(cudaMemsetAsync(V.emit_total, 0, sizeof(unsigned long long), ctx->stream));
     max_tab = std::max(max_tab, 1 << (3 * V.block_level));
   }
   alloc_mark_kernel<<<dim3(div_up(WH, 256), ids.n), 256, 0, ctx->stream>>>(
@@ -731,8 +835,9 @@ int launch_integrate_blocks(Context* ctx, const Pool& pool, int variant, int cta
 }
 
 // projective_functor::build_active_list over the instances in `inst_mask`.
-int build_visit_list(Context* ctx, uint32_t inst_mask) {
-  MF_CUDA(cudaMemsetAsync(ctx->d_visit_count, 0, sizeof(int), ctx->stream));
+// zeroed: stage_prepare has reset the list's counter.
+int build_visit_list(Context* ctx, uint32_t inst_mask, bool zeroed) {
+  if (!zeroed) MF_CUDA(cudaMemsetAsync(ctx->d_visit_count, 0, sizeof(int), ctx->stream));
   visit_list_kernel<<<div_up(ctx->pool.cap, 256), 256, 0, ctx->stream>>>(
       ctx->pool, ctx->d_vols, ctx->d_frames, inst_mask, ctx->W, ctx->H, ctx->d_visit,
       ctx->d_visit_count);
@@ -740,6 +845,7 @@ int build_visit_list(Context* ctx, uint32_t inst_mask) {
   return MF_OK;
 }
 
+// After stage_prepare(ids, reset = true).
 int stage_integrate(Context* ctx, const IdList& ids, int ctas) {
   if (ids.n == 0) return MF_OK;
   const mf_config& c = ctx->cfg;
@@ -749,7 +855,7 @@ int stage_integrate(Context* ctx, const IdList& ids, int ctas) {
     mask |= 1u << ids.v[i];
     max_nodes = std::max(max_nodes, ctx->inst[ids.v[i]].vol.n_nodes);
   }
-  if (int rc = build_visit_list(ctx, mask)) return rc;
+  if (int rc = build_visit_list(ctx, mask, true)) return rc;
   if (int rc = launch_integrate_blocks(ctx, ctx->pool, ctx->tune.integrate, ctas)) return rc;
   SdfArgs a{ctx->d_depth, ctx->d_rgb, ctx->d_masks, ctx->W, ctx->H, c.mu, (float)c.max_weight};
   const F4 k{c.k[0], c.k[1], c.k[2], c.k[3]};
