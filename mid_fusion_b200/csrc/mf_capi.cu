@@ -226,7 +226,7 @@ int mf_destroy(mf_context* ctx) {
                 ctx->d_visit_side, ctx->d_visit_count_side, ctx->d_depth, ctx->d_rgb8, ctx->d_rgb, ctx->d_grey, ctx->d_masks,
                 ctx->d_labels, ctx->d_vertex, ctx->d_normal, ctx->d_label, ctx->d_export,
                 ctx->d_render, ctx->d_render_small, ctx->d_rayhit, ctx->d_raytf,
-                ctx->d_mc_tris};
+                ctx->d_mc_tris, ctx->d_mesh};
   for (void* p : ps) if (p) cudaFree(p);
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->side) cudaStreamDestroy(ctx->side);

@@ -109,6 +109,8 @@ struct Context {
   F4* d_rayhit = nullptr;
   float2* d_raytf = nullptr;
   int8_t* d_mc_tris = nullptr;      // marching-cubes triangulation table (mf_mesh)
+  float* d_mesh = nullptr;          // triangles on their way to host memory (mf_mesh)
+  size_t mesh_bytes = 0;
 
   // staging
   float* h_pinned = nullptr;        // small pinned host staging area
