@@ -889,8 +889,8 @@ constexpr int ADJ_MAX_CP = 64;   // checkpoints: rays of up to 2048 samples
 
 // Scatters g * d f / d tsdf of the trilinear interpolation at `pos`
 // (volume_interp_m) and returns d f / d t along `dir`.
-__device__ float interp_adjoint(const Pool& P, const Volume& V, BlockMemo& m, F3 pos, F3 dir,
-                                float g, float* __restrict__ grad) {
+__device__ __noinline__ float interp_adjoint(const Pool& P, const Volume& V, F3 pos, F3 dir,
+                                             float g, float* __restrict__ grad) {
   const float inv = V.size / V.dim;
   const F3 pv = mk3(pos.x * inv, pos.y * inv, pos.z * inv);
   const F3 fl = floor3(pv);
@@ -898,15 +898,15 @@ __device__ float interp_adjoint(const Pool& P, const Volume& V, BlockMemo& m, F3
   const F3 f = mk3(pv.x - fl.x, pv.y - fl.y, pv.z - fl.z);
   const int lx = imx(base.x, 0), ly = imx(base.y, 0), lz = imx(base.z, 0);
   float dfx = 0.f, dfy = 0.f, dfz = 0.f;
+  Cube c;
+  cube_at(V, lx, ly, lz, c);
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const int x = lx + (i & 1), y = ly + ((i >> 1) & 1), z = lz + (i >> 2);
-    const int ts = memo_slot(V, m, x, y, z);
-    const float val = ts < 0 ? 1.f : __ldg(P.tsdf + (size_t)ts * 512 + voxel_index(x, y, z));
+    const int ts = c.slot[i];
+    const float val = ts < 0 ? 1.f : __ldg(P.tsdf + (size_t)ts * 512 + c.off[i]);
     const float wx = (i & 1) ? f.x : 1.f - f.x, wy = (i & 2) ? f.y : 1.f - f.y,
                 wz = (i & 4) ? f.z : 1.f - f.z;
-    if (ts >= 0 && g != 0.f)
-      atomicAdd(grad + (size_t)ts * 512 + voxel_index(x, y, z), g * wx * wy * wz);
+    if (ts >= 0 && g != 0.f) atomicAdd(grad + (size_t)ts * 512 + c.off[i], g * wx * wy * wz);
     dfx += val * ((i & 1) ? 1.f : -1.f) * wy * wz;
     dfy += val * ((i & 2) ? 1.f : -1.f) * wx * wz;
     dfz += val * ((i & 4) ? 1.f : -1.f) * wx * wy;
@@ -922,7 +922,7 @@ __device__ float sample_adjoint(const Pool& P, const Volume& V, BlockMemo& m, F3
   const I3 s = to_i3(mk3(pos.x * inv, pos.y * inv, pos.z * inv));
   const int sl = memo_slot(V, m, s.x, s.y, s.z);
   const float fv = sl < 0 ? 1.f : __ldg(P.tsdf + (size_t)sl * 512 + voxel_index(s.x, s.y, s.z));
-  if (fv < 0.1f && fv >= -0.5f) return interp_adjoint(P, V, m, pos, dir, g, grad);
+  if (fv < 0.1f && fv >= -0.5f) return interp_adjoint(P, V, pos, dir, g, grad);
   if (sl >= 0 && g != 0.f) atomicAdd(grad + (size_t)sl * 512 + voxel_index(s.x, s.y, s.z), g);
   return 0.f;
 }
@@ -1015,7 +1015,7 @@ __device__ __noinline__ int march_adjoint(const Pool& P, const Volume& V, F3 ori
     }
   }
   if (k == 0)  // the opening interpolation was the secant's other end
-    (void)interp_adjoint(P, V, memo, p0, direction, g_a, grad);
+    (void)interp_adjoint(P, V, p0, direction, g_a, grad);
   return 1;
 }
 
@@ -1045,8 +1045,12 @@ __device__ F3 grad_adjoint(const Pool& P, const Volume& V, F3 pos_m, F3 gG,
   };
   const float wx[2] = {1.f - f.x, f.x}, wy[2] = {1.f - f.y, f.y}, wz[2] = {1.f - f.z, f.z};
   F3 gf = mk3(0.f);  // dE/d(fractional position)
+  // one body for the eight cells (unrolled it is 96 block lookups in a row)
+#pragma unroll 1
   for (int a = 0; a < 2; ++a)
+#pragma unroll 1
     for (int b = 0; b < 2; ++b)
+#pragma unroll 1
       for (int c = 0; c < 2; ++c) {
         const float w = wx[a] * wy[b] * wz[c];
         const float sx = a ? 1.f : -1.f, sy = b ? 1.f : -1.f, sz = c ? 1.f : -1.f;
@@ -1202,8 +1206,10 @@ __global__ void __launch_bounds__(128) render_volume_kernel(RenderArgs a) {
       const F3 o_origin = xform(F.inv_T_w_o, a.w_origin);
       const F3 o_dir = normalize(rotate(F.inv_T_w_o, w_dir));
       const float nfar = fmn(nearest, a.farPlane);
-      const float t_min = ray_first_block(V, o_origin, o_dir, a.nearPlane, nfar, a.epsilon,
-                                          a.status);
+      const float t_min =
+          ray_misses_blocks(V, V.bbox, o_origin, o_dir, a.nearPlane, nfar, a.epsilon)
+              ? -1.f
+              : ray_first_block(V, o_origin, o_dir, a.nearPlane, nfar, a.epsilon, a.status);
       const F4 hit = t_min > 0.f
                          ? raycast_volume(a.pool, V, o_origin, o_dir,
                                           t_min * V.dim / (unsigned)V.size, nfar, a.mu, step,
@@ -1250,8 +1256,7 @@ __global__ void __launch_bounds__(128) render_volume_kernel(RenderArgs a) {
     F3 rgb;
     if (a.render_color) {
       const Volume& V = a.vols[i];
-      rgb = mk3(volume_interp(a.pool, V, o_hit, 2), volume_interp(a.pool, V, o_hit, 3),
-                volume_interp(a.pool, V, o_hit, 4));
+      rgb = volume_interp_rgb(a.pool, V, o_hit);
     } else if (w_label == 0) {
       rgb = mk3(1.f);
     } else {
