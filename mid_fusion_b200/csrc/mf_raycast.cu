@@ -23,17 +23,19 @@ namespace mf {
 __device__ __noinline__ float ray_first_block(const Volume& V, F3 origin, F3 direction,
                                               float nearPlane,
                                  float farPlane, float epsilon, int* status) {
-  int st_m[MAX_LEVELS];
-  float st_t[MAX_LEVELS];
-  int st_l[MAX_LEVELS];
+  // the entry of level l: the node's Morton index and t_max there
+  struct alignas(8) Entry { int m; float t; } st[MAX_LEVELS];
 #pragma unroll
-  for (int i = 0; i < MAX_LEVELS; ++i) { st_m[i] = 0; st_t[i] = 0.f; st_l[i] = 0; }
+  for (int i = 0; i < MAX_LEVELS; ++i) st[i] = Entry{0, 0.f};
+  const int32_t* __restrict__ block_tab = V.block_tab;
+  const uint8_t* __restrict__ node_tab = V.node_tab;
+  const int block_level = V.block_level;
   F3 pos = mk3(1.f, 1.f, 1.f);
   int idx = 0;
   int p_level = 0, p_m = 0;  // parent: the root
   float scale_exp2 = 0.5f;
   int scale = CAST_STACK_DEPTH - 1;
-  const int min_scale = CAST_STACK_DEPTH - V.block_level;
+  const int min_scale = CAST_STACK_DEPTH - block_level;
   const float voxelSize = V.dim / V.size;
   F3 d;
   d.x = fabsf(direction.x) < epsilon ? copysignf(epsilon, direction.x) : direction.x;
@@ -63,8 +65,9 @@ __device__ __noinline__ float ray_first_block(const Volume& V, F3 origin, F3 dir
     const int ci = idx ^ octant_mask ^ 7;
     const int c_m = p_m * 8 + ci;
     bool has_child;
-    if (p_level + 1 == V.block_level) has_child = V.block_tab[c_m] >= 0;
-    else has_child = V.node_tab[V.node_off[p_level + 1] + c_m] != 0;
+    // node_off of level l is 8 + 8^2 + ... + 8^(l - 1): a bit every third place
+    if (p_level + 1 == block_level) has_child = __ldg(block_tab + c_m) >= 0;
+    else has_child = __ldg(node_tab + (0x49249248u & ((1u << (3 * p_level + 3)) - 1u)) + c_m) != 0;
     if (scale == min_scale && has_child) {
       return t_min * V.dim / voxelSize;
     } else if (has_child && t_min <= t_max) {  // descend
@@ -73,7 +76,7 @@ __device__ __noinline__ float ray_first_block(const Volume& V, F3 origin, F3 dir
       const F3 t_center = half * t_coef + t_corner;
       if (tc_max < h) {
         const int si = CAST_STACK_DEPTH - 1 - scale;  // = parent level
-        st_m[si] = p_m; st_l[si] = p_level; st_t[si] = t_max;
+        st[si] = Entry{p_m, t_max};
       }
       h = tc_max;
       p_level += 1;
@@ -104,11 +107,11 @@ __device__ __noinline__ float ray_first_block(const Volume& V, F3 origin, F3 dir
       scale_exp2 = __int_as_float((scale - CAST_STACK_DEPTH + 127) << 23);
       if (scale >= CAST_STACK_DEPTH) return -1.f;  // left the root: no block on the ray
       const int si = CAST_STACK_DEPTH - 1 - scale;
-      if (si < 0 || si >= V.block_level) {
+      if (si < 0 || si >= block_level) {
         atomicOr(status, ST_RAY_GUARD);
         return -1.f;
       }
-      p_m = st_m[si]; p_level = st_l[si]; t_max = st_t[si];
+      p_m = st[si].m; p_level = si; t_max = st[si].t;
       const int shx = __float_as_int(pos.x) >> scale;
       const int shy = __float_as_int(pos.y) >> scale;
       const int shz = __float_as_int(pos.z) >> scale;
@@ -141,9 +144,11 @@ __device__ __forceinline__ bool ray_misses_blocks(const Volume& V, const int* bo
   // the volume cube is [0, 1]^3 and t runs along d in these units
   const float vn = 1.f / (float)V.size;
   const float mg = 2.f * vn;
-  const F3 o = origin / V.dim;
-  const F3 inv = mk3(1.f / d.x, 1.f / d.y, 1.f / d.z);
-  const float t0 = nearPlane / V.dim - mg, t1 = farPlane / V.dim + mg;
+  // (approximate quotients: their error is far below the margins too)
+  const float idim = __fdividef(1.f, V.dim);
+  const F3 o = origin * idim;
+  const F3 inv = mk3(__fdividef(1.f, d.x), __fdividef(1.f, d.y), __fdividef(1.f, d.z));
+  const float t0 = nearPlane * idim - mg, t1 = farPlane * idim + mg;
   auto hits = [&](float lx, float ly, float lz, float hx, float hy, float hz) {
     const float ax = (lx - o.x) * inv.x, bx = (hx - o.x) * inv.x;
     const float ay = (ly - o.y) * inv.y, by = (hy - o.y) * inv.y;
@@ -178,20 +183,36 @@ __device__ __noinline__ F4 raycast_volume(const Pool& P, const Volume& V, F3 ori
   const float tnear = fmx(largest_tmin, nearPlane);
   const float tfar = fmn(smallest_tmax, farPlane);
   const float inv = V.size / V.dim;
+  const float* __restrict__ tsdf = P.tsdf;
+  const int32_t* __restrict__ tab = V.block_tab;
+  const unsigned size = (unsigned)V.size;
   if (tnear < tfar) {
-    BlockMemo memo;
+    int key = -1, slot = -1;   // the last sample's block (BlockMemo, in registers)
     float t = tnear, stepsize = largestep;
     F3 position = origin + direction * t;
-    float f_t = volume_interp_m<0>(P, V, position, memo), f_tt = 0;
+    float f_t = interp_tsdf(tsdf, tab, size,
+                            mk3(position.x * inv, position.y * inv, position.z * inv), -1, -1, -1,
+                            -1), f_tt = 0;
     if (f_t > 0) {
       // (guarded: a valid march takes at most (far - near) / step steps)
       for (int guard = 0; t < tfar && guard < (1 << 20); t += stepsize, ++guard) {
         // Volume::get -> get_fine at the truncated voxel (volume_template.hpp:83-88);
         // the weight test data.y < 0 can never hold for SDF voxels.
-        const I3 s = to_i3(mk3(position.x * inv, position.y * inv, position.z * inv));
-        f_tt = tsdf_at_m(P, V, memo, s.x, s.y, s.z);
+        const F3 pv = mk3(position.x * inv, position.y * inv, position.z * inv);
+        const I3 s = to_i3(pv);
+        int cur = -1;
+        if ((unsigned)s.x < size && (unsigned)s.y < size && (unsigned)s.z < size) {
+          const int k = (s.x >> 3) | ((s.y >> 3) << 10) | ((s.z >> 3) << 20);
+          if (k != key) {
+            key = k;
+            slot = __ldg(tab + block_index(s.x >> 3, s.y >> 3, s.z >> 3));
+          }
+          cur = slot;
+        }
+        f_tt = cur < 0 ? 1.f : __ldg(tsdf + (size_t)cur * 512 + voxel_index(s.x, s.y, s.z));
         // f_tt <= 0.1 compares in double; for a float that is f_tt < 0.1f.
-        if (f_tt < 0.1f && f_tt >= -0.5f) f_tt = volume_interp_m<0>(P, V, position, memo);
+        if (f_tt < 0.1f && f_tt >= -0.5f)
+          f_tt = interp_tsdf(tsdf, tab, size, pv, s.x, s.y, s.z, cur);
         if (f_tt < 0) break;
         stepsize = fmx(f_tt * mu, step);
         position = position + stepsize * direction;
@@ -220,7 +241,7 @@ struct RayArgs {
 // each pixel alike, so the autotuner may pick any of them (ray_variants).
 template <int TW, int MINB>
 __global__ void __launch_bounds__(128, MINB)
-raycast_objects_kernel(Pool pool, const Volume* __restrict__ vols,
+raycast_objects_kernel(const __grid_constant__ Pool pool, const Volume* __restrict__ vols,
                        const InstFrame* __restrict__ frames, IdList ids, RayArgs a,
                        int* __restrict__ status) {
   const int x = blockIdx.x * TW + (threadIdx.x % TW);
@@ -316,7 +337,7 @@ struct RayRec {
 
 template <int TW>
 __global__ void __launch_bounds__(128)
-raycast_hits_kernel(Pool pool, const Volume* __restrict__ vols,
+raycast_hits_kernel(const __grid_constant__ Pool pool, const Volume* __restrict__ vols,
                     const InstFrame* __restrict__ frames, IdList ids, RayArgs a, RayRec rec,
                     int rec_base, int* __restrict__ status) {
   const int x = blockIdx.x * TW + (threadIdx.x % TW);
@@ -349,7 +370,7 @@ raycast_hits_kernel(Pool pool, const Volume* __restrict__ vols,
 
 template <int TW>
 __global__ void __launch_bounds__(128)
-raycast_fold_kernel(Pool pool, const Volume* __restrict__ vols,
+raycast_fold_kernel(const __grid_constant__ Pool pool, const Volume* __restrict__ vols,
                     const InstFrame* __restrict__ frames, IdList ids, RayArgs a, RayRec rec) {
   const int x = blockIdx.x * TW + (threadIdx.x % TW);
   const int y = blockIdx.y * (128 / TW) + (threadIdx.x / TW);
@@ -438,7 +459,7 @@ raycast_fold_kernel(Pool pool, const Volume* __restrict__ vols,
 // phased path's records, with the world normal of every crossing computed by
 // the GPU that holds the volume, so that the fold needs no volume.
 __global__ void __launch_bounds__(128)
-raycast_records_kernel(Pool pool, const Volume* __restrict__ vols,
+raycast_records_kernel(const __grid_constant__ Pool pool, const Volume* __restrict__ vols,
                        const InstFrame* __restrict__ frames, IdList ids, M4 view, RayArgs a,
                        mf_ray_record* __restrict__ rec, int* __restrict__ status) {
   __shared__ int s_slot[8 * 128];
@@ -483,7 +504,7 @@ raycast_records_kernel(Pool pool, const Volume* __restrict__ vols,
 }
 
 // foreground and world normal of each listed instance at the zero hit
-__global__ void raycast_origins_kernel(Pool pool, const Volume* __restrict__ vols,
+__global__ void raycast_origins_kernel(const __grid_constant__ Pool pool, const Volume* __restrict__ vols,
                                        const InstFrame* __restrict__ frames, IdList ids,
                                        mf_ray_origin* __restrict__ out) {
   __shared__ int s_slot[8 * 32];
@@ -673,7 +694,7 @@ __device__ __noinline__ void march_count(const Pool& P, const Volume& V, F3 orig
   cnt[1] += interps;
 }
 
-__global__ void raycast_count_kernel(Pool pool, const Volume* __restrict__ vols,
+__global__ void raycast_count_kernel(const __grid_constant__ Pool pool, const Volume* __restrict__ vols,
                                      const InstFrame* __restrict__ frames, IdList ids, RayArgs a,
                                      int* __restrict__ status,
                                      unsigned long long* __restrict__ totals) {
@@ -1070,7 +1091,7 @@ __device__ F3 grad_adjoint(const Pool& P, const Volume& V, F3 pos_m, F3 gG,
 
 // One thread per model pixel; pixels whose map adjoints are zero return.
 __global__ void __launch_bounds__(128)
-raycast_adjoint_kernel(Pool pool, const Volume* __restrict__ vols,
+raycast_adjoint_kernel(const __grid_constant__ Pool pool, const Volume* __restrict__ vols,
                        const InstFrame* __restrict__ frames, IdList ids, RayArgs a,
                        const double* __restrict__ gV, const double* __restrict__ gN,
                        float* __restrict__ grad, int* __restrict__ status) {
@@ -1185,7 +1206,7 @@ struct RenderArgs {
 // composite hit is found again with this function's own rules (the tie and
 // the zero-gradient cases differ from raycastObjectList); otherwise the maps
 // of the last raycast are shaded.
-__global__ void __launch_bounds__(128) render_volume_kernel(RenderArgs a) {
+__global__ void __launch_bounds__(128) render_volume_kernel(const __grid_constant__ RenderArgs a) {
   const int x = blockIdx.x * 16 + (threadIdx.x & 15);
   const int y = blockIdx.y * 8 + (threadIdx.x >> 4);
   if (x >= a.W || y >= a.H) return;

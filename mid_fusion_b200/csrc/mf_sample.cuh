@@ -54,9 +54,8 @@ __device__ __forceinline__ float tap_val(const Pool& P, int slot, int v) {
 struct Cube {
   int slot[8], off[8];
 };
-__device__ __forceinline__ void cube_at(const Volume& V, int x, int y, int z, Cube& c) {
-  const unsigned n = (unsigned)V.size;
-  const int32_t* __restrict__ tab = V.block_tab;
+__device__ __forceinline__ void cube_at(const int32_t* __restrict__ tab, unsigned n, int x, int y,
+                                        int z, Cube& c) {
   uint32_t sx[2], sy[2], sz[2];
   bool ix[2], iy[2], iz[2];
 #pragma unroll
@@ -75,6 +74,10 @@ __device__ __forceinline__ void cube_at(const Volume& V, int x, int y, int z, Cu
     c.slot[i] = in ? __ldg(tab + (sx[a] | sy[b] | sz[d])) : -1;
     c.off[i] = voxel_index(x + a, y + b, z + d);
   }
+}
+
+__device__ __forceinline__ void cube_at(const Volume& V, int x, int y, int z, Cube& c) {
+  cube_at(V.block_tab, (unsigned)V.size, x, y, z, c);
 }
 
 __device__ __forceinline__ float trilinear(const float* p, F3 f) {
@@ -106,6 +109,38 @@ __device__ __noinline__ float volume_interp_m(const Pool& P, const Volume& V, F3
     cube_at(V, lx, ly, lz, c);
 #pragma unroll
     for (int i = 0; i < 8; ++i) p[i] = tap_val<FIELD>(P, c.slot[i], c.off[i]);
+  }
+  return trilinear(p, f);
+}
+
+// The TSDF (field 0) at voxel position pos, for the march: the volume's
+// pointers by value, and the slot of the block that holds the march's last
+// sample (`hint`, at voxel (hx, hy, hz)), so that nothing of the caller's
+// loop has to live in memory.
+static __device__ __noinline__ float interp_tsdf(const float* __restrict__ tsdf,
+                                                 const int32_t* __restrict__ tab, unsigned size,
+                                                 F3 pos, int hx, int hy, int hz, int hint) {
+  const F3 fl = floor3(pos);
+  const I3 base = to_i3(fl);
+  const F3 f = mk3(pos.x - fl.x, pos.y - fl.y, pos.z - fl.z);
+  const int lx = imx(base.x, 0), ly = imx(base.y, 0), lz = imx(base.z, 0);
+  float p[8];
+  if ((lx & 7) != 7 && (ly & 7) != 7 && (lz & 7) != 7) {
+    int slot = hint;
+    if (lx != hx || ly != hy || lz != hz)
+      slot = (unsigned)lx < size && (unsigned)ly < size && (unsigned)lz < size
+                 ? __ldg(tab + block_index(lx >> 3, ly >> 3, lz >> 3)) : -1;
+    const int v0 = voxel_index(lx, ly, lz);
+    const float* q = tsdf + (size_t)slot * 512 + v0;
+    constexpr int off[8] = {0, 1, 8, 9, 64, 65, 72, 73};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) p[i] = slot < 0 ? 1.f : __ldg(q + off[i]);
+  } else {
+    Cube c;
+    cube_at(tab, size, lx, ly, lz, c);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      p[i] = c.slot[i] < 0 ? 1.f : __ldg(tsdf + (size_t)c.slot[i] * 512 + c.off[i]);
   }
   return trilinear(p, f);
 }
