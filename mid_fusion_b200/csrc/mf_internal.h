@@ -169,8 +169,9 @@ bool raycast_is_phased(const Context* ctx);
 int stage_raycast_hits(Context* ctx, const IdList& ids, int base, float epsilon);
 int stage_raycast_fold(Context* ctx, const IdList& ids, float epsilon);
 // The same raycast into other map buffers.
+// win, win_hit: also each pixel's winner (list position + 1) and its hit.
 int stage_raycast_to(Context* ctx, const IdList& ids, float epsilon, F3* vertex, F3* normal,
-                     int* label);
+                     int* label, uint8_t* win = nullptr, F4* win_hit = nullptr);
 int alloc_keys(Context* ctx, int id, const uint64_t* keys, int n);
 int export_blocks(Context* ctx, int id, uint64_t* keys, int32_t* coords, uint8_t* active,
                   void* voxels, int cap, int* n);
@@ -236,8 +237,8 @@ int render_track(Context* ctx, int mode, const int8_t* d_res, const float* d_err
 int render_mask(Context* ctx, int mode, const int32_t* d_labels, const uint8_t* colors,
                 int n_colors, const int8_t* const* d_rows, int n_rows, uint8_t* out);
 int refine_mask_use_motion(Context* ctx, int id, const int8_t* d_res, int use_icp, int use_rgb);
-int stage_raycast_adjoint(Context* ctx, const IdList& ids, const double* gV, const double* gN,
-                          float* d_grad);
+int stage_raycast_adjoint(Context* ctx, const IdList& ids, uint8_t* win, F4* win_hit,
+                          const double* gV, const double* gN, float* d_grad);
 int track_download_level(Context* ctx, int L, int which, float* out);
 void track_save_prev_camera(Context* ctx);
 bool track_has_ref(Context* ctx);

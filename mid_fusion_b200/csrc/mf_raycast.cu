@@ -163,6 +163,43 @@ __device__ __forceinline__ bool ray_misses_blocks(const Volume& V, const int* bo
                (box[4] + 8) * vn + mg, (box[5] + 8) * vn + mg);
 }
 
+// One sample of the march: Volume::get -> get_fine at the truncated voxel
+// (volume_template.hpp:83-88; the weight test data.y < 0 can never hold for
+// SDF voxels), or the interpolation where that value lies in [-0.5, 0.1).
+// (f <= 0.1 compares in double; for a float that is f < 0.1f.)  The last
+// sample's block stays in registers.
+struct MarchVolume {
+  const float* __restrict__ tsdf;
+  const int32_t* __restrict__ tab;
+  unsigned size;
+  float inv;   // voxels per metre
+};
+struct MarchMemo { int key = -1, slot = -1; };
+__device__ __forceinline__ MarchVolume march_volume(const Pool& P, const Volume& V) {
+  return MarchVolume{P.tsdf, V.block_tab, (unsigned)V.size, V.size / V.dim};
+}
+__device__ __forceinline__ float march_sample(const MarchVolume& v, MarchMemo& m, F3 position) {
+  const F3 pv = mk3(position.x * v.inv, position.y * v.inv, position.z * v.inv);
+  const I3 s = to_i3(pv);
+  int cur = -1;
+  if ((unsigned)s.x < v.size && (unsigned)s.y < v.size && (unsigned)s.z < v.size) {
+    const int k = (s.x >> 3) | ((s.y >> 3) << 10) | ((s.z >> 3) << 20);
+    if (k != m.key) {
+      m.key = k;
+      m.slot = __ldg(v.tab + block_index(s.x >> 3, s.y >> 3, s.z >> 3));
+    }
+    cur = m.slot;
+  }
+  const float f = cur < 0 ? 1.f : __ldg(v.tsdf + (size_t)cur * 512 + voxel_index(s.x, s.y, s.z));
+  return f < 0.1f && f >= -0.5f ? interp_tsdf(v.tsdf, v.tab, v.size, pv, s.x, s.y, s.z, cur) : f;
+}
+// The interpolation that opens a march.
+__device__ __forceinline__ float march_open(const MarchVolume& v, F3 position) {
+  return interp_tsdf(v.tsdf, v.tab, v.size,
+                     mk3(position.x * v.inv, position.y * v.inv, position.z * v.inv), -1, -1, -1,
+                     -1);
+}
+
 // raycast(const Volume<SDF>&, origin, direction, ...),
 // apps/kfusion/src/cpp/kfusion/rendering_impl.hpp:80-140.  With TC, *tc gets
 // the march parameter t of the sample at which the crossing was found
@@ -182,37 +219,16 @@ __device__ __noinline__ F4 raycast_volume(const Pool& P, const Volume& V, F3 ori
   const float smallest_tmax = fmn(fmn(tmax.x, tmax.y), fmn(tmax.x, tmax.z));
   const float tnear = fmx(largest_tmin, nearPlane);
   const float tfar = fmn(smallest_tmax, farPlane);
-  const float inv = V.size / V.dim;
-  const float* __restrict__ tsdf = P.tsdf;
-  const int32_t* __restrict__ tab = V.block_tab;
-  const unsigned size = (unsigned)V.size;
+  const MarchVolume mv = march_volume(P, V);
   if (tnear < tfar) {
-    int key = -1, slot = -1;   // the last sample's block (BlockMemo, in registers)
+    MarchMemo memo;
     float t = tnear, stepsize = largestep;
     F3 position = origin + direction * t;
-    float f_t = interp_tsdf(tsdf, tab, size,
-                            mk3(position.x * inv, position.y * inv, position.z * inv), -1, -1, -1,
-                            -1), f_tt = 0;
+    float f_t = march_open(mv, position), f_tt = 0;
     if (f_t > 0) {
       // (guarded: a valid march takes at most (far - near) / step steps)
       for (int guard = 0; t < tfar && guard < (1 << 20); t += stepsize, ++guard) {
-        // Volume::get -> get_fine at the truncated voxel (volume_template.hpp:83-88);
-        // the weight test data.y < 0 can never hold for SDF voxels.
-        const F3 pv = mk3(position.x * inv, position.y * inv, position.z * inv);
-        const I3 s = to_i3(pv);
-        int cur = -1;
-        if ((unsigned)s.x < size && (unsigned)s.y < size && (unsigned)s.z < size) {
-          const int k = (s.x >> 3) | ((s.y >> 3) << 10) | ((s.z >> 3) << 20);
-          if (k != key) {
-            key = k;
-            slot = __ldg(tab + block_index(s.x >> 3, s.y >> 3, s.z >> 3));
-          }
-          cur = slot;
-        }
-        f_tt = cur < 0 ? 1.f : __ldg(tsdf + (size_t)cur * 512 + voxel_index(s.x, s.y, s.z));
-        // f_tt <= 0.1 compares in double; for a float that is f_tt < 0.1f.
-        if (f_tt < 0.1f && f_tt >= -0.5f)
-          f_tt = interp_tsdf(tsdf, tab, size, pv, s.x, s.y, s.z, cur);
+        f_tt = march_sample(mv, memo, position);
         if (f_tt < 0) break;
         stepsize = fmx(f_tt * mu, step);
         position = position + stepsize * direction;
@@ -233,6 +249,10 @@ struct RayArgs {
   F3* vertex; F3* normal; int* label;
   int W, H;
   float nearPlane, farPlane, mu, epsilon;
+  // for the adjoint (null otherwise): the winner's list position + 1 (0: none)
+  // and its hit (x, y, z, t) in its own frame
+  uint8_t* win = nullptr;
+  F4* win_hit = nullptr;
 };
 
 // One thread per pixel, instances in list order (the reference's object loop).
@@ -263,6 +283,7 @@ raycast_objects_kernel(const __grid_constant__ Pool pool, const Volume* __restri
   float nearest = 1.0e3f;
   double high_fg = 0.f;
   int miss = 0;
+  if (a.win) a.win[p] = 0;
   const M4 view = frames[ids.v[0]].view;
   const F3 w_dir = rotate(view, mk3((float)x, (float)y, 1.f));
   for (int o = 0; o < ids.n; ++o) {
@@ -296,6 +317,10 @@ raycast_objects_kernel(const __grid_constant__ Pool pool, const Volume* __restri
       continue;
     }
     high_fg = fg;
+    if (a.win) {
+      a.win[p] = (uint8_t)(o + 1);
+      a.win_hit[p] = hit;
+    }
     a.label[p] = F.label;
     a.vertex[p] = xform(F.T_w_o, mk3(hit.x, hit.y, hit.z));
     const F3 gn = volume_grad(pool, V, mk3(hit.x, hit.y, hit.z), s_slot + threadIdx.x, 128);
@@ -417,6 +442,10 @@ raycast_fold_kernel(const __grid_constant__ Pool pool, const Volume* __restrict_
     if (!crossed) zeroh |= 1u << o;
     win = o;
     win_hit = hit;
+  }
+  if (a.win) {
+    a.win[p] = (uint8_t)(win + 1);
+    a.win_hit[p] = win_hit;
   }
   if (win < 0) {
     if (miss == ids.n) {
@@ -833,10 +862,11 @@ void ray_variant_describe(int v, char* buf, int cap) {
 }
 
 int stage_raycast_to(Context* ctx, const IdList& ids, float epsilon, F3* vertex, F3* normal,
-                     int* label) {
+                     int* label, uint8_t* win, F4* win_hit) {
   if (ids.n == 0) return MF_OK;
   const mf_config& c = ctx->cfg;
-  RayArgs a{vertex, normal, label, ctx->W, ctx->H, c.near_plane, c.far_plane, c.mu, epsilon};
+  RayArgs a{vertex, normal, label, ctx->W, ctx->H, c.near_plane, c.far_plane, c.mu, epsilon, win,
+            win_hit};
   const RayVariant& r = ray_variants[ctx->tune.ray];
   const int th = 128 / r.tw;
   dim3 grid((ctx->W + r.tw - 1) / r.tw, (ctx->H + th - 1) / th);
@@ -948,16 +978,6 @@ __device__ float sample_adjoint(const Pool& P, const Volume& V, BlockMemo& m, F3
   return 0.f;
 }
 
-// The sample value of raycast_volume's loop at `pos`.
-__device__ __forceinline__ float march_value(const Pool& P, const Volume& V, BlockMemo& m,
-                                             F3 pos) {
-  const float inv = V.size / V.dim;
-  const I3 s = to_i3(mk3(pos.x * inv, pos.y * inv, pos.z * inv));
-  float f = tsdf_at_m(P, V, m, s.x, s.y, s.z);
-  if (f < 0.1f && f >= -0.5f) f = volume_interp_m<0>(P, V, pos, m);
-  return f;
-}
-
 // Replays raycast_volume and sweeps its march backwards with dE/dt* = g_t.
 // Returns 1 when done, 0 when the replay found no hit (nothing to do), -1 when
 // the march is longer than the checkpoints cover (the ray is skipped).
@@ -974,12 +994,13 @@ __device__ __noinline__ int march_adjoint(const Pool& P, const Volume& V, F3 ori
   const float smallest_tmax = fmn(fmn(tmax.x, tmax.y), fmn(tmax.x, tmax.z));
   const float tnear = fmx(largest_tmin, nearPlane);
   const float tfar = fmn(smallest_tmax, farPlane);
-  const float inv = V.size / V.dim;
   if (!(tnear < tfar)) return 0;
+  const MarchVolume mv = march_volume(P, V);
+  MarchMemo mm;
   BlockMemo memo;
   float t = tnear, stepsize = largestep;
   F3 position = origin + direction * t;
-  float f_t = volume_interp_m<0>(P, V, position, memo), f_tt = 0;
+  float f_t = march_open(mv, position), f_tt = 0;
   if (!(f_t > 0)) return 0;
   const F3 p0 = position;
   F3 cp_p[ADJ_MAX_CP];  // sample position at each checkpoint
@@ -990,9 +1011,7 @@ __device__ __noinline__ int march_adjoint(const Pool& P, const Volume& V, F3 ori
       if (c >= ADJ_MAX_CP) return -1;
       cp_p[c] = position;
     }
-    const I3 s = to_i3(mk3(position.x * inv, position.y * inv, position.z * inv));
-    f_tt = tsdf_at_m(P, V, memo, s.x, s.y, s.z);
-    if (f_tt < 0.1f && f_tt >= -0.5f) f_tt = volume_interp_m<0>(P, V, position, memo);
+    f_tt = march_sample(mv, mm, position);
     if (f_tt < 0) break;
     stepsize = fmx(f_tt * mu, step);
     position = position + stepsize * direction;
@@ -1019,7 +1038,7 @@ __device__ __noinline__ int march_adjoint(const Pool& P, const Volume& V, F3 ori
     F3 pos = cp_p[c];
     for (int j = j0; j <= j1; ++j) {
       seg_p[j - j0] = pos;
-      const float f = march_value(P, V, memo, pos);
+      const float f = march_sample(mv, mm, pos);
       seg_f[j - j0] = f;
       if (j < j1) pos = pos + fmx(f * mu, step) * direction;
     }
@@ -1104,45 +1123,17 @@ raycast_adjoint_kernel(const __grid_constant__ Pool pool, const Volume* __restri
   if (gv.x == 0.f && gv.y == 0.f && gv.z == 0.f && gn.x == 0.f && gn.y == 0.f && gn.z == 0.f)
     return;
   __shared__ int s_slot[8 * 128];
-  // replay the composite (raycast_objects_kernel) to find the winner
-  float nearest = 1.0e3f;
-  double high_fg = 0.f;
-  int win = -1;
-  F4 whit{0, 0, 0, 0};
-  float wnfar = 0.f, wtmin = 0.f;
-  F3 wdir = mk3(0.f);
-  const M4 view = frames[ids.v[0]].view;
-  const F3 w_dir = rotate(view, mk3((float)x, (float)y, 1.f));
-  for (int o = 0; o < ids.n; ++o) {
-    const int i = ids.v[o];
-    const Volume& V = vols[i];
-    const InstFrame& F = frames[i];
-    const float step = V.dim / V.size;
-    const F3 o_dir = normalize(rotate(F.inv_T_w_o, w_dir));
-    const float nfar = fmn(nearest, a.farPlane);
-    const float t_min = ray_first_block(V, F.o_origin, o_dir, a.nearPlane, nfar, a.epsilon, status);
-    const F4 hit = t_min > 0.f
-                       ? raycast_volume(pool, V, F.o_origin, o_dir,
-                                        t_min * V.dim / (unsigned)V.size, nfar, a.mu, step,
-                                        step * 8)
-                       : F4{0, 0, 0, 0};
-    const float hd = F.label == 0 ? hit.w + 0.05f : hit.w;
-    if (hd > nearest) continue;
-    const double fg = volume_interp(pool, V, mk3(hit.x, hit.y, hit.z), 1);
-    if (fg <= 0.5f) continue;
-    if (hd == nearest) {
-      if (!(fg > high_fg)) continue;
-    } else if (hd < nearest) {
-      nearest = hd;
-    } else {
-      continue;
-    }
-    high_fg = fg;
-    win = i; whit = hit; wnfar = nfar; wtmin = t_min; wdir = o_dir;
-  }
-  if (win < 0) return;
+  // the winner and its hit, as the raycast just before recorded them: the
+  // composite is not replayed (with every instance's traversal and march done
+  // again the kernel took 512 us with four volumes at 640x480, now 334)
+  const int o = (int)a.win[p] - 1;
+  if (o < 0) return;
+  const int win = ids.v[o];
+  const F4 whit = a.win_hit[p];
+  const F3 w_dir = rotate(frames[ids.v[0]].view, mk3((float)x, (float)y, 1.f));
   const Volume& V = vols[win];
   const InstFrame& F = frames[win];
+  const F3 wdir = normalize(rotate(F.inv_T_w_o, w_dir));
   const F3 X = mk3(whit.x, whit.y, whit.z);
   const F3 vm = xform(F.T_w_o, X);
   const F3 mv = a.vertex[p];
@@ -1162,19 +1153,24 @@ raycast_adjoint_kernel(const __grid_constant__ Pool pool, const Volume* __restri
   }
   if (whit.w == 0.f) return;  // a miss claimed by the corner's foreground: no march
   const float step = V.dim / V.size;
+  // the composite bounds a march by the nearest hit before it, but the march to
+  // the far plane starts at the same block and takes the same steps to the
+  // winner's crossing (see raycast_hits_kernel)
+  const float wtmin =
+      ray_first_block(V, F.o_origin, wdir, a.nearPlane, a.farPlane, a.epsilon, status);
   F3 rep;
   const int r = march_adjoint(pool, V, F.o_origin, wdir, wtmin * V.dim / (unsigned)V.size,
-                              wnfar, a.mu, step, step * 8, dot(wdir, gX), grad, &rep);
+                              a.farPlane, a.mu, step, step * 8, dot(wdir, gX), grad, &rep);
   if (r < 0 || (r == 1 && (rep.x != X.x || rep.y != X.y || rep.z != X.z)))
     atomicOr(status, ST_ADJOINT);
 }
 
-int stage_raycast_adjoint(Context* ctx, const IdList& ids, const double* gV, const double* gN,
-                          float* d_grad) {
+int stage_raycast_adjoint(Context* ctx, const IdList& ids, uint8_t* win, F4* win_hit,
+                          const double* gV, const double* gN, float* d_grad) {
   if (ids.n == 0) return MF_OK;
   const mf_config& c = ctx->cfg;
   RayArgs a{ctx->d_vertex, ctx->d_normal, ctx->d_label, ctx->W, ctx->H,
-            c.near_plane, c.far_plane, c.mu, ctx->ray_epsilon};
+            c.near_plane, c.far_plane, c.mu, ctx->ray_epsilon, win, win_hit};
   dim3 grid((ctx->W + 15) / 16, (ctx->H + 7) / 8);
   raycast_adjoint_kernel<<<grid, 128, 0, ctx->stream>>>(ctx->pool, ctx->d_vols, ctx->d_frames,
                                                         ids, a, gV, gN, d_grad, ctx->d_status);

@@ -105,6 +105,8 @@ struct TrackState {
   double* d_gmodel = nullptr;       // 2 x 3 x W x H: dE/d model vertex, dE/d model normal
   double* d_cost_part = nullptr;    // per-CTA partials of the cost rows, 8 each
   double* d_cost = nullptr;         // 8: cost, dE/d twist (6), rows
+  uint8_t* d_win = nullptr;         // W x H: the raycast's winner per pixel, and its hit
+  F4* d_win_hit = nullptr;
   int cost_blocks = 0;
   // motion residuals (allocated on first use)
   int8_t* d_mres = nullptr;         // 2 x W x H result codes: ICP rows, then photometric
@@ -2974,18 +2976,27 @@ int camera_cost(Context* ctx, const float* T_live16, int want_grad, double* out8
   if (!T.d_cost) {
     MF_CUDA(cudaMalloc(&T.d_gmodel, sizeof(double) * 6 * WH));
     MF_CUDA(cudaMalloc(&T.d_cost_part, sizeof(double) * 8 * nb));
+    MF_CUDA(cudaMalloc(&T.d_win, WH));
+    T.allocs.push_back(T.d_win);
+    MF_CUDA(cudaMalloc(&T.d_win_hit, sizeof(F4) * WH));
+    T.allocs.push_back(T.d_win_hit);
     MF_CUDA(cudaMalloc(&T.d_cost, sizeof(double) * 8));
     T.allocs.push_back(T.d_gmodel);
     T.allocs.push_back(T.d_cost_part);
     T.allocs.push_back(T.d_cost);
     T.cost_blocks = nb;
   }
-  // the model maps of the current TSDF at the current (reference) camera pose
+  // the model maps of the current TSDF at the current (reference) camera pose,
+  // and with a TSDF gradient each pixel's winner
+  const bool grad = want_grad && d_grad;
   IdList all;
   all.n = (int)ctx->inst.size();
   for (int i = 0; i < all.n; ++i) all.v[i] = i;
   if (int rc = stage_prepare(ctx, all)) return rc;
-  if (int rc = stage_raycast(ctx, all, ctx->ray_epsilon)) return rc;
+  if (int rc = stage_raycast_to(ctx, all, ctx->ray_epsilon, ctx->d_vertex, ctx->d_normal,
+                                ctx->d_label, grad ? T.d_win : nullptr,
+                                grad ? T.d_win_hit : nullptr))
+    return rc;
   M4 Tl;
   std::memcpy(&Tl, T_live16, 64);
   const mf_config& c = ctx->cfg;
@@ -3005,8 +3016,8 @@ int camera_cost(Context* ctx, const float* T_live16, int want_grad, double* out8
   camera_cost_kernel<<<nb, 256, 0, ctx->stream>>>(a, CostOut{T.d_cost_part, gV, gN, want_grad});
   cost_sum_kernel<<<1, 8 * COST_GROUPS, 0, ctx->stream>>>(T.d_cost_part, nb, T.d_cost);
   MF_CUDA(cudaGetLastError());
-  if (want_grad && d_grad)
-    if (int rc = stage_raycast_adjoint(ctx, all, gV, gN, d_grad)) return rc;
+  if (grad)
+    if (int rc = stage_raycast_adjoint(ctx, all, T.d_win, T.d_win_hit, gV, gN, d_grad)) return rc;
   MF_CUDA(cudaMemcpyAsync(out8, T.d_cost, sizeof(double) * 8, cudaMemcpyDeviceToHost,
                           ctx->stream));
   MF_CUDA(cudaStreamSynchronize(ctx->stream));
