@@ -3053,9 +3053,11 @@ struct MotionArgs {
 };
 
 __global__ void motion_residual_kernel(MotionArgs a) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
   const int n = a.W * a.H;
-  if (p >= n) return;
+  // the last CTA's idle threads repeat the last pixel (its rows are written
+  // with the same values) and count nothing
+  const int p0 = blockIdx.x * blockDim.x + threadIdx.x;
+  const int p = min(p0, n - 1);
   const int x = p % a.W, y = p / a.W;
   int8_t ri = 0, rr = 0;
   float ei = 0.f, er = 0.f;
@@ -3131,13 +3133,22 @@ __global__ void motion_residual_kernel(MotionArgs a) {
   // check_static_state: an object pixel of the live render is an inlier when
   // its rows' results are > -3
   const int l = a.llabel[p];
-  if (l >= 1 && l < 32) {
-    bool inl;
-    if (a.use_icp && a.use_rgb) inl = ri > -3 && rr > -3;
-    else if (a.use_icp) inl = ri > -3;
-    else inl = a.use_rgb && rr > -3;
-    atomicAdd(a.count + l, 1);
-    if (inl) atomicAdd(a.count + 32 + l, 1);
+  bool inl;
+  if (a.use_icp && a.use_rgb) inl = ri > -3 && rr > -3;
+  else if (a.use_icp) inl = ri > -3;
+  else inl = a.use_rgb && rr > -3;
+  // one atomic per warp and label: 31 -> 12 us at 640x480 (one per pixel, all
+  // of an object's on the same two words, was a serial chain in L2)
+  const int mine = p0 < n && l >= 1 && l < 32 ? l : 0;
+  for (unsigned left = __ballot_sync(0xffffffffu, mine); left;) {
+    const int lab = __shfl_sync(0xffffffffu, mine, __ffs(left) - 1);
+    const unsigned m = __ballot_sync(0xffffffffu, mine == lab);
+    const unsigned in = __ballot_sync(0xffffffffu, mine == lab && inl);
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd(a.count + lab, __popc(m));
+      if (in) atomicAdd(a.count + 32 + lab, __popc(in));
+    }
+    left &= ~m;
   }
 }
 
