@@ -192,7 +192,8 @@ struct CameraCostFunction : public torch::autograd::Function<CameraCostFunction>
     }
     const auto gE = grad_out[0].detach().to(torch::kCPU, torch::kFloat64);
     const double scale = gE.item<double>();
-    return {(g_twist * scale).to(twist.options()), (grad * scale).view_as(tsdf),
+    if (scale != 1.0) grad.mul_(scale);  // in place: it is this call's own tensor
+    return {(g_twist * scale).to(twist.options()), grad.view_as(tsdf),
             torch::Tensor(), torch::Tensor()};
   }
 };
