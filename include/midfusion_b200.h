@@ -555,7 +555,7 @@ int mf_set_overlap(mf_context* ctx, int ctas);
  *   MF_TUNE_RAYCAST    the composite raycast (raycastObjectList): the pixel
  *                      tile of a 128-thread CTA and the register bound;
  *   MF_TUNE_INTEGRATE  the voxel-block integration (projective_functor::
- *                      update_block): 512-thread CTAs resident per SM.
+ *                      update_block): 256-thread CTAs resident per SM.
  * Variant 0 of each is the default.  A context starts with the defaults. */
 #define MF_TUNE_RAYCAST 0
 #define MF_TUNE_INTEGRATE 1

@@ -5,7 +5,7 @@
 // the same inputs whatever the shape:
 //  - raycast_objects_kernel: the pixel tile of a 128-thread CTA and the
 //    register bound (residency) it is compiled for (ray_variants);
-//  - integrate_blocks_kernel: how many 512-thread CTAs are resident per SM,
+//  - integrate_blocks_kernel: how many 256-thread CTAs are resident per SM,
 //    which sets both the register bound and the persistent grid (int_variants).
 // autotune() times every candidate on the context's current frame with CUDA
 // events and keeps the fastest.  The map is never touched: the raycasts write

@@ -352,10 +352,12 @@ __global__ void alloc_keys_kernel(const Volume* __restrict__ vols, int inst,
 // projective_functor::build_active_list, lib/functors/projective_functor.hpp:54-71
 // with algorithms::filter (lib/algorithms/filter.hpp:42-61, predicates ORed):
 // a block is visited when it is active or its corner projects into the frame.
+// clear: the integration that follows sets VoxelBlock::active_ anew; it is
+// cleared here, so that each of its warps can set it without a barrier.
 __global__ void __launch_bounds__(256)
 visit_list_kernel(Pool pool, const Volume* __restrict__ vols,
                   const InstFrame* __restrict__ frames, uint32_t inst_mask, int W, int H,
-                  int* __restrict__ visit, int* __restrict__ visit_count) {
+                  int* __restrict__ visit, int* __restrict__ visit_count, int clear) {
   const int slot = blockIdx.x * blockDim.x + threadIdx.x;
   bool take = false;
   if (slot < *pool.count) {
@@ -380,7 +382,10 @@ visit_list_kernel(Pool pool, const Volume* __restrict__ vols,
   int base = 0;
   if (lane == __ffs(ballot) - 1) base = atomicAdd(visit_count, __popc(ballot));
   base = __shfl_sync(0xffffffffu, base, __ffs(ballot) - 1);
-  if (take) visit[base + __popc(ballot & ((1u << lane) - 1))] = slot;
+  if (take) {
+    visit[base + __popc(ballot & ((1u << lane) - 1))] = slot;
+    if (clear) pool.active[slot] = 0;
+  }
 }
 
 struct SdfArgs {
@@ -419,39 +424,49 @@ __device__ __forceinline__ void sdf_update(const SdfArgs& a, const float* mask, 
   }
 }
 
-// Hint: bring the 144 128-byte lines holding the eight voxel fields of pool
-// slot `slot` (7 x 2 KB of 4-byte fields, 4 KB of fg) into L2, one line per
-// thread of the first 144.
-__device__ __forceinline__ void prefetch_block_fields(const Pool& pool, int slot) {
-  const int t = threadIdx.x;
-  if (t >= 144) return;
-  const size_t o = (size_t)slot * 512;
-  const int fi = t >> 4;
-  const void* base = fi == 0   ? (const void*)(pool.tsdf + o)
-                     : fi == 1 ? (const void*)(pool.wt + o)
-                     : fi == 2 ? (const void*)(pool.r + o)
-                     : fi == 3 ? (const void*)(pool.g + o)
-                     : fi == 4 ? (const void*)(pool.b + o)
-                     : fi == 5 ? (const void*)(pool.c + o)
-                     : fi == 6 ? (const void*)(pool.w + o)
-                               : (const void*)(pool.fg + o);
-  const char* p = (const char*)base + (fi < 7 ? (t & 15) : t - 112) * 128;
+// Hint: bring the 36 128-byte lines holding the eight fields of this warp's
+// 128 voxels (from v0 on) of pool slot `slot` into L2.
+__device__ __forceinline__ void prefetch_fields(const Pool& pool, int slot, int v0, int lane) {
+  const size_t o = (size_t)slot * 512 + v0;
+  const int f = lane >> 2;
+  const void* base = f == 0   ? (const void*)(pool.tsdf + o)
+                     : f == 1 ? (const void*)(pool.wt + o)
+                     : f == 2 ? (const void*)(pool.r + o)
+                     : f == 3 ? (const void*)(pool.g + o)
+                     : f == 4 ? (const void*)(pool.b + o)
+                     : f == 5 ? (const void*)(pool.c + o)
+                     : f == 6 ? (const void*)(pool.w + o)
+                              : (const void*)(pool.fg + o);
+  const char* p = (const char*)base + (lane & 3) * 128;
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+  if (f == 7) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + 512));
 }
 
 // projective_functor::update_block, lib/functors/projective_functor.hpp:73-111.
-// Persistent CTAs of 512 threads, one visited block at a time, one voxel per
-// thread: every field plane is read and written coalesced, and only for voxels
-// that pass the update test.  The next block's slot and corner are loaded
-// during the current one, and the instances' constants come from shared
-// memory, so a block's dependent chain is the pixel fetch and the voxel
-// read-modify-write.
-// MINB 512-thread CTAs are resident per SM (the register bound) and the grid
-// is MINB CTAs per SM; with PF the CTA prefetches the next block's voxel
-// fields into L2 while it works on the current one.  Every variant updates
-// each voxel alike (int_variants).
+// A warp takes a quarter of a visited block (two z layers), four neighbouring
+// voxels of a row per thread: the row's transforms are computed once for the
+// four, their depth and mask fetches are in flight together, and every field
+// plane is read and written 16 bytes at a time, only where one of the four
+// passes the update test.  Warps never wait for each other
+// (VoxelBlock::active_ is cleared by the visit list and set by any warp that
+// sees a voxel).  The next block's slot and corner are loaded during the
+// current one; the instances' constants come from shared memory.
+// Bound by instruction issue (seven divisions and a square root per updated
+// voxel; the double one of the foreground mean is left out where the mean is
+// 0 or 1 exactly, as for every voxel that one kind of mask has seen) and by
+// the fields' traffic.  Background 512^3 and three objects 256^3 at 640x480:
+// 98 us, 4.0 TB/s, issue slots 55 % busy (one voxel per thread and a barrier
+// per block: 130 us, 65 %, half again as many instructions; without the barrier
+// alone 131).  Registers bound the warps in flight: 4 CTAs per SM (64
+// registers, 98 us) beat 5 (48, spills, 114) and 3 (80, 117); the prefetch
+// gains nothing here, since the loads wait for the pixels, not for DRAM.
+// Persistent: MINB 256-thread CTAs per SM (the register bound); with PF the
+// warp prefetches its quarter of the next block's fields into L2 while it
+// works on the current one.  Every variant updates each voxel alike
+// (int_variants).
+constexpr int INT_THREADS = 256;  // two blocks per CTA
 template <int MINB, bool PF>
-__global__ void __launch_bounds__(512, MINB)
+__global__ void __launch_bounds__(INT_THREADS, MINB)
 integrate_blocks_kernel(Pool pool, const Volume* __restrict__ vols,
                         const InstFrame* __restrict__ frames, SdfArgs args, F4 k,
                         const int* __restrict__ visit, const int* __restrict__ visit_count) {
@@ -472,25 +487,27 @@ integrate_blocks_kernel(Pool pool, const Volume* __restrict__ vols,
     s_vs[i] = vols[i].dim / vols[i].size;
   }
   __syncthreads();
-  // one voxel per thread; the next block's corner is fetched one block ahead
-  // and (PF) the slot after it two blocks ahead
-  const int v = threadIdx.x;
-  const int x = v & 7, y = (v >> 3) & 7, z = v >> 6;
-  int item = blockIdx.x;
+  // four warps per block; the next block's corner is
+  // fetched one block ahead and (PF) the slot after it two blocks ahead
+  const int lane = threadIdx.x & 31;
+  const int v = (threadIdx.x & 127) * 4;
+  const int x0 = v & 7, y = (v >> 3) & 7, z = v >> 6;
+  const int stride = INT_THREADS / 128 * gridDim.x;
+  int item = (threadIdx.x >> 7) * gridDim.x + blockIdx.x;
   int next_slot = item < n ? visit[item] : 0;
   int4 next_m = item < n ? pool.meta[next_slot] : make_int4(0, 0, 0, 0);
   int after_slot = 0;
-  if (PF && item + (int)gridDim.x < n) after_slot = visit[item + gridDim.x];
-  for (; item < n; item += gridDim.x) {
+  if (PF && item + stride < n) after_slot = visit[item + stride];
+  for (; item < n; item += stride) {
     const int slot = next_slot;
     const int4 m = next_m;
-    if (item + gridDim.x < n) {
+    if (item + stride < n) {
       if (PF) {
-        prefetch_block_fields(pool, after_slot);
+        prefetch_fields(pool, after_slot, v & ~127, lane);
         next_slot = after_slot;
-        if (item + 2 * gridDim.x < n) after_slot = visit[item + 2 * gridDim.x];
+        if (item + 2 * stride < n) after_slot = visit[item + 2 * stride];
       } else {
-        next_slot = visit[item + gridDim.x];
+        next_slot = visit[item + stride];
       }
       next_m = pool.meta[next_slot];
     }
@@ -499,50 +516,91 @@ integrate_blocks_kernel(Pool pool, const Volume* __restrict__ vols,
     // voxel -> pixel
     const F3 start = xform(s_Tcw[m.w], mk3(m.x * vs, (m.y + y) * vs, (m.z + z) * vs));
     const F3 camerastart = xform(K, start);
-    const F3 cv = camerastart + ((float)x * s_cdelta[m.w]);
-    const F3 pos = start + ((float)x * s_delta[m.w]);
-    bool vis = false;
-    int pix = 0;
-    if (pos.z >= 0.0001f) {
-      const float inv = 1.f / cv.z;
-      const float pxf = cv.x * inv + 0.5f, pyf = cv.y * inv + 0.5f;
-      if (!(pxf < 0.5f || pxf > wlim || pyf < 0.5f || pyf > hlim)) {
-        vis = true;
-        pix = (int)((unsigned)pxf + W * (unsigned)pyf);
+    const F3 delta = s_delta[m.w], cdelta = s_cdelta[m.w];
+    int pix[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const F3 cv = camerastart + ((float)(x0 + i) * cdelta);
+      pix[i] = -1;
+      if (start.z + (float)(x0 + i) * delta.z >= 0.0001f) {
+        const float inv = 1.f / cv.z;
+        const float pxf = cv.x * inv + 0.5f, pyf = cv.y * inv + 0.5f;
+        if (!(pxf < 0.5f || pxf > wlim || pyf < 0.5f || pyf > hlim))
+          pix[i] = (int)((unsigned)pxf + W * (unsigned)pyf);
       }
     }
+    const bool vis = (pix[0] & pix[1] & pix[2] & pix[3]) >= 0;
+    if (__any_sync(0xffffffffu, vis) && lane == 0) pool.active[slot] = 1;
     // depth / mask at the pixel, the update test of sdf_update
-    const float depthS = vis ? __ldg(args.depth + pix) : 0.f;
-    const float mval = vis ? __ldg(mask + pix) : -1.f;
-    bool upd = false;
-    float sdf = 0.f;
-    if (vis && depthS > 0 && mval >= 0) {
-      const float diff = (depthS - pos.z) * sqrtf(1 + sq(pos.x / pos.z) + sq(pos.y / pos.z));
-      if (diff > -mu) {
-        upd = true;
-        sdf = fmn(1.f, diff / mu);
+    float depthS[4], mval[4], sdf[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      depthS[i] = pix[i] >= 0 ? __ldg(args.depth + pix[i]) : 0.f;
+      mval[i] = pix[i] >= 0 ? __ldg(mask + pix[i]) : -1.f;
+    }
+    bool any = false;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      bool upd = false;
+      if (depthS[i] > 0 && mval[i] >= 0) {
+        const F3 pos = start + ((float)(x0 + i) * delta);
+        const float diff =
+            (depthS[i] - pos.z) * sqrtf(1 + sq(pos.x / pos.z) + sq(pos.y / pos.z));
+        if (diff > -mu) {
+          upd = true;
+          sdf[i] = fmn(1.f, diff / mu);
+        }
       }
+      if (!upd) pix[i] = -1;
+      any |= upd;
     }
-    // read-modify-write of the voxel
-    if (upd) {
-      const size_t o = (size_t)slot * 512 + v;
-      const float t = pool.tsdf[o], wt = pool.wt[o], r = pool.r[o], g = pool.g[o],
-                  b = pool.b[o];
-      const int c = pool.c[o], w = pool.w[o];
-      const double fg = pool.fg[o];
-      const F3 rgb = args.rgb[pix];
-      // sdf_update, apps/kfusion/src/cpp/kfusion/mapping_impl.hpp:26-46
-      pool.tsdf[o] = clampf((wt * t + sdf) / (wt + 1), -1.f, 1.f);
-      pool.wt[o] = fmn(wt + 1, maxweight);
-      pool.r[o] = (rgb.x + r * c) / (c + 1);
-      pool.g[o] = (rgb.y + g * c) / (c + 1);
-      pool.b[o] = (rgb.z + b * c) / (c + 1);
-      pool.c[o] = c + 1;
-      pool.fg[o] = ((double)mval + fg * w) / (w + 1);
-      pool.w[o] = w + 1;
+    // read-modify-write of the voxels: sdf_update,
+    // apps/kfusion/src/cpp/kfusion/mapping_impl.hpp:26-46
+    if (any) {
+      const size_t o = ((size_t)slot * 512 + v) / 4;
+      float4 t4 = ((const float4*)pool.tsdf)[o], wt4 = ((const float4*)pool.wt)[o];
+      float4 r4 = ((const float4*)pool.r)[o], g4 = ((const float4*)pool.g)[o],
+             b4 = ((const float4*)pool.b)[o];
+      int4 c4 = ((const int4*)pool.c)[o];
+      int4 w4 = ((const int4*)pool.w)[o];
+      float *t = &t4.x, *wt = &wt4.x, *r = &r4.x, *g = &g4.x, *b = &b4.x;
+      int *c = &c4.x, *w = &w4.x;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (pix[i] >= 0) {
+          const F3 rgb = args.rgb[pix[i]];
+          t[i] = clampf((wt[i] * t[i] + sdf[i]) / (wt[i] + 1), -1.f, 1.f);
+          wt[i] = fmn(wt[i] + 1, maxweight);
+          const float cf = c[i], c1 = c[i] + 1;
+          r[i] = (rgb.x + r[i] * cf) / c1;
+          g[i] = (rgb.y + g[i] * cf) / c1;
+          b[i] = (rgb.z + b[i] * cf) / c1;
+          c[i] = c[i] + 1;
+        }
+      ((float4*)pool.tsdf)[o] = t4;
+      ((float4*)pool.wt)[o] = wt4;
+      ((float4*)pool.r)[o] = r4;
+      ((float4*)pool.g)[o] = g4;
+      ((float4*)pool.b)[o] = b4;
+      ((int4*)pool.c)[o] = c4;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        double2 f2 = ((const double2*)pool.fg)[2 * o + h];
+        double* f = &f2.x;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          if (pix[2 * h + i] >= 0) {
+            const int wi = w[2 * h + i];
+            const double num = (double)mval[2 * h + i] + f[i] * wi, den = (double)(wi + 1);
+            // den / den and +-0 / den of a positive den
+            f[i] = wi >= 0 && num == den ? 1.0 : wi >= 0 && num == 0.0 ? num : num / den;
+            w[2 * h + i] = wi + 1;
+          }
+        ((double2*)pool.fg)[2 * o + h] = f2;
+      }
+      ((int4*)pool.w)[o] = w4;
     }
-    const int any = __syncthreads_or(vis);
-    if (threadIdx.x == 0) pool.active[slot] = any ? 1 : 0;
+    __syncwarp();
   }
 }
 
@@ -760,7 +818,7 @@ int profile_integrate(Context* ctx, int reps, double* us, double* bytes) {
   MF_CUDA(cudaMemsetAsync(ctx->d_visit_count, 0, sizeof(int), ctx->stream));
   visit_list_kernel<<<div_up(ctx->pool.cap, 256), 256, 0, ctx->stream>>>(
       ctx->pool, ctx->d_vols, ctx->d_frames, mask, ctx->W, ctx->H, ctx->d_visit,
-      ctx->d_visit_count);
+      ctx->d_visit_count, 1);
   SdfArgs a{ctx->d_depth, ctx->d_rgb, ctx->d_masks, ctx->W, ctx->H, c.mu, (float)c.max_weight};
   const F4 k{c.k[0], c.k[1], c.k[2], c.k[3]};
   int sms = 148;
@@ -804,9 +862,9 @@ struct IntVariant {
   void (*fn)(Pool, const Volume*, const InstFrame*, SdfArgs, F4, const int*, const int*);
 };
 static const IntVariant int_variants[] = {
-    {4, false, integrate_blocks_kernel<4, false>}, {3, false, integrate_blocks_kernel<3, false>},
-    {2, false, integrate_blocks_kernel<2, false>}, {4, true, integrate_blocks_kernel<4, true>},
-    {3, true, integrate_blocks_kernel<3, true>},   {2, true, integrate_blocks_kernel<2, true>},
+    {4, false, integrate_blocks_kernel<4, false>}, {5, false, integrate_blocks_kernel<5, false>},
+    {3, false, integrate_blocks_kernel<3, false>}, {4, true, integrate_blocks_kernel<4, true>},
+    {5, true, integrate_blocks_kernel<5, true>},   {3, true, integrate_blocks_kernel<3, true>},
 };
 constexpr int N_INT_VARIANTS = (int)(sizeof(int_variants) / sizeof(int_variants[0]));
 static_assert(N_INT_VARIANTS <= MAX_TUNE_VARIANTS, "integration candidate table too long");
@@ -814,7 +872,7 @@ static_assert(N_INT_VARIANTS <= MAX_TUNE_VARIANTS, "integration candidate table 
 int int_variant_count() { return N_INT_VARIANTS; }
 
 void int_variant_describe(int v, char* buf, int cap) {
-  snprintf(buf, cap, "integrate %d x 512-thread CTAs per SM%s", int_variants[v].minb,
+  snprintf(buf, cap, "integrate %d x 256-thread CTAs per SM%s", int_variants[v].minb,
            int_variants[v].prefetch ? ", next block's fields prefetched to L2" : "");
 }
 
@@ -827,20 +885,22 @@ int launch_integrate_blocks(Context* ctx, const Pool& pool, int variant, int cta
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   const IntVariant& v = int_variants[variant];
-  const int grid = ctas > 0 ? ctas : sms * v.minb;
-  v.fn<<<grid, 512, 0, ctx->stream>>>(pool, ctx->d_vols, ctx->d_frames, a, k, ctx->d_visit,
+  // `ctas` counts 512 threads (mf_set_overlap)
+  const int grid = ctas > 0 ? ctas * (512 / INT_THREADS) : sms * v.minb;
+  v.fn<<<grid, INT_THREADS, 0, ctx->stream>>>(pool, ctx->d_vols, ctx->d_frames, a, k, ctx->d_visit,
                                       ctx->d_visit_count);
   MF_CUDA(cudaGetLastError());
   return MF_OK;
 }
 
 // projective_functor::build_active_list over the instances in `inst_mask`.
-// zeroed: stage_prepare has reset the list's counter.
+// zeroed: stage_prepare has reset the list's counter, and the integration of
+// the listed blocks follows (else the pool is left as it is).
 int build_visit_list(Context* ctx, uint32_t inst_mask, bool zeroed) {
   if (!zeroed) MF_CUDA(cudaMemsetAsync(ctx->d_visit_count, 0, sizeof(int), ctx->stream));
   visit_list_kernel<<<div_up(ctx->pool.cap, 256), 256, 0, ctx->stream>>>(
       ctx->pool, ctx->d_vols, ctx->d_frames, inst_mask, ctx->W, ctx->H, ctx->d_visit,
-      ctx->d_visit_count);
+      ctx->d_visit_count, zeroed);
   MF_CUDA(cudaGetLastError());
   return MF_OK;
 }
