@@ -44,3 +44,72 @@ def test_floor_test_equals_range_test_and_truncation(size):
     assert np.array_equal(v_r[ok_r], v_k[ok_k])
     assert np.all((v_k[ok_k] >= 0) & (v_k[ok_k] < size))
 
+
+
+def test_block_index_is_the_morton_index():
+    """spread3_10 / block_index (mf_common.cuh) against the bit-by-bit Morton
+    code, every coordinate below 1024."""
+    def spread(v):
+        v = v.astype(np.uint32)
+        v = (v | v << np.uint32(16)) & np.uint32(0x030000ff)
+        v = (v | v << np.uint32(8)) & np.uint32(0x0300f00f)
+        v = (v | v << np.uint32(4)) & np.uint32(0x030c30c3)
+        return (v | v << np.uint32(2)) & np.uint32(0x09249249)
+    v = np.arange(1024, dtype=np.uint32)
+    want = sum(((v >> np.uint32(b)) & 1).astype(np.uint32) << np.uint32(3 * b) for b in range(10))
+    assert np.array_equal(spread(v), want)
+
+
+def test_length_threshold_without_the_square_root():
+    """sqrtf(x) > 0.1f exactly when x > 0x1.47ae16p-7f (longer_than_10cm)."""
+    t = np.float32(float.fromhex("0x1.47ae16p-7"))
+    assert np.sqrt(t) <= np.float32(0.1) < np.sqrt(np.nextafter(t, np.float32(1)))
+    rng = np.random.default_rng(1)
+    x = np.abs(t + rng.standard_normal(1 << 20).astype(np.float32) * np.float32(1e-6))
+    assert np.array_equal(np.sqrt(x) > np.float32(0.1), x > t)
+
+
+def test_float_quotient_equals_the_rounded_double_quotient():
+    """(float)(1.0 / (double)s) == 1.0f / s for normal results (inv_sigma)."""
+    rng = np.random.default_rng(2)
+    s = np.exp(rng.uniform(-60, 60, 1 << 21)).astype(np.float32)
+    assert np.array_equal((1.0 / s.astype(np.float64)).astype(np.float32), np.float32(1) / s)
+
+
+def test_huber_inlier_loss_in_float():
+    """0.5f * (e * e) is the double loss 0.5 e^2 rounded once, up to the largest
+    float that is at most 1.345 (mf_robust.cuh)."""
+    k = np.float32(float.fromhex("0x1.5851eap+0"))
+    assert float(k) <= 1.345 < float(np.nextafter(k, np.float32(2)))
+    e = np.random.default_rng(3).uniform(-1, 1, 1 << 21).astype(np.float32) * k
+    e = np.concatenate([e, np.float32([0, 1e-15, -1e-15]), k[None], -k[None]])
+    want = (0.5 * e.astype(np.float64) ** 2).astype(np.float32)
+    assert np.array_equal(np.float32(0.5) * (e * e), want)
+
+
+def test_constant_division_with_one_correction():
+    """div_e2 (mf_track.cu): x / 0.02f as q = x rc; q += rc (x - q b), both
+    multiply-adds rounded once, equals the IEEE quotient for every mantissa."""
+    b = np.float32(np.float32(0.1) * np.float32(0.1)) * np.float32(2)
+    rc = np.float32(1) / b
+    assert float(b).hex() == "0x1.47ae160000000p-6" and float(rc).hex() == "0x1.8ffffe0000000p+5"
+    x = ((np.uint32(127) << np.uint32(23)) | np.arange(1 << 23, dtype=np.uint32)).view(np.float32)
+    q = x * rc
+    # q b has 48 bits and x - q b cancels: exact in double, as in the fma
+    r = (x.astype(np.float64) - q.astype(np.float64) * np.float64(b)).astype(np.float32)
+    got = (r.astype(np.longdouble) * np.longdouble(rc) + q).astype(np.float32)
+    assert np.array_equal(got, x / b)
+
+
+def test_block_coordinate_by_a_round_down_addition():
+    """f + (2^26 + 2^25) rounded towards minus infinity is a multiple of 8: its
+    low bits are floor(f / 8) for 0 <= f < 4096 (alloc_mark_kernel)."""
+    rng = np.random.default_rng(4)
+    f = rng.uniform(0, 4096, 1 << 20).astype(np.float32)
+    f = np.concatenate([f, np.arange(0, 4096, 8, dtype=np.float32),
+                        np.nextafter(np.arange(8, 4097, 8, dtype=np.float32), np.float32(0)),
+                        np.float32([0.0, -0.0, 4095.9998])])
+    big = np.float64(2 ** 26 + 2 ** 25)
+    down = (np.floor((f.astype(np.float64) + big) / 8) * 8).astype(np.float32)
+    bits = down.view(np.uint32) - np.uint32(0x4cc00000)
+    assert np.array_equal(bits, (f.astype(np.int64) >> 3).astype(np.uint32))
