@@ -38,6 +38,17 @@ MF_HD float sq(float r) { return r * r; }
 struct F3 { float x, y, z; };
 struct alignas(16) F4 { float x, y, z, w; };  // matrix rows move as one 16-byte access
 struct I3 { int x, y, z; };
+
+// n / d where n is often exactly 0: the general quotient takes a slow path then
+// (one warp in flight: 286 cycles against 63, in double 471 against 126), and
+// the whole warp waits for a single such lane.  For a finite d != 0 the
+// quotient of a zero is n * d, the zero with the right sign.
+template <typename T>
+MF_HD T div0(T n, T d) {
+  const bool z = n == 0 && d != 0 && d - d == 0;
+  const T q = (z ? d : n) / d;
+  return z ? n * d : q;
+}
 struct M4 { F4 r[4]; };  // Matrix4: r[i] is row i (utils/math_utils.h:47-49)
 
 MF_HD F3 mk3(float x, float y, float z) { F3 v; v.x = x; v.y = y; v.z = z; return v; }
@@ -126,7 +137,7 @@ MF_HD M4 inverse(const M4& A) {
     }
 #pragma unroll
     for (int r = c + 1; r < 4; ++r) {
-      const float f = a[r][c] / a[c][c];
+      const float f = div0(a[r][c], a[c][c]);
 #pragma unroll
       for (int j = c; j < 4; ++j) a[r][j] -= f * a[c][j];
 #pragma unroll
@@ -141,7 +152,7 @@ MF_HD M4 inverse(const M4& A) {
       float s = b[r][j];
 #pragma unroll
       for (int k = r + 1; k < 4; ++k) s -= a[r][k] * R[k][j];
-      R[r][j] = s / a[r][r];
+      R[r][j] = div0(s, a[r][r]);
     }
   M4 out;
 #pragma unroll

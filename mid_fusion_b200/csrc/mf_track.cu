@@ -248,7 +248,7 @@ __global__ void half_sample_kernel(const float* __restrict__ in0, float* __restr
       const float cur = in[ux + uy * iw];
       if (fabsf(cur - center) < e_d) { sum += 1.0f; t += cur; }
     }
-  out[p] = t / sum;
+  out[p] = div0(t, sum);
 }
 
 // depth2vertexKernel, preprocessing.cpp:52-71.
@@ -383,7 +383,7 @@ __global__ void half_sample_slots_kernel(SlotPtrs sp, int iw, int ih, float e_d)
       const float cur = in[ux + uy * iw];
       if (fabsf(cur - center) < e_d) { sum += 1.0f; t += cur; }
     }
-  out[p] = t / sum;
+  out[p] = div0(t, sum);
 }
 
 // The rendered reference depth and vertex planes of every slot at every level.
@@ -650,12 +650,10 @@ __device__ __forceinline__ bool solve6_warp(const double* s, int lane, double x[
     piv[j] = pr[j];
     pmax = fmax(pmax, pr[j]);
     ok = ok && (pr[j] > 0);
-    if (r != j) {
-      const double f = a[j] / pr[j];
+    const double f = a[j] / pr[j];
 #pragma unroll
-      for (int k = j; k < 6; ++k) a[k] -= f * pr[k];
-      c -= f * pc;
-    }
+    for (int k = j; k < 6; ++k) a[k] = r != j ? a[k] - f * pr[k] : a[k];
+    c = r != j ? c - f * pc : c;
   }
 #pragma unroll
   for (int j = 0; j < 6; ++j) ok = ok && (piv[j] > 1e-5 * pmax);
@@ -701,7 +699,9 @@ __device__ __noinline__ void gn_step_warp(GNState* Sp, const double* s, int leve
     double nx = 0;
 #pragma unroll
     for (int i = 0; i < 6; ++i) nx += x[i] * x[i];
-    if (sqrt(nx) < (double)1e-05f && sqrt(s[0] / s[28]) < 2e-3) {
+    // sqrt(nx) < (double)1e-05f without the square root: the smallest double
+    // whose root is not below is 0x1.b7cdfc28ae3ffp-34
+    if (nx < 0x1.b7cdfc28ae3ffp-34 && sqrt(s[0] / s[28]) < 2e-3) {
       done = 1;
     } else {
       // se3_exp(x): element (i, j) of the update on lane 4 i + j
@@ -875,8 +875,9 @@ __device__ __forceinline__ float bil(const float* img, int w, float px, float py
 template <int KIND>
 __device__ __forceinline__ void rgb_finish(const GNState& S, const F4& k, float ic, float residual,
                                            float gx, float gy, F3 wv, F3 live, Row& r) {
+  // in a flat patch the numerator is 0
   F3 Jt = (1.f / live.z) * mk3(gx * k.x, gy * k.y,
-                               -(gx * live.x * k.x + gy * live.y * k.y) / live.z);
+                               div0(-(gx * live.x * k.x + gy * live.y * k.y), live.z));
   F3 Jr;
   if (KIND == 0) {
     Jt = -1.f * rotate(S.Tf, Jt);  // rotate(Jtrans, transpose(T_w_l))
@@ -937,7 +938,10 @@ __device__ __forceinline__ void camera_rows(const GNArgs& a, const GNView& lv, c
     const F3 pn = rotate(S.Tf, n);
     if (ri.result == 0)
       ri.result = rn.x == INVALIDF ? -3 : longer_than_10cm(diff) ? -4 : dot(pn, rn) < 0.8f ? -5 : 1;
-    const float sig = rn.x * rn.x * P.x + rn.y * rn.y * P.y + rn.z * rn.z * P.z;
+    // a row that is not used has sig = 1: a zero would take the general
+    // quotient's slow path, and the warp with it
+    const float sig = ri.result == 1 ? rn.x * rn.x * P.x + rn.y * rn.y * P.y + rn.z * rn.z * P.z
+                                     : 1.f;
     const float ic = inv_sigma(sig);
     ri.e = ic * dot(rn, diff);
     const F3 j1 = ic * cross(pv, rn);
@@ -1041,7 +1045,8 @@ __device__ __forceinline__ void object_rows(const GNArgs& a, const GNView& lv, c
     if (ri.result == 0)
       ri.result = wrn.x == INVALIDF ? -3 : longer_than_10cm(diff) ? -4
                   : dot(o2n, o1rn) < 0.8f ? -5 : 1;
-    const float sig = o1rn.x * o1rn.x * P.x + o1rn.y * o1rn.y * P.y + o1rn.z * o1rn.z * P.z;
+    const float sig = ri.result == 1
+        ? o1rn.x * o1rn.x * P.x + o1rn.y * o1rn.y * P.y + o1rn.z * o1rn.z * P.z : 1.f;
     const float ic = inv_sigma(sig);
     ri.e = ic * residual;
     const F3 Jt = rotate(S.Tf, o1rn);
