@@ -118,6 +118,32 @@ static int frame_overlapped(Context* ctx, bool gen, const IdList& all, const IdL
   return track_set_ref(ctx);
 }
 
+// The pyramid on the main stream and, beside it on the side stream, what needs
+// no live frame: the camera's problem and its rendered reference (five small
+// launches, some 3 us each, that only read the last raycast), then the
+// integration masks (gen).  The main stream then waits for both.
+// One 160x120 volume: a frame 225 us in order (2 us of it the setup by one
+// thread), 217 so; 320x240 284 and 274.
+static int pyramid_and_camera_pre(Context* ctx, bool gen) {
+  cudaStream_t main = ctx->stream, side = ctx->side;
+  cudaError_t e = cudaSuccess;
+  auto ok = [&](cudaError_t x) { if (x != cudaSuccess && e == cudaSuccess) e = x; };
+  ok(cudaEventRecord(ctx->ev_start, main));
+  ok(cudaStreamWaitEvent(side, ctx->ev_start, 0));
+  ctx->stream = side;
+  int rc = track_camera_pre(ctx, 0);
+  if (!rc && gen) rc = launch_generalize(ctx);
+  ok(cudaEventRecord(ctx->ev_gen, side));
+  ctx->stream = main;
+  if (!rc) rc = track_preprocess(ctx);
+  ok(cudaStreamWaitEvent(main, ctx->ev_gen, 0));
+  if (!rc && e != cudaSuccess) {
+    ctx->last_error = std::string("overlapped pyramid: ") + cudaGetErrorString(e);
+    rc = MF_E_CUDA;
+  }
+  return rc;
+}
+
 // Everything of one frame after the inputs are on the device.
 static int frame_body(Context* ctx, bool track, bool labels) {
   const int n = (int)ctx->inst.size();
@@ -136,13 +162,18 @@ static int frame_body(Context* ctx, bool track, bool labels) {
   const bool gen = labels && n > 0;
   if (track && objs.n && ctx->cfg.batched && ctx->overlap_ctas != 0)
     return frame_overlapped(ctx, gen, all, objs, moving);
-  if (gen)
-    if (int rc = launch_generalize(ctx)) return rc;
-  if (int rc = track_preprocess(ctx)) return rc;
-  if (track) {
-    if (int rc = track_camera(ctx, moving)) return rc;
-    if (objs.n)
-      if (int rc = track_objects(ctx, objs)) return rc;
+  if (track && ctx->cfg.batched && ctx->overlap_ctas != 0) {   // no objects
+    if (int rc = pyramid_and_camera_pre(ctx, gen)) return rc;
+    if (int rc = track_camera_gn(ctx)) return rc;
+  } else {
+    if (gen)
+      if (int rc = launch_generalize(ctx)) return rc;
+    if (int rc = track_preprocess(ctx)) return rc;
+    if (track) {
+      if (int rc = track_camera(ctx, moving)) return rc;
+      if (objs.n)
+        if (int rc = track_objects(ctx, objs)) return rc;
+    }
   }
   if (ctx->cfg.batched) {
     if (int rc = stage_prepare(ctx, all, true)) return rc;
@@ -243,9 +274,14 @@ int process_frame_motion(Context* ctx, float thr, float moved, uint32_t* moving_
   if (!ctx->d_motion_rows) MF_CUDA(cudaMalloc(&ctx->d_motion_rows, 4 * WH));
   int8_t* cam_rows = ctx->d_motion_rows;
   int8_t* obj_rows = ctx->d_motion_rows + 2 * WH;
-  if (int rc = launch_generalize(ctx)) return rc;
-  if (int rc = track_preprocess(ctx)) return rc;
-  if (int rc = track_camera(ctx, 0)) return rc;
+  if (ctx->cfg.batched && ctx->overlap_ctas != 0) {
+    if (int rc = pyramid_and_camera_pre(ctx, true)) return rc;
+    if (int rc = track_camera_gn(ctx)) return rc;
+  } else {
+    if (int rc = launch_generalize(ctx)) return rc;
+    if (int rc = track_preprocess(ctx)) return rc;
+    if (int rc = track_camera(ctx, 0)) return rc;
+  }
   uint32_t moving = 0, again = 0;
   float ratio[MAX_INSTANCES];
   if (n > 1)
