@@ -186,6 +186,9 @@ int mf_create(const mf_config* cfg, mf_context** out) {
   cudaMemsetAsync(P.c, 0, nv * 4, ctx->stream);
   cudaMemsetAsync(P.fg, 0, nv * 8, ctx->stream);
   cudaMemsetAsync(P.w, 0, nv * 4, ctx->stream);
+  // no instance yet (-1): while one stream hands out slots, the other's visit
+  // list may already count one whose corner and instance are not written
+  cudaMemsetAsync(P.meta, 0xff, cap * sizeof(int4), ctx->stream);
   cudaMemsetAsync(P.active, 0, cap, ctx->stream);
   cudaMemsetAsync(P.count, 0, sizeof(int), ctx->stream);
   cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream);

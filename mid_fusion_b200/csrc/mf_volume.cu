@@ -362,7 +362,9 @@ visit_list_kernel(Pool pool, const Volume* __restrict__ vols,
   bool take = false;
   if (slot < *pool.count) {
     const int4 m = pool.meta[slot];
-    if ((inst_mask >> m.w) & 1u) {
+    // a slot that the other stream's allocation has counted but not written
+    // yet (w < 0) belongs to that stream's instances
+    if (m.w >= 0 && ((inst_mask >> m.w) & 1u)) {
       if (pool.active[slot]) {
         take = true;
       } else {
