@@ -542,8 +542,10 @@ int mf_set_gn_persistent(mf_context* ctx, int enable);
  * run on a low-priority side stream while the objects are tracked on the
  * context's stream (highest priority); the objects' allocation and
  * integration follow.  ctas < 0 (the default): the integration launch shape's
- * own grid; ctas > 0: that many integration CTAs; 0: everything in order on
- * the context's stream.  The volumes and poses are the in-order frame's (pool
+ * own grid; ctas > 0: as many integration threads as that many CTAs of 512; 0:
+ * everything in order on the context's stream.  Frames without objects, and
+ * mf_process_frame_motion, set up the camera's problem and the masks beside the
+ * pyramid unless it is 0.  The volumes and poses are the in-order frame's (pool
  * slots are handed out in another order).  Applies to frames captured after
  * the call. */
 int mf_set_overlap(mf_context* ctx, int ctas);
@@ -568,7 +570,11 @@ int mf_tune_describe(int stage, int variant, char* buf, int cap);
  * best of 3 trials, CUDA events) and keeps the fastest of each; the current
  * choice stays unless another is more than 1 % faster.  raycast_us and
  * integrate_us (MF_TUNE_MAX_VARIANTS floats each, may be NULL) receive the
- * microseconds per launch of every candidate.  Needs a processed frame (the
+ * microseconds per launch of every candidate; in a context whose frames overlap
+ * (mf_set_overlap) a phased raycast's time leaves out the background's marches,
+ * which such frames run beside the objects' tracking.  Until a raycast shape is
+ * chosen, by this call or mf_tune_set, overlapped frames use the phased one
+ * (same maps).  Needs a processed frame (the
  * instances, the frame inputs and the map of the last mf_process_frame or
  * mf_integrate).  Leaves the map and the model maps unchanged: the raycasts
  * write scratch maps and the integrations update a scratch copy of the pool

@@ -884,7 +884,16 @@ int stage_raycast_to(Context* ctx, const IdList& ids, float epsilon, F3* vertex,
   return MF_OK;
 }
 
-bool raycast_is_phased(const Context* ctx) { return ray_variants[ctx->tune.ray].fn == nullptr; }
+// The shape of an overlapped frame's raycast.  Until one is chosen it is the
+// phased one with 8x16 tiles: alone it is as fast as one kernel (107 against
+// 106-113 us at 640x480, 341 against 326-361 at 1280x720), but its
+// background marches run beside the objects' tracking, so that only the
+// objects' marches and the fold are on the frame's critical path.  Frame with
+// six objects at 1280x720: 1823 us with one kernel, 1768 so.
+static const RayVariant& overlapped_ray(const Context* ctx) {
+  return ray_variants[ctx->tune.ray_chosen ? ctx->tune.ray : N_RAY_VARIANTS - 1];
+}
+bool raycast_is_phased(const Context* ctx) { return overlapped_ray(ctx).fn == nullptr; }
 
 // The phased composite in parts: the per-instance marches of `ids` into the
 // records of list positions base .. base + ids.n - 1 (each instance's march
@@ -892,7 +901,7 @@ bool raycast_is_phased(const Context* ctx) { return ray_variants[ctx->tune.ray].
 // with a phased launch shape (raycast_is_phased).
 int stage_raycast_hits(Context* ctx, const IdList& ids, int base, float epsilon) {
   if (ids.n == 0) return MF_OK;
-  const RayVariant& r = ray_variants[ctx->tune.ray];
+  const RayVariant& r = overlapped_ray(ctx);
   if (r.fn || base < 0 || base + ids.n > ctx->cfg.max_instances) return MF_E_STATE;
   const mf_config& c = ctx->cfg;
   RayArgs a{ctx->d_vertex, ctx->d_normal, ctx->d_label, ctx->W, ctx->H, c.near_plane,
@@ -908,7 +917,7 @@ int stage_raycast_hits(Context* ctx, const IdList& ids, int base, float epsilon)
 
 int stage_raycast_fold(Context* ctx, const IdList& ids, float epsilon) {
   if (ids.n == 0) return MF_OK;
-  const RayVariant& r = ray_variants[ctx->tune.ray];
+  const RayVariant& r = overlapped_ray(ctx);
   if (r.fn || ids.n > ctx->cfg.max_instances) return MF_E_STATE;
   const mf_config& c = ctx->cfg;
   RayArgs a{ctx->d_vertex, ctx->d_normal, ctx->d_label, ctx->W, ctx->H, c.near_plane,

@@ -1584,7 +1584,8 @@ __device__ __forceinline__ void gn_copy_state(const GNState* from, GNState* to) 
 // the FP64 of the weights included), then the serial tail of an iteration
 // (barrier, row sums, step).  One launch per iteration, chained by
 // programmatic dependent launch, with the step in the CTA that finished last,
-// took 260 us for a frame's iterations (ncu, their sum); this launch takes 130.
+// took 342 us for a frame's iterations at 640x480 (ncu, their sum); this launch
+// takes 175 (160x120: 19 iterations of 11 us in launches, now 89 in all).
 __global__ void __launch_bounds__(GN_BLOCK, 1)
 gn_camera_kernel(GNArgs a, GNLoop g) {
   extern __shared__ __align__(16) unsigned char gn_smem[];
@@ -2604,7 +2605,7 @@ int track_download_level(Context* ctx, int L, int which, float* out) {
 // Normal-equation evaluation that allocates nothing (mf_track_eval_static).
 //
 // Same sums as track_eval (the per-pixel rows and the FP64 reduction of
-// gn_iter_kernel, in the same order, so the two agree bit for bit), but the
+// gn_eval_kernel, in the same order, so the two agree bit for bit), but the
 // scratch -- the per-CTA FP64 partials, the 32 result sums and the CTA ticket
 // -- is the file-scope array below, not a cudaMalloc'd buffer, and the pose is
 // a kernel argument, so the context's GN state is not touched either.
@@ -2872,7 +2873,7 @@ int gn_step_check(Context* ctx, int n, const double* state, const double* sums, 
 //
 //   E(T_live, tsdf) = sum_p rho(e_icp(p)) + rho(e_rgb(p))
 //
-// with the camera rows of gn_iter_kernel (the same validity tests, residuals,
+// with the camera rows of the GN (the same validity tests, residuals,
 // whitening and robust kernel) at level 0.  Per valid row the kernel adds
 // rho'(e) de/d(twist) -- the exact derivative for a left perturbation
 // T <- exp(twist) T_live, with the bilinear image gradient of the photometric
