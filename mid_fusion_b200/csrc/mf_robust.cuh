@@ -32,39 +32,39 @@ namespace mf {
 // r = 1 / (1 + j / 64) rounded to nearest, and -log(r)
 struct alignas(16) LogEntry { double r, t; };
 MF_ROBUST_TABLE(LogEntry, log_64, {
-    {0x1p+0, 0x0p+0}, {0x1.f81f81f81f820p-1, 0x1.fc0a8b0fc03c4p-7},
-    {0x1.f07c1f07c1f08p-1, 0x1.f829b0e7832f8p-6}, {0x1.e9131abf0b767p-1, 0x1.77458f632dcffp-5},
-    {0x1.e1e1e1e1e1e1ep-1, 0x1.f0a30c01162a8p-5}, {0x1.dae6076b981dbp-1, 0x1.341d7961bd1d0p-4},
-    {0x1.d41d41d41d41dp-1, 0x1.6f0d28ae56b4ep-4}, {0x1.cd85689039b0bp-1, 0x1.a926d3a4ad562p-4},
-    {0x1.c71c71c71c71cp-1, 0x1.e27076e2af2eap-4}, {0x1.c0e070381c0e0p-1, 0x1.0d77e7cd08e5bp-3},
-    {0x1.bacf914c1bad0p-1, 0x1.29552f81ff521p-3}, {0x1.b4e81b4e81b4fp-1, 0x1.44d2b6ccb7d1cp-3},
-    {0x1.af286bca1af28p-1, 0x1.5ff3070a793d6p-3}, {0x1.a98ef606a63bep-1, 0x1.7ab890210d907p-3},
-    {0x1.a41a41a41a41ap-1, 0x1.9525a9cf456b6p-3}, {0x1.9ec8e951033d9p-1, 0x1.af3c94e80bff3p-3},
-    {0x1.999999999999ap-1, 0x1.c8ff7c79a9a20p-3}, {0x1.948b0fcd6e9e0p-1, 0x1.e27076e2af2e8p-3},
-    {0x1.8f9c18f9c18fap-1, 0x1.fb9186d5e3e29p-3}, {0x1.8acb90f6bf3aap-1, 0x1.0a324e27390e2p-2},
-    {0x1.8618618618618p-1, 0x1.1675cababa60fp-2}, {0x1.8181818181818p-1, 0x1.22941fbcf7966p-2},
-    {0x1.7d05f417d05f4p-1, 0x1.2e8e2bae11d31p-2}, {0x1.78a4c8178a4c8p-1, 0x1.3a64c556945eap-2},
-    {0x1.745d1745d1746p-1, 0x1.4618bc21c5ec2p-2}, {0x1.702e05c0b8170p-1, 0x1.51aad872df82ep-2},
-    {0x1.6c16c16c16c17p-1, 0x1.5d1bdbf5809cap-2}, {0x1.6816816816817p-1, 0x1.686c81e9b14adp-2},
-    {0x1.642c8590b2164p-1, 0x1.739d7f6bbd007p-2}, {0x1.6058160581606p-1, 0x1.7eaf83b82afc2p-2},
-    {0x1.5c9882b931057p-1, 0x1.89a3386c1425bp-2}, {0x1.58ed2308158edp-1, 0x1.947941c2116fbp-2},
-    {0x1.5555555555555p-1, 0x1.9f323ecbf984dp-2}, {0x1.51d07eae2f815p-1, 0x1.a9cec9a9a084ap-2},
-    {0x1.4e5e0a72f0539p-1, 0x1.b44f77bcc8f64p-2}, {0x1.4afd6a052bf5bp-1, 0x1.beb4d9da71b7ap-2},
-    {0x1.47ae147ae147bp-1, 0x1.c8ff7c79a9a21p-2}, {0x1.446f86562d9fbp-1, 0x1.d32fe7e00ebd5p-2},
-    {0x1.4141414141414p-1, 0x1.dd46a04c1c4a1p-2}, {0x1.3e22cbce4a902p-1, 0x1.e744261d68789p-2},
-    {0x1.3b13b13b13b14p-1, 0x1.f128f5faf06ecp-2}, {0x1.3813813813814p-1, 0x1.faf588f78f31dp-2},
-    {0x1.3521cfb2b78c1p-1, 0x1.02552a5a5d0ffp-1}, {0x1.323e34a2b10bfp-1, 0x1.0723e5c1cdf41p-1},
-    {0x1.2f684bda12f68p-1, 0x1.0be72e4252a83p-1}, {0x1.2c9fb4d812ca0p-1, 0x1.109f39e2d4c96p-1},
-    {0x1.29e4129e4129ep-1, 0x1.154c3d2f4d5eap-1}, {0x1.27350b8812735p-1, 0x1.19ee6b467c96fp-1},
-    {0x1.2492492492492p-1, 0x1.1e85f5e7040d1p-1}, {0x1.21fb78121fb78p-1, 0x1.23130d7bebf43p-1},
-    {0x1.1f7047dc11f70p-1, 0x1.2795e1289b11bp-1}, {0x1.1cf06ada2811dp-1, 0x1.2c0e9ed448e8cp-1},
-    {0x1.1a7b9611a7b96p-1, 0x1.307d7334f10bep-1}, {0x1.1811811811812p-1, 0x1.34e289d9ce1d2p-1},
-    {0x1.15b1e5f75270dp-1, 0x1.393e0d3562a1ap-1}, {0x1.135c81135c811p-1, 0x1.3d9026a7156fbp-1},
-    {0x1.1111111111111p-1, 0x1.41d8fe84672afp-1}, {0x1.0ecf56be69c90p-1, 0x1.4618bc21c5ec2p-1},
-    {0x1.0c9714fbcda3bp-1, 0x1.4a4f85db03ebbp-1}, {0x1.0a6810a6810a7p-1, 0x1.4e7d811b75bb0p-1},
-    {0x1.0842108421084p-1, 0x1.52a2d265bc5abp-1}, {0x1.0624dd2f1a9fcp-1, 0x1.56bf9d5b3f399p-1},
-    {0x1.0410410410410p-1, 0x1.5ad404c359f2dp-1}, {0x1.0204081020408p-1, 0x1.5ee02a9241676p-1},
-    {0x1.0000000000000p-1, 0x1.62e42fefa39efp-1},
+    {1.0, 0.0}, {0.9846153846153847, 0.015504186535965199},
+    {0.9696969696969697, 0.03077165866675366}, {0.9552238805970149, 0.04580953603129422},
+    {0.9411764705882353, 0.060624621816434854}, {0.927536231884058, 0.07522342123758752},
+    {0.9142857142857143, 0.08961215868968717}, {0.9014084507042254, 0.10379679368164355},
+    {0.8888888888888888, 0.11778303565638351}, {0.8767123287671232, 0.13157635778871932},
+    {0.8648648648648649, 0.14518200984449783}, {0.8533333333333334, 0.15860503017663852},
+    {0.8421052631578947, 0.17185025692665928}, {0.8311688311688312, 0.18492233849401193},
+    {0.8205128205128205, 0.19782574332991992}, {0.810126582278481, 0.21056476910734964},
+    {0.8, 0.2231435513142097}, {0.7901234567901234, 0.23556607131276697},
+    {0.7804878048780488, 0.2478361639045812}, {0.7710843373493976, 0.259957524436926},
+    {0.7619047619047619, 0.2719337154836418}, {0.7529411764705882, 0.2837681731306446},
+    {0.7441860465116279, 0.2954642128938359}, {0.735632183908046, 0.3070250352949119},
+    {0.7272727272727273, 0.3184537311185346}, {0.7191011235955056, 0.32975328637246804},
+    {0.7111111111111111, 0.3409265869705932}, {0.7032967032967034, 0.3519764231571781},
+    {0.6956521739130435, 0.3629054936893685}, {0.6881720430107527, 0.373716409793584},
+    {0.6808510638297872, 0.38441169891033206}, {0.6736842105263158, 0.394993808240869},
+    {0.6666666666666666, 0.40546510810816444}, {0.6597938144329897, 0.415827895143711},
+    {0.6530612244897959, 0.42608439531090014}, {0.6464646464646465, 0.43623676677491796},
+    {0.64, 0.4462871026284195}, {0.6336633663366337, 0.4562374334815876},
+    {0.6274509803921569, 0.46608972992459924}, {0.6213592233009708, 0.475845904869964},
+    {0.6153846153846154, 0.48550781578170077}, {0.6095238095238096, 0.4950772667978514},
+    {0.6037735849056604, 0.5045560107523953}, {0.5981308411214953, 0.5139457511022344},
+    {0.5925925925925926, 0.5232481437645479}, {0.5871559633027523, 0.5324647988694717},
+    {0.5818181818181818, 0.5415972824327444}, {0.5765765765765766, 0.5506471179526623},
+    {0.5714285714285714, 0.5596157879354228}, {0.5663716814159292, 0.5685047353526688},
+    {0.5614035087719298, 0.5773153650348236}, {0.5565217391304348, 0.5860490450035782},
+    {0.5517241379310345, 0.5947071077466928}, {0.5470085470085471, 0.6032908514380841},
+    {0.5423728813559322, 0.6118015411059929}, {0.5378151260504201, 0.6202404097518576},
+    {0.5333333333333333, 0.6286086594223742}, {0.5289256198347108, 0.6369074622370692},
+    {0.5245901639344263, 0.6451379613735847}, {0.5203252032520326, 0.6533012720127456},
+    {0.5161290322580645, 0.661398482245365}, {0.512, 0.6694306539426292},
+    {0.5079365079365079, 0.6773988235918061}, {0.5039370078740157, 0.6853040030989195},
+    {0.5, 0.6931471805599453},
 });
 
 // 1 / x up to about 2^-22, for x within [1, 1e30]
@@ -124,7 +124,7 @@ MF_ROBUST_HD double robust_log(double s) {
   p = fma(u, p, 1.0 / 3);
   p = fma(u, p, -1.0 / 2);
   p = fma(u * u, p, u);
-  return fma((double)((hi >> 20) - 1023), 0x1.62e42fefa39efp-1, t) + p;
+  return fma((double)((hi >> 20) - 1023), 0.6931471805599453, t) + p;
 }
 
 // robust() below, for the arguments and kinds where a cheaper evaluation gives
@@ -162,7 +162,7 @@ MF_ROBUST_HD bool robust_fast(float e, int kind, float& w, float& loss) {
     return true;
   }
   if (kind == 1) {
-    if (!(ae > 0x1.5851eap+0f && ae < 1e30f)) return false;
+    if (!(ae > 1.34499991f && ae < 1e30f)) return false;
     const double a = fabs(r), y0 = robust_rcp(ae);
     const double wd = 1.345 * fma(fma(-a, y0, 1.0), y0, y0);
     w = (float)wd;
@@ -177,10 +177,10 @@ MF_ROBUST_HD bool robust_fast(float e, int kind, float& w, float& loss) {
 MF_ROBUST_HD void robust(float e, int kind, float& w, float& loss) {
   // Within the quadratic part the double loss is 0.5 e^2 exactly, rounded once:
   // 0.5f * (e * e), unless e * e leaves the normal range (the double path then).
-  // 0x1.5851eap+0f is the largest float at most 1.345.
+  // 1.34499991f is the largest float at most 1.345.
   if (kind <= 1) {
     const float q = e * e;
-    if ((kind == 0 || fabsf(e) <= 0x1.5851eap+0f) && ((q >= 1e-30f && q <= 1e38f) || e == 0.f)) {
+    if ((kind == 0 || fabsf(e) <= 1.34499991f) && ((q >= 1e-30f && q <= 1e38f) || e == 0.f)) {
       w = 1.f;
       loss = 0.5f * q;
       return;

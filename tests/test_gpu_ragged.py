@@ -129,3 +129,60 @@ def test_mesh_block_order(size):
     known = order[order >= 0]
     assert len(known) >= 0.9 * len(tri)
     assert np.mean(np.diff(known) >= 0) > 0.98   # up to corners on a block's face
+
+
+def _half(a):
+    """The reference's robust half-sampling in float32, element by element in
+    its order (centre, right, below, diagonal)."""
+    h, w = a.shape[0] // 2, a.shape[1] // 2
+    c = a[0:2 * h:2, 0:2 * w:2]
+    s = np.zeros_like(c)
+    t = np.zeros_like(c)
+    for dy in (0, 1):
+        for dx in (0, 1):
+            v = a[dy:2 * h:2, dx:2 * w:2]
+            near = np.abs(v - c) < np.float32(np.float32(0.1) * 3)
+            s = np.where(near, s + np.float32(1), s)
+            t = np.where(near, t + v, t)
+    return t / s
+
+
+@pytest.mark.parametrize("W,H,levels", [(17, 19, 2), (97, 65, 3), (161, 119, 4), (350, 267, 4),
+                                        (64, 48, 1)])
+def test_pyramid_levels_at_ragged_sizes(W, H, levels):
+    """Every level of depth and intensity is the half-sampled finer level bit
+    for bit, and the vertex planes (live and rendered reference) have the
+    depth as z where there is one, at sizes that the 16 x 16 tiles do not
+    divide."""
+    s = make_scene("multi", W, H, n_frames=2, seed=5, n_objects=0)
+    ctx = Context(W, H, k=s.k, pool_blocks=1 << 14, gn_iterations=(2,) * levels)
+    ctx.add_instance(128, 5.12, np.eye(4, dtype=np.float32), 0)
+    ctx.set_camera_pose(s.cam_poses[0])
+    for f in range(2):
+        d, rgb, lab = s.render(f)
+        d = np.array(d, np.float32)
+        d[H // 3:H // 3 + 3, :W // 2] = 0   # missing depths
+        ctx.upload(d, rgb)
+        ctx.upload_labels(lab)
+        ctx.preprocess()
+        if f:
+            ctx.track_camera([])
+        ctx.integrate([0])
+        ctx.raycast()
+        if f == 0:
+            ctx.set_ref_from_current()
+    for which in (0, 1):
+        for l in range(1, levels):
+            fine = ctx.pyramid(l - 1, which)
+            got = ctx.pyramid(l, which)
+            assert np.array_equal(got, _half(fine)[:got.shape[0], :got.shape[1]]), (which, l)
+    ref = ctx.pyramid(0, 7)[..., 2]
+    for l in range(levels):
+        d = ctx.pyramid(l, 0)
+        assert np.array_equal(ctx.pyramid(l, 2)[..., 2], np.where(d > 0, d, np.float32(0)))
+        if l:
+            ref = _half(ref)
+        got = ctx.pyramid(l, 7)[..., 2]
+        assert np.array_equal(got, np.where(ref > 0, ref, np.float32(0))[:got.shape[0],
+                                                                        :got.shape[1]]), l
+    ctx.close()

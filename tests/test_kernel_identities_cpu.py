@@ -113,3 +113,48 @@ def test_block_coordinate_by_a_round_down_addition():
     down = (np.floor((f.astype(np.float64) + big) / 8) * 8).astype(np.float32)
     bits = down.view(np.uint32) - np.uint32(0x4cc00000)
     assert np.array_equal(bits, (f.astype(np.int64) >> 3).astype(np.uint32))
+
+
+def test_cheap_robust_weights_equal_the_double_formulas(tmp_path):
+    """robust_fast (mf_robust.cuh), compiled for the host, returns the floats of
+    the double formulas, or leaves the residual to them: thresholds, residuals
+    across each kernel's range, extremes, infinities and NaN."""
+    import ctypes as C
+    import os
+    import subprocess
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                        "mid_fusion_b200", "csrc")
+    src = tmp_path / "r.cpp"
+    src.write_text('#include "mf_robust.cuh"\n'
+                   'extern "C" void run(int kind, const float* e, int n, float* w, float* l, '
+                   'int* fast) { for (int i = 0; i < n; ++i) '
+                   'fast[i] = mf::robust_fast(e[i], kind, w[i], l[i]); }\n')
+    so = tmp_path / "r.so"
+    subprocess.run(["g++", "-O2", "-std=c++14", "-ffp-contract=off", "-fPIC", "-shared", "-I",
+                    csrc, "-o", str(so), str(src)], check=True)
+    lib = C.CDLL(str(so))
+    rng = np.random.default_rng(6)
+    e = np.concatenate([
+        rng.normal(scale=s, size=200000) for s in (1e-3, 0.5, 3.0, 50.0)] + [
+        np.exp(rng.uniform(-80, 80, 100000)),
+        [0.0, 1.345, 4.6851, 2.3849, 1e-30, 1e-45, 3e38, np.inf, np.nan]]).astype(np.float32)
+    e = np.concatenate([e, -e, np.nextafter(np.float32([1.345, 4.6851]), np.float32(9))])
+    w, loss = np.zeros_like(e), np.zeros_like(e)
+    fast = np.zeros(e.size, np.int32)
+    p = lambda a: a.ctypes.data_as(C.c_void_p)
+    r = e.astype(np.float64)
+    a = np.abs(r)
+    with np.errstate(all="ignore"):
+        x2 = (r / 2.3849) * (r / 2.3849)
+        u = 1.0 - r * r / (4.6851 * 4.6851)
+        v = 1.0 - (r / 4.6851) * (r / 4.6851)
+        want = {1: (1.345 / a, 1.345 * (a - 0.5 * 1.345), a > 1.345),
+                2: (u * u, 4.6851 * 4.6851 / 6.0 * (1.0 - v * v * v), a <= 4.6851),
+                3: (1 / (1 + x2), 0.5 * 2.3849 * 2.3849 * np.log(1.0 + x2), a < 1e15)}
+        for kind, (ww, ll, domain) in want.items():
+            lib.run(kind, p(e), e.size, p(w), p(loss), p(fast))
+            on = fast != 0
+            assert not np.any(on & ~domain)
+            assert np.count_nonzero(on) > 0.999 * np.count_nonzero(domain & (a < 1e14))
+            assert np.array_equal(w[on], ww[on].astype(np.float32)), kind
+            assert np.array_equal(loss[on], ll[on].astype(np.float32)), kind
