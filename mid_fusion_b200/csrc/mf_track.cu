@@ -1743,7 +1743,9 @@ __device__ __forceinline__ bool object_segment_live(const GNArgs& a, const GOSha
       floorf(qy1) + 3.f >= (float)S.box[1] && floorf(qy0) - 2.f <= (float)S.box[3])
     return true;
   // the frustum's box in the live camera: x and y reach z times the directions
-  const float x0 = fminf(zr.x * xs[0], zr.y * xs[0]), x1 = fmaxf(zr.x * xs[1], zr.y * xs[1]);
+  // (which run from right to left, or from below, for a negative focal length)
+  const float xlo = fminf(xs[0], xs[1]), xhi = fmaxf(xs[0], xs[1]);
+  const float x0 = fminf(zr.x * xlo, zr.y * xlo), x1 = fmaxf(zr.x * xhi, zr.y * xhi);
   const float ylo = fminf(ys[0], ys[1]), yhi = fmaxf(ys[0], ys[1]);
   const float y0 = fminf(zr.x * ylo, zr.y * ylo), y1 = fmaxf(zr.x * yhi, zr.y * yhi);
   const float ox = fmaxf(fmaxf(x0 - sm.origin.x, sm.origin.x - x1), 0.f);

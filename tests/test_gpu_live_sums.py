@@ -96,3 +96,40 @@ def test_live_sums_equal_the_evaluation(W, H, objects, level, kw):
     assert W < 97 or any(rows[1:])
     assert ctx.status() & 32 == 0
     ctx.close()
+
+
+def _far_wall_to_origin(s, px, normal):
+    """The rigid motion of the world that brings the point of the far wall (z =
+    room_hi[2]) that frame 1 sees at column px, middle row, to the origin, and
+    the wall's normal (facing the room) to `normal` times the x axis."""
+    fx, fy, cx, cy = [float(v) for v in s.k]
+    T = s.cam_poses[1]
+    d = T[:3, :3] @ np.array([(px - cx) / fx, 0.0, 1.0])
+    p = T[:3, 3] + d * (s.room_hi[2] - T[2, 3]) / d[2]
+    R = np.array([[0, 0, -normal], [0, 1, 0], [normal, 0, 0]], np.float64)
+    D = np.eye(4)
+    D[:3, :3] = R
+    D[:3, 3] = -R @ p
+    return D
+
+
+@pytest.mark.parametrize("fx_sign", [1.0, -1.0])
+@pytest.mark.parametrize("normal", [1.0, -1.0])
+@pytest.mark.parametrize("level", [0, 1])
+def test_pixels_beside_the_object_near_the_world_origin(fx_sign, normal, level):
+    """Beside an object its model map holds (0, 0, 0) with an invalid normal,
+    whose bilinear interpolation may round to a valid one: a live point within
+    10 cm of the world origin then has a row.  Segments there are evaluated for
+    either sign of the focal length (x runs from right to left for fx < 0)."""
+    W, H = 161, 119
+    s = make_scene("multi", W, H, n_frames=2, seed=13, bg_size=128, obj_size=64, n_objects=1)
+    s.statics = []
+    s.k = s.k * np.array([fx_sign, 1, 1, 1], np.float32)
+    _, _, lab = s.render(1)
+    # a column away from the object
+    px = W - 30 if np.nonzero(lab == 1)[1].mean() < W / 2 else 30
+    ctx = _second_frame(s, _far_wall_to_origin(s, px, normal), robust="huber", use_rgb=False,
+                        gn_iterations=(0,) * level + (2,))
+    for i in range(2):
+        _compare(ctx, i, level, counts=i == 0)
+    ctx.close()
