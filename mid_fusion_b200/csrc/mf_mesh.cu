@@ -27,13 +27,21 @@ namespace mf {
 // its first corner to its second
 __constant__ int8_t c_corner[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 0, 1}, {0, 0, 1},
                                       {0, 1, 0}, {1, 1, 0}, {1, 1, 1}, {0, 1, 1}};
-__constant__ int8_t c_edge[12][2] = {{0, 1}, {1, 2}, {2, 3}, {0, 3}, {4, 5}, {5, 6},
-                                     {6, 7}, {4, 7}, {0, 4}, {1, 5}, {2, 6}, {3, 7}};
+#define MF_EDGE_CORNERS                                           \
+  {{0, 1}, {1, 2}, {2, 3}, {0, 3}, {4, 5}, {5, 6}, {6, 7}, {4, 7}, \
+   {0, 4}, {1, 5}, {2, 6}, {3, 7}}
+__constant__ int8_t c_edge[12][2] = MF_EDGE_CORNERS;
+static const int8_t edge_corners[12][2] = MF_EDGE_CORNERS;   // the host's
+
+// A row that lists an edge whose two corners are on the same side (a caller's
+// table may): its vertices lie anywhere on the edge's line, or nowhere.
+constexpr int ROW_ANY_EDGE = 0x80;
 
 struct MeshArgs {
   Pool pool;
   Volume V;
   const int8_t* tris;      // triangulation table, 256 x 3 * MF_MC_MAX_TRIS edge indices
+  const uint8_t* rows;     // triangles of each table row, with ROW_ANY_EDGE
   const int* slots;        // the instance's blocks, Morton order
   const int* n_blocks;
   const long long* offset; // first triangle of each block (pass 2)
@@ -50,7 +58,7 @@ struct MeshTile {
   int slot[8];             // the block and its upper neighbours
   int8_t corner[8];        // a cell corner's offset, as bits x | y << 1 | z << 2
   int8_t edge[12][2];
-  uint8_t n_tris[256];     // triangles of each table row
+  uint8_t rows[256];       // MeshArgs::rows
   int warp[16];
 };
 __device__ __forceinline__ int mesh_at(int x, int y, int z) {
@@ -86,9 +94,10 @@ __device__ __forceinline__ void mesh_load(const MeshArgs& a, MeshTile& s, int4 m
 }
 
 // meshing::compute_intersection (meshing.hpp:20-29) on edge e of the cell at
-// voxel (x, y, z), element `cell` of the tile
+// voxel (x, y, z), element `cell` of the tile; any_edge: the edge's corners may
+// be on the same side
 __device__ __forceinline__ F3 edge_vertex(const MeshArgs& a, const MeshTile& t, int cell, int x,
-                                          int y, int z, int e) {
+                                          int y, int z, int e, bool any_edge) {
   const float voxelSize = a.V.dim / a.V.size;
   const int c0 = t.corner[t.edge[e][0]], c1 = t.corner[t.edge[e][1]];
   const unsigned sx = x + (c0 & 1), sy = y + ((c0 >> 1) & 1), sz = z + (c0 >> 2);
@@ -100,8 +109,9 @@ __device__ __forceinline__ F3 edge_vertex(const MeshArgs& a, const MeshTile& t, 
   const float k = (float)(0.0 - v1);
   const float den = v2 - v1;
   // s + (k * (d - s)) / den: on the two axes along which the edge does not run
-  // the addend is +-0, unless k or den is not finite
-  if (fabsf(k) < INFINITY && fabsf(den) < INFINITY) {
+  // the addend is +-0, unless k or den is not finite, or den is 0 (which takes
+  // corners on the same side)
+  if (!any_edge && fabsf(k) < INFINITY && fabsf(den) < INFINITY) {
     const int axis = c0 ^ c1;   // one bit: the axis of the edge
     const float ss = axis == 1 ? s.x : axis == 2 ? s.y : s.z;
     const float ds = axis == 1 ? d.x : axis == 2 ? d.y : d.z;
@@ -124,12 +134,7 @@ __global__ void __launch_bounds__(512) mesh_kernel(MeshArgs a) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   if (t < 8) s.corner[t] = c_corner[t][0] | (c_corner[t][1] << 1) | (c_corner[t][2] << 2);
   if (t < 24) s.edge[t >> 1][t & 1] = c_edge[t >> 1][t & 1];
-  if (t < 256) {
-    const int8_t* tr = a.tris + t * (3 * MF_MC_MAX_TRIS);
-    int n = 0;
-    while (n < MF_MC_MAX_TRIS && tr[3 * n] != -1) ++n;
-    s.n_tris[t] = (uint8_t)n;
-  }
+  if (t < 256) s.rows[t] = a.rows[t];
   const float voxelSize = a.V.dim / a.V.size;
   const int nb = *a.n_blocks;
   const int bound = a.V.size - 1;  // clamp(corner + 8, 0, size - 1)
@@ -155,14 +160,17 @@ __global__ void __launch_bounds__(512) mesh_kernel(MeshArgs a) {
     }
     // kept triangles of this cell, in table order
     const int8_t* tr = a.tris + index * (3 * MF_MC_MAX_TRIS);
-    // a vertex lies between its edge's corners, so only cells next to 0 or
-    // within two voxels of the bound can have one outside
-    unsigned keep = (1u << s.n_tris[index]) - 1u;
-    if (keep && !(x > 0 && y > 0 && z > 0 && (max(x, max(y, z)) + 2) * voxelSize <= a.bound))
+    // the vertex of an edge whose corners are on different sides lies between
+    // them, so only cells next to 0 or within two voxels of the bound can have
+    // one outside
+    const bool any_edge = s.rows[index] & ROW_ANY_EDGE;
+    unsigned keep = (1u << (s.rows[index] & ~ROW_ANY_EDGE)) - 1u;
+    if (keep && (any_edge || !(x > 0 && y > 0 && z > 0 &&
+                               (max(x, max(y, z)) + 2) * voxelSize <= a.bound)))
       for (int e = 0; e < 3 * MF_MC_MAX_TRIS && tr[e] != -1; e += 3)
-        if (outside_dim(edge_vertex(a, s, cell, x, y, z, tr[e]), a.bound) ||
-            outside_dim(edge_vertex(a, s, cell, x, y, z, tr[e + 1]), a.bound) ||
-            outside_dim(edge_vertex(a, s, cell, x, y, z, tr[e + 2]), a.bound))
+        if (outside_dim(edge_vertex(a, s, cell, x, y, z, tr[e], any_edge), a.bound) ||
+            outside_dim(edge_vertex(a, s, cell, x, y, z, tr[e + 1], any_edge), a.bound) ||
+            outside_dim(edge_vertex(a, s, cell, x, y, z, tr[e + 2], any_edge), a.bound))
           keep &= ~(1u << (e / 3));
     const int kept = __popc(keep);
     // exclusive scan of the cells' counts in thread (cell) order
@@ -193,7 +201,7 @@ __global__ void __launch_bounds__(512) mesh_kernel(MeshArgs a) {
       if (!(keep & 1u)) continue;
 #pragma unroll
       for (int c = 0; c < 3; ++c, o += 3) {
-        const F3 v = edge_vertex(a, s, cell, x, y, z, tr[3 * k + c]);
+        const F3 v = edge_vertex(a, s, cell, x, y, z, tr[3 * k + c], any_edge);
         o[0] = v.x;
         o[1] = v.y;
         o[2] = v.z;
@@ -294,7 +302,11 @@ mesh_offsets_kernel(const int* __restrict__ count, const int* __restrict__ n_blo
 // ints, edge triples ended by -1, the layout of the reference's triTable,
 // lib/algorithms/edge_tables.h), or the built-in one when table is NULL.
 int mesh_set_table(Context* ctx, const int* table) {
-  int8_t t[256][3 * MF_MC_MAX_TRIS];
+  struct {
+    int8_t t[256][3 * MF_MC_MAX_TRIS];
+    uint8_t rows[256];   // MeshArgs::rows, behind the table on the device
+  } host;
+  auto& t = host.t;
   if (!table) {
     std::memcpy(t, MF_MC_TRIS, sizeof(t));
   } else {
@@ -317,8 +329,18 @@ int mesh_set_table(Context* ctx, const int* table) {
       }
     }
   }
-  if (!ctx->d_mc_tris) MF_CUDA(cudaMalloc(&ctx->d_mc_tris, sizeof(t)));
-  MF_CUDA(cudaMemcpyAsync(ctx->d_mc_tris, t, sizeof(t), cudaMemcpyHostToDevice, ctx->stream));
+  for (int r = 0; r < 256; ++r) {
+    int n = 0;
+    bool any_edge = false;
+    for (; n < 3 * MF_MC_MAX_TRIS && t[r][n] != -1; ++n) {
+      const int8_t* e = edge_corners[t[r][n]];
+      any_edge = any_edge || ((r >> e[0]) & 1) == ((r >> e[1]) & 1);
+    }
+    host.rows[r] = (uint8_t)(n / 3 | (any_edge ? ROW_ANY_EDGE : 0));
+  }
+  if (!ctx->d_mc_tris) MF_CUDA(cudaMalloc(&ctx->d_mc_tris, sizeof(host)));
+  MF_CUDA(cudaMemcpyAsync(ctx->d_mc_tris, &host, sizeof(host), cudaMemcpyHostToDevice,
+                          ctx->stream));
   MF_CUDA(cudaStreamSynchronize(ctx->stream));
   return MF_OK;
 }
@@ -350,6 +372,7 @@ int mesh_volume(Context* ctx, int id, int float_bounds, float* tris, long long c
                                                              d_slots, cap_blocks, d_nblocks);
   MeshArgs a;
   a.tris = ctx->d_mc_tris;
+  a.rows = (const uint8_t*)ctx->d_mc_tris + 256 * 3 * MF_MC_MAX_TRIS;
   a.pool = ctx->pool;
   a.V = V;
   a.slots = d_slots;
