@@ -105,8 +105,8 @@ struct TrackState {
   double* d_gmodel = nullptr;       // 2 x 3 x W x H: dE/d model vertex, dE/d model normal
   double* d_cost_part = nullptr;    // per-CTA partials of the cost rows, 8 each
   double* d_cost = nullptr;         // 8: cost, dE/d twist (6), rows
-  uint8_t* d_win = nullptr;         // W x H: the raycast's winner per pixel, and its hit
-  F4* d_win_hit = nullptr;
+  F4* d_win_hit = nullptr;          // W x H: the hit of the raycast's winner per pixel (for
+  uint8_t* d_win = nullptr;         // TSDF gradients), and behind them the winners
   int cost_blocks = 0;
   // motion residuals (allocated on first use)
   int8_t* d_mres = nullptr;         // 2 x W x H result codes: ICP rows, then photometric
@@ -3060,10 +3060,6 @@ int camera_cost(Context* ctx, const float* T_live16, int want_grad, double* out8
   if (!T.d_cost) {
     MF_CUDA(cudaMalloc(&T.d_gmodel, sizeof(double) * 6 * WH));
     MF_CUDA(cudaMalloc(&T.d_cost_part, sizeof(double) * 8 * nb));
-    MF_CUDA(cudaMalloc(&T.d_win, WH));
-    T.allocs.push_back(T.d_win);
-    MF_CUDA(cudaMalloc(&T.d_win_hit, sizeof(F4) * WH));
-    T.allocs.push_back(T.d_win_hit);
     MF_CUDA(cudaMalloc(&T.d_cost, sizeof(double) * 8));
     T.allocs.push_back(T.d_gmodel);
     T.allocs.push_back(T.d_cost_part);
@@ -3073,6 +3069,11 @@ int camera_cost(Context* ctx, const float* T_live16, int want_grad, double* out8
   // the model maps of the current TSDF at the current (reference) camera pose,
   // and with a TSDF gradient each pixel's winner
   const bool grad = want_grad && d_grad;
+  if (grad && !T.d_win_hit) {
+    MF_CUDA(cudaMalloc(&T.d_win_hit, (sizeof(F4) + 1) * WH));
+    T.allocs.push_back(T.d_win_hit);
+    T.d_win = (uint8_t*)(T.d_win_hit + WH);
+  }
   IdList all;
   all.n = (int)ctx->inst.size();
   for (int i = 0; i < all.n; ++i) all.v[i] = i;
