@@ -345,6 +345,11 @@ int mesh_set_table(Context* ctx, const int* table) {
   return MF_OK;
 }
 
+// Scratch for a mesh that a context keeps between calls: 1.8 million
+// triangles, six times those of a 3.2 m room at 1 cm.  A larger mesh allocates
+// for its call, so that a single export does not hold that much for good.
+constexpr size_t MESH_KEEP = 64 << 20;
+
 int mesh_volume(Context* ctx, int id, int float_bounds, float* tris, long long cap,
                 long long* n_tris) {
   if (!ctx->d_mc_tris)
@@ -393,7 +398,7 @@ int mesh_volume(Context* ctx, int id, int float_bounds, float* tris, long long c
   *n_tris = total;
   if (!tris || cap < total || total == 0) return MF_OK;
   // the triangles: straight into a device destination, else through scratch
-  // that the context keeps (the largest mesh so far; mf_destroy frees it)
+  // that the context keeps up to MESH_KEEP (mf_destroy frees it)
   cudaPointerAttributes at{};
   const bool dev = cudaPointerGetAttributes(&at, tris) == cudaSuccess &&
                    (at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged);
@@ -406,12 +411,18 @@ int mesh_volume(Context* ctx, int id, int float_bounds, float* tris, long long c
     MF_CUDA(cudaMalloc(&ctx->d_mesh, bytes));
     ctx->mesh_bytes = bytes;
   }
-  a.out = dev ? tris : ctx->d_mesh;
+  float* const scratch = ctx->d_mesh;
+  a.out = dev ? tris : scratch;
   mesh_kernel<true><<<grid, 512, 0, ctx->stream>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess && !dev)
-    e = cudaMemcpyAsync(tris, ctx->d_mesh, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+    e = cudaMemcpyAsync(tris, scratch, bytes, cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  if (ctx->mesh_bytes > MESH_KEEP) {
+    cudaFree(ctx->d_mesh);
+    ctx->d_mesh = nullptr;
+    ctx->mesh_bytes = 0;
+  }
   if (e != cudaSuccess) {
     ctx->last_error = std::string("mf_mesh: ") + cudaGetErrorString(e);
     return MF_E_CUDA;

@@ -57,3 +57,25 @@ def test_cost_without_a_gradient_keeps_no_gradient_scratch():
     assert a[0] == b[0] == c[0] and a[2] == b[2] > 0
     assert float(grad.abs().max()) > 0
     ctx.close()
+
+
+def test_a_large_mesh_is_given_back():
+    """Up to 64 MiB of triangles on their way to host memory stay with the
+    context for the next call; more is freed before the call returns."""
+    s = make_scene("multi", 640, 480, n_frames=1, seed=4, n_objects=0, noise=False)
+    ctx = Context(640, 480, k=s.k, mu=0.02, pool_blocks=1 << 17, max_instances=1)
+    ctx.add_instance(2048, 5.12, np.eye(4, dtype=np.float32), 0)
+    d, rgb, lab = s.render(0)
+    ctx.set_camera_pose(s.cam_poses[0])
+    ctx.upload(d, rgb, generalize_masks(lab, [0]))
+    for _ in range(5):
+        ctx.integrate([0])
+    before = _free()
+    tri = ctx.mesh(0, float_bounds=True)
+    kept = before - _free()
+    assert tri.nbytes > 72 << 20, tri.nbytes
+    # next to the triangles the call keeps its block list and offsets: 16 B per
+    # block of the pool (and what the driver rounds up to)
+    assert kept <= 8 << 20, kept
+    assert np.array_equal(tri, ctx.mesh(0, float_bounds=True))
+    ctx.close()
