@@ -555,7 +555,11 @@ int mf_set_overlap(mf_context* ctx, int ctas);
  * their speed but not their results (each pixel / voxel is computed by one
  * thread from the same inputs in every shape):
  *   MF_TUNE_RAYCAST    the composite raycast (raycastObjectList): the pixel
- *                      tile of a 128-thread CTA and the register bound;
+ *                      tile of a 128-thread CTA and the register bound, or
+ *                      the phased form (per-instance marches, then a fold).
+ *                      Overlapped frames (mf_set_overlap) always run the
+ *                      phased form, in the chosen phased shape or else with
+ *                      8x16 tiles (same maps);
  *   MF_TUNE_INTEGRATE  the voxel-block integration (projective_functor::
  *                      update_block): 256-thread CTAs resident per SM.
  * Variant 0 of each is the default.  A context starts with the defaults. */
@@ -572,9 +576,7 @@ int mf_tune_describe(int stage, int variant, char* buf, int cap);
  * integrate_us (MF_TUNE_MAX_VARIANTS floats each, may be NULL) receive the
  * microseconds per launch of every candidate; in a context whose frames overlap
  * (mf_set_overlap) a phased raycast's time leaves out the background's marches,
- * which such frames run beside the objects' tracking.  Until a raycast shape is
- * chosen, by this call or mf_tune_set, overlapped frames use the phased one
- * (same maps).  Needs a processed frame (the
+ * which such frames run beside the objects' tracking.  Needs a processed frame (the
  * instances, the frame inputs and the map of the last mf_process_frame or
  * mf_integrate).  Leaves the map and the model maps unchanged: the raycasts
  * write scratch maps and the integrations update a scratch copy of the pool

@@ -62,7 +62,6 @@ struct TrackState;
 constexpr int MAX_TUNE_VARIANTS = MF_TUNE_MAX_VARIANTS;
 struct Tune {
   int ray = 0;        // raycast_objects_kernel (ray_variants, mf_raycast.cu)
-  bool ray_chosen = false;   // by mf_autotune or mf_tune_set (overlapped_ray, mf_raycast.cu)
   int integrate = 0;  // integrate_blocks_kernel (int_variants, mf_volume.cu)
   unsigned gen = 0;
 };
@@ -166,7 +165,7 @@ int stage_prepare(Context* ctx, const IdList& ids, bool reset = false);
 int stage_alloc(Context* ctx, const IdList& ids);
 int stage_integrate(Context* ctx, const IdList& ids, int ctas = 0);
 int stage_raycast(Context* ctx, const IdList& ids, float epsilon);
-bool raycast_is_phased(const Context* ctx);   // in an overlapped frame
+bool raycast_is_phased(const Context* ctx);
 int stage_raycast_hits(Context* ctx, const IdList& ids, int base, float epsilon);
 int stage_raycast_fold(Context* ctx, const IdList& ids, float epsilon);
 // The same raycast into other map buffers.

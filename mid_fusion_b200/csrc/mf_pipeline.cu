@@ -59,7 +59,6 @@ static int frame_overlapped(Context* ctx, bool gen, const IdList& all, const IdL
   IdList bg;
   bg.n = 1;
   bg.v[0] = 0;
-  const bool phased = raycast_is_phased(ctx);
   cudaStream_t main = ctx->stream, side = ctx->side;
   int rc = MF_OK;
   cudaError_t e = cudaSuccess;
@@ -93,7 +92,7 @@ static int frame_overlapped(Context* ctx, bool gen, const IdList& all, const IdL
   if (!rc) rc = stage_prepare(ctx, bg, true);
   if (!rc) rc = stage_alloc(ctx, bg);
   if (!rc) rc = stage_integrate(ctx, bg, ctx->overlap_ctas > 0 ? ctx->overlap_ctas : 0);
-  if (!rc && phased) rc = stage_raycast_hits(ctx, bg, 0, ctx->ray_epsilon);
+  if (!rc) rc = stage_raycast_hits(ctx, bg, 0, ctx->ray_epsilon);
   ok(cudaEventRecord(ctx->ev_join, side));
   std::swap(ctx->d_visit, ctx->d_visit_side);
   std::swap(ctx->d_visit_count, ctx->d_visit_count_side);
@@ -105,16 +104,14 @@ static int frame_overlapped(Context* ctx, bool gen, const IdList& all, const IdL
   if (!rc) rc = stage_prepare(ctx, objs, true);
   if (!rc) rc = stage_alloc(ctx, objs);
   if (!rc) rc = stage_integrate(ctx, objs);
-  if (!rc && phased) rc = stage_raycast_hits(ctx, objs, 1, ctx->ray_epsilon);
+  if (!rc) rc = stage_raycast_hits(ctx, objs, 1, ctx->ray_epsilon);
   ok(cudaStreamWaitEvent(main, ctx->ev_join, 0));
   if (rc) return rc;
   if (e != cudaSuccess) {
     ctx->last_error = std::string("overlapped frame: ") + cudaGetErrorString(e);
     return MF_E_CUDA;
   }
-  if (int rc2 = phased ? stage_raycast_fold(ctx, all, ctx->ray_epsilon)
-                       : stage_raycast(ctx, all, ctx->ray_epsilon))
-    return rc2;
+  if (int rc2 = stage_raycast_fold(ctx, all, ctx->ray_epsilon)) return rc2;
   return track_set_ref(ctx);
 }
 

@@ -833,7 +833,7 @@ struct RayVariant {
   HitsFn hits;
   FoldFn fold;
 };
-static const RayVariant ray_variants[] = {
+static constexpr RayVariant ray_variants[] = {
     {16, 1, raycast_objects_kernel<16, 1>, nullptr, nullptr},
     {32, 1, raycast_objects_kernel<32, 1>, nullptr, nullptr},
     {8, 1, raycast_objects_kernel<8, 1>, nullptr, nullptr},
@@ -849,6 +849,7 @@ static const RayVariant ray_variants[] = {
 };
 constexpr int N_RAY_VARIANTS = (int)(sizeof(ray_variants) / sizeof(ray_variants[0]));
 static_assert(N_RAY_VARIANTS <= MAX_TUNE_VARIANTS, "raycast candidate table too long");
+static_assert(ray_variants[N_RAY_VARIANTS - 1].fn == nullptr, "overlapped_ray: a phased shape");
 
 int ray_variant_count() { return N_RAY_VARIANTS; }
 
@@ -887,25 +888,27 @@ int stage_raycast_to(Context* ctx, const IdList& ids, float epsilon, F3* vertex,
   return MF_OK;
 }
 
-// The shape of an overlapped frame's raycast.  Until one is chosen it is the
-// phased one with 8x16 tiles: alone it is as fast as one kernel (107 against
-// 106-113 us at 640x480, 341 against 326-361 at 1280x720), but its
-// background marches run beside the objects' tracking, so that only the
-// objects' marches and the fold are on the frame's critical path.  Frame with
-// six objects at 1280x720: 1823 us with one kernel, 1768 so.
+bool raycast_is_phased(const Context* ctx) { return ray_variants[ctx->tune.ray].fn == nullptr; }
+
+// The shape of an overlapped frame's raycast: always a phased one, since its
+// background marches run beside the objects' tracking and only the objects'
+// marches and the fold are on the frame's critical path.  A context whose
+// raycast (MF_TUNE_RAYCAST) is one kernel takes 8x16 tiles here.  Frames, best
+// one-kernel shape against 8x16 phased (us): one object 160x120 492 / 480,
+// 640x480 583 / 551, 1280x720 1067 / 972; three at 640x480 733 / 693; twelve
+// uneven 1119 / 1083; six at 1280x720 1657 / 1668 (two runs differ by 10).
 static const RayVariant& overlapped_ray(const Context* ctx) {
-  return ray_variants[ctx->tune.ray_chosen ? ctx->tune.ray : N_RAY_VARIANTS - 1];
+  return ray_variants[raycast_is_phased(ctx) ? ctx->tune.ray : N_RAY_VARIANTS - 1];
 }
-bool raycast_is_phased(const Context* ctx) { return overlapped_ray(ctx).fn == nullptr; }
 
 // The phased composite in parts: the per-instance marches of `ids` into the
 // records of list positions base .. base + ids.n - 1 (each instance's march
-// is independent of the others'), and the fold over the whole list.  Only
-// with a phased launch shape (raycast_is_phased).
+// is independent of the others'), and the fold over the whole list, in the
+// overlapped frame's shape.
 int stage_raycast_hits(Context* ctx, const IdList& ids, int base, float epsilon) {
   if (ids.n == 0) return MF_OK;
   const RayVariant& r = overlapped_ray(ctx);
-  if (r.fn || base < 0 || base + ids.n > ctx->cfg.max_instances) return MF_E_STATE;
+  if (base < 0 || base + ids.n > ctx->cfg.max_instances) return MF_E_STATE;
   const mf_config& c = ctx->cfg;
   RayArgs a{ctx->d_vertex, ctx->d_normal, ctx->d_label, ctx->W, ctx->H, c.near_plane,
             c.far_plane, c.mu, epsilon};
@@ -921,7 +924,7 @@ int stage_raycast_hits(Context* ctx, const IdList& ids, int base, float epsilon)
 int stage_raycast_fold(Context* ctx, const IdList& ids, float epsilon) {
   if (ids.n == 0) return MF_OK;
   const RayVariant& r = overlapped_ray(ctx);
-  if (r.fn || ids.n > ctx->cfg.max_instances) return MF_E_STATE;
+  if (ids.n > ctx->cfg.max_instances) return MF_E_STATE;
   const mf_config& c = ctx->cfg;
   RayArgs a{ctx->d_vertex, ctx->d_normal, ctx->d_label, ctx->W, ctx->H, c.near_plane,
             c.far_plane, c.mu, epsilon};

@@ -109,7 +109,6 @@ int autotune(Context* ctx, int reps, float* ray_us, float* int_us) {
   const int nr = ray_variant_count();
   for (int v = 0; v < nr; ++v) {
     ctx->tune.ray = v;
-    ctx->tune.ray_chosen = true;
     int rc = time_launches(ctx, s, reps, 3, [&] {
       return stage_raycast_to(ctx, all, ctx->ray_epsilon, vert, norm, lab);
     }, &ray_us[v]);
@@ -158,9 +157,8 @@ int autotune(Context* ctx, int reps, float* ray_us, float* int_us) {
   MF_CUDA(cudaStreamSynchronize(ctx->stream));
   const int best_r = pick(ray_us, nr, before.ray);
   const int best_i = used > 0 ? pick(int_us, ni, before.integrate) : before.integrate;
-  if (best_r != before.ray || best_i != before.integrate || !before.ray_chosen) {
+  if (best_r != before.ray || best_i != before.integrate) {
     ctx->tune.ray = best_r;
-    ctx->tune.ray_chosen = true;
     ctx->tune.integrate = best_i;
     ++ctx->tune.gen;
   }
@@ -170,10 +168,8 @@ int autotune(Context* ctx, int reps, float* ray_us, float* int_us) {
 int tune_set(Context* ctx, int stage, int variant) {
   if (variant < 0 || variant >= tune_variant_count(stage)) return MF_E_ARG;
   int& slot = stage == MF_TUNE_RAYCAST ? ctx->tune.ray : ctx->tune.integrate;
-  const bool first = stage == MF_TUNE_RAYCAST && !ctx->tune.ray_chosen;
-  if (slot != variant || first) {
+  if (slot != variant) {
     slot = variant;
-    if (first) ctx->tune.ray_chosen = true;
     ++ctx->tune.gen;
   }
   return MF_OK;
