@@ -574,10 +574,9 @@ int mf_tune_describe(int stage, int variant, char* buf, int cap);
  * best of 3 trials, CUDA events) and keeps the fastest of each; the current
  * choice stays unless another is more than 1 % faster.  raycast_us and
  * integrate_us (MF_TUNE_MAX_VARIANTS floats each, may be NULL) receive the
- * microseconds per launch of every candidate; in a context whose frames overlap
- * (mf_set_overlap) a phased raycast's time leaves out the background's marches,
- * which such frames run beside the objects' tracking.  Needs a processed frame (the
- * instances, the frame inputs and the map of the last mf_process_frame or
+ * microseconds per launch of every candidate (of the whole raycast, as
+ * mf_raycast and every frame that does not overlap runs it).  Needs a processed
+ * frame (the instances, the frame inputs and the map of the last mf_process_frame or
  * mf_integrate).  Leaves the map and the model maps unchanged: the raycasts
  * write scratch maps and the integrations update a scratch copy of the pool
  * slots in use (allocated for the call and freed before it returns).  The

@@ -165,7 +165,6 @@ int stage_prepare(Context* ctx, const IdList& ids, bool reset = false);
 int stage_alloc(Context* ctx, const IdList& ids);
 int stage_integrate(Context* ctx, const IdList& ids, int ctas = 0);
 int stage_raycast(Context* ctx, const IdList& ids, float epsilon);
-bool raycast_is_phased(const Context* ctx);
 int stage_raycast_hits(Context* ctx, const IdList& ids, int base, float epsilon);
 int stage_raycast_fold(Context* ctx, const IdList& ids, float epsilon);
 // The same raycast into other map buffers.

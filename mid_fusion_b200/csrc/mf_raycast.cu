@@ -888,8 +888,6 @@ int stage_raycast_to(Context* ctx, const IdList& ids, float epsilon, F3* vertex,
   return MF_OK;
 }
 
-bool raycast_is_phased(const Context* ctx) { return ray_variants[ctx->tune.ray].fn == nullptr; }
-
 // The shape of an overlapped frame's raycast: always a phased one, since its
 // background marches run beside the objects' tracking and only the objects'
 // marches and the fold are on the frame's critical path.  A context whose
@@ -898,7 +896,8 @@ bool raycast_is_phased(const Context* ctx) { return ray_variants[ctx->tune.ray].
 // 640x480 583 / 551, 1280x720 1067 / 972; three at 640x480 733 / 693; twelve
 // uneven 1119 / 1083; six at 1280x720 1657 / 1668 (two runs differ by 10).
 static const RayVariant& overlapped_ray(const Context* ctx) {
-  return ray_variants[raycast_is_phased(ctx) ? ctx->tune.ray : N_RAY_VARIANTS - 1];
+  const RayVariant& r = ray_variants[ctx->tune.ray];
+  return r.fn ? ray_variants[N_RAY_VARIANTS - 1] : r;
 }
 
 // The phased composite in parts: the per-instance marches of `ids` into the

@@ -109,22 +109,9 @@ int autotune(Context* ctx, int reps, float* ray_us, float* int_us) {
   const int nr = ray_variant_count();
   for (int v = 0; v < nr; ++v) {
     ctx->tune.ray = v;
-    int rc = time_launches(ctx, s, reps, 3, [&] {
+    const int rc = time_launches(ctx, s, reps, 3, [&] {
       return stage_raycast_to(ctx, all, ctx->ray_epsilon, vert, norm, lab);
     }, &ray_us[v]);
-    // a frame with objects runs the phased background's marches beside the
-    // objects' tracking: what counts is the rest
-    if (!rc && raycast_is_phased(ctx) && all.n > 1 && ctx->cfg.batched &&
-        ctx->overlap_ctas != 0) {
-      IdList bg;
-      bg.n = 1;
-      bg.v[0] = 0;
-      float bg_us = 0.f;
-      rc = time_launches(ctx, s, reps, 3, [&] {
-        return stage_raycast_hits(ctx, bg, 0, ctx->ray_epsilon);
-      }, &bg_us);
-      ray_us[v] = std::max(ray_us[v] - bg_us, 0.f);
-    }
     if (rc) { ctx->tune = before; return rc; }
   }
   ctx->tune = before;

@@ -51,3 +51,23 @@ def test_setting_the_shape_in_use_changes_nothing():
         _frames(ctx, s, 5, 2)
         assert ctx.frame_stats()["graph_kernels"] == before, v
     ctx.close()
+
+
+def test_the_tuner_times_whole_raycasts():
+    """Whether frames overlap or not, the tuner's time of a raycast shape is
+    that of the whole raycast, as mf_raycast, motion frames, costs and frames
+    in order run it.  (Without the background's marches a phased shape takes
+    less than half.)"""
+    s = make_scene("multi", 640, 480, n_frames=3, seed=11, n_objects=2, bg_size=512,
+                   obj_size=128)
+    ctx = _context(s)
+    _frames(ctx, s, 0, 3)
+    us = {}
+    for overlap in (-1, 0):
+        ctx.set_overlap(overlap)
+        us[overlap] = np.array(ctx.autotune(reps=10)["raycast"]["us"])
+    phased = [v for v in range(len(us[0]))
+              if "phased" in capi.tune_describe(capi.TUNE_RAYCAST, v)]
+    # the same launches: run to run a few percent apart
+    assert np.all(us[-1][phased] > 0.75 * us[0][phased]), us
+    ctx.close()
