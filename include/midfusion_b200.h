@@ -561,7 +561,10 @@ int mf_set_overlap(mf_context* ctx, int ctas);
  *                      phased form, in the chosen phased shape or else with
  *                      8x16 tiles (same maps);
  *   MF_TUNE_INTEGRATE  the voxel-block integration (projective_functor::
- *                      update_block): 256-thread CTAs resident per SM.
+ *                      update_block): without (0..2) or with (3..5) a
+ *                      prefetch of the next block's fields.  The three numbers
+ *                      of each, which a saved choice may hold, used to be three
+ *                      residencies; they are one shape, the fastest, now.
  * Variant 0 of each is the default.  A context starts with the defaults. */
 #define MF_TUNE_RAYCAST 0
 #define MF_TUNE_INTEGRATE 1

@@ -256,6 +256,7 @@ int ray_variant_count();
 void ray_variant_describe(int v, char* buf, int cap);
 int int_variant_count();
 void int_variant_describe(int v, char* buf, int cap);
+int int_variant_first(int v);
 // integrate_blocks_kernel alone, on `pool` (the live pool or a scratch copy),
 // over the visit list of the last stage_integrate / visit_list
 int launch_integrate_blocks(Context* ctx, const Pool& pool, int variant, int ctas = 0);

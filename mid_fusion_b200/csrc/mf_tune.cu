@@ -5,8 +5,8 @@
 // the same inputs whatever the shape:
 //  - raycast_objects_kernel: the pixel tile of a 128-thread CTA and the
 //    register bound (residency) it is compiled for (ray_variants);
-//  - integrate_blocks_kernel: how many 256-thread CTAs are resident per SM,
-//    which sets both the register bound and the persistent grid (int_variants).
+//  - integrate_blocks_kernel: with or without a prefetch of the next block
+//    (int_variants).
 // autotune() times every candidate on the context's current frame with CUDA
 // events and keeps the fastest.  The map is never touched: the raycasts write
 // scratch maps and the integrations update a scratch copy of the pool slots
@@ -133,6 +133,11 @@ int autotune(Context* ctx, int reps, float* ray_us, float* int_us) {
     if (rc) return MF_E_CUDA;
     if (int e = build_visit_list(ctx, mask)) return e;
     for (int v = 0; v < ni; ++v) {
+      const int same = int_variant_first(v);
+      if (same != v) {
+        int_us[v] = int_us[same];
+        continue;
+      }
       const int e = time_launches(ctx, s, reps, 3, [&] {
         return launch_integrate_blocks(ctx, sp, v);
       }, &int_us[v]);

@@ -460,15 +460,16 @@ __device__ __forceinline__ void prefetch_fields(const Pool& pool, int slot, int 
 // 98 us, 4.0 TB/s, issue slots 55 % busy (one voxel per thread and a barrier
 // per block: 130 us, 65 %, half again as many instructions; without the barrier
 // alone 131).  Registers bound the warps in flight: 4 CTAs per SM (64
-// registers, 98 us) beat 5 (48, spills, 114) and 3 (80, 117); the prefetch
-// gains nothing here, since the loads wait for the pixels, not for DRAM.
-// Persistent: MINB 256-thread CTAs per SM (the register bound); with PF the
-// warp prefetches its quarter of the next block's fields into L2 while it
-// works on the current one.  Every variant updates each voxel alike
-// (int_variants).
+// registers) beat 5 (48, spills) by 4 to 14 % and 3 (80) by 12 to 20 % from one
+// object at 160x120 to six at 1280x720.
+// Persistent: INT_CTAS CTAs per SM; with PF the warp prefetches its quarter of
+// the next block's fields into L2 while it works on the current one (mostly no
+// gain, since the loads wait for the pixels, not for DRAM).  Both forms update
+// each voxel alike (int_variants).
 constexpr int INT_THREADS = 256;  // two blocks per CTA
-template <int MINB, bool PF>
-__global__ void __launch_bounds__(INT_THREADS, MINB)
+constexpr int INT_CTAS = 4;
+template <bool PF>
+__global__ void __launch_bounds__(INT_THREADS, INT_CTAS)
 integrate_blocks_kernel(Pool pool, const Volume* __restrict__ vols,
                         const InstFrame* __restrict__ frames, SdfArgs args, F4 k,
                         const int* __restrict__ visit, const int* __restrict__ visit_count) {
@@ -858,15 +859,20 @@ int profile_integrate(Context* ctx, int reps, double* us, double* bytes) {
 }
 
 // Launch-shape candidates of integrate_blocks_kernel; entry 0 is the default.
+// Callers keep the numbers (mf_tune_get): 0..2 have stood for three residencies
+// without the prefetch and 3..5 for the same with it.  One residency is the
+// fastest everywhere now, so each three are one shape.  Integration alone, 0 and
+// 3 (us): one object 160x120 53 / 55, 640x480 59 / 62; three at 640x480
+// 105 / 109; twelve uneven 72 / 76; six at 1280x720 157 / 169; whole frames are
+// within 1 % of each other.
 struct IntVariant {
-  int minb;
   bool prefetch;
   void (*fn)(Pool, const Volume*, const InstFrame*, SdfArgs, F4, const int*, const int*);
 };
 static const IntVariant int_variants[] = {
-    {4, false, integrate_blocks_kernel<4, false>}, {5, false, integrate_blocks_kernel<5, false>},
-    {3, false, integrate_blocks_kernel<3, false>}, {4, true, integrate_blocks_kernel<4, true>},
-    {5, true, integrate_blocks_kernel<5, true>},   {3, true, integrate_blocks_kernel<3, true>},
+    {false, integrate_blocks_kernel<false>}, {false, integrate_blocks_kernel<false>},
+    {false, integrate_blocks_kernel<false>}, {true, integrate_blocks_kernel<true>},
+    {true, integrate_blocks_kernel<true>},   {true, integrate_blocks_kernel<true>},
 };
 constexpr int N_INT_VARIANTS = (int)(sizeof(int_variants) / sizeof(int_variants[0]));
 static_assert(N_INT_VARIANTS <= MAX_TUNE_VARIANTS, "integration candidate table too long");
@@ -874,8 +880,15 @@ static_assert(N_INT_VARIANTS <= MAX_TUNE_VARIANTS, "integration candidate table 
 int int_variant_count() { return N_INT_VARIANTS; }
 
 void int_variant_describe(int v, char* buf, int cap) {
-  snprintf(buf, cap, "integrate %d x 256-thread CTAs per SM%s", int_variants[v].minb,
+  snprintf(buf, cap, "integrate %d x 256-thread CTAs per SM%s", INT_CTAS,
            int_variants[v].prefetch ? ", next block's fields prefetched to L2" : "");
+}
+
+// The first number of the same shape.
+int int_variant_first(int v) {
+  int f = 0;
+  while (int_variants[f].fn != int_variants[v].fn) ++f;
+  return f;
 }
 
 // ctas > 0: that many CTAs instead of the variant's residency times the SM
@@ -888,7 +901,7 @@ int launch_integrate_blocks(Context* ctx, const Pool& pool, int variant, int cta
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
   const IntVariant& v = int_variants[variant];
   // `ctas` counts 512 threads (mf_set_overlap)
-  const int grid = ctas > 0 ? ctas * (512 / INT_THREADS) : sms * v.minb;
+  const int grid = ctas > 0 ? ctas * (512 / INT_THREADS) : sms * INT_CTAS;
   v.fn<<<grid, INT_THREADS, 0, ctx->stream>>>(pool, ctx->d_vols, ctx->d_frames, a, k, ctx->d_visit,
                                       ctx->d_visit_count);
   MF_CUDA(cudaGetLastError());
