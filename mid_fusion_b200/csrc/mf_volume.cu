@@ -360,7 +360,7 @@ visit_list_kernel(Pool pool, const Volume* __restrict__ vols,
                   int* __restrict__ visit, int* __restrict__ visit_count, int clear) {
   const int slot = blockIdx.x * blockDim.x + threadIdx.x;
   bool take = false;
-  if (slot < *pool.count) {
+  if (slot < min(*pool.count, pool.cap)) {   // the count runs on when the pool is full
     const int4 m = pool.meta[slot];
     // a slot that the other stream's allocation has counted but not written
     // yet (w < 0) belongs to that stream's instances
