@@ -38,7 +38,7 @@ def _run(s, pool, frames=3):
 
 @pytest.mark.parametrize("pool", [1, 44, 255, 257, 300])
 def test_full_pool_keeps_to_its_slots(pool):
-    s = make_scene("room", 160, 120, n_frames=1, seed=4, bg_size=128, noise=False)
+    s = make_scene("room", 160, 120, n_frames=1, seed=4, bg_size=256, noise=False)
     keys, active, vox, status, _ = _run(s, 1 << 13)
     assert status == 0 and len(keys) > 320
     k, a, v, st, stats = _run(s, pool)
