@@ -39,7 +39,7 @@ extern "C" {
 #define MF_STATUS_RAY_GUARD 4
 #define MF_STATUS_GN_FALLBACK 8     /* a 6x6 system used the truncated eigen solve */
 #define MF_STATUS_ADJOINT 16        /* mf_camera_cost skipped the TSDF adjoint of a ray */
-#define MF_STATUS_GN_TIMEOUT 32     /* a grid barrier of the persistent GN launch gave up */
+#define MF_STATUS_GN_TIMEOUT 32     /* a barrier of a GN launch gave up (MF_E_TIMEOUT) */
 
 /* Robust kernels of Tracking::calc_robust_weight,
  * apps/kfusion/src/cpp/tracking/tracking.cpp:1504-1532 (enum RobustW,
@@ -71,7 +71,13 @@ int mf_config_default(mf_config* cfg, int width, int height);
 int mf_create(const mf_config* cfg, mf_context** out);
 int mf_destroy(mf_context* ctx);
 const char* mf_last_error(const mf_context* ctx);
-/* Pending device status flags (MF_STATUS_*), cleared by the call. */
+/* Pending device status flags (MF_STATUS_*), cleared by the call.
+ * After MF_STATUS_GN_TIMEOUT a pose is the one before its tracking.  Until this
+ * call clears the flag, the calls that read poses or tracking results
+ * (mf_get_camera_pose, mf_instance_get_pose, mf_get_poses, mf_save_poses,
+ * mf_track_info, mf_track_results with a pose, mf_motion_residuals,
+ * mf_object_residuals, mf_process_frame_motion, tracking without `batched`) and
+ * mf_synchronize return MF_E_TIMEOUT. */
 int mf_status(mf_context* ctx, int* flags);
 /* The cudaStream_t all work is queued on. */
 int mf_get_stream(mf_context* ctx, void** stream);
@@ -242,6 +248,11 @@ int mf_camera_cost(mf_context* ctx, const float T_live[16], double* out, float* 
  * Allocates and synchronises. */
 int mf_debug_gn_step(mf_context* ctx, int n, const double* state, const double* sums,
                      double* out_device, double* out_host);
+/* Diagnostic, no reference counterpart: polls after which a GN launch gives up
+ * waiting for its own CTAs (2^21 in a new context: about a second).  With 0 a
+ * CTA gives up unless it arrives last.  Applies to frames captured after the
+ * call. */
+int mf_debug_gn_wait(mf_context* ctx, unsigned polls);
 
 /* --- motion segmentation ------------------------------------------------
  * Tracking::compute_residuals (tracking/tracking.cpp:1535-1747) with the

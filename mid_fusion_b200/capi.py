@@ -35,7 +35,7 @@ EXPORTS = [
     "mf_track_info", "mf_track_eval", "mf_download_pyramid", "mf_process_frame",
     "mf_process_frame_device", "mf_get_poses", "mf_frame_stats", "mf_set_graphs",
     "mf_profile", "mf_track_eval_static", "mf_camera_cost", "mf_pool_tsdf", "mf_pool_slots",
-    "mf_debug_gn_step", "mf_set_overlap",
+    "mf_debug_gn_step", "mf_debug_gn_wait", "mf_set_overlap",
     "mf_motion_residuals", "mf_motion_download", "mf_track_results",
     "mf_refine_mask_use_motion", "mf_download_mask", "mf_retrack_camera",
     "mf_render_volume", "mf_render_depth", "mf_render_intensity", "mf_render_normal",
@@ -285,6 +285,9 @@ class Context:
         f = C.c_int()
         self._check(self.lib.mf_status(self.h, C.byref(f)))
         return f.value
+
+    def debug_gn_wait(self, polls):
+        self._check(self.lib.mf_debug_gn_wait(self.h, C.c_uint(polls)))
 
     def synchronize(self):
         self._check(self.lib.mf_synchronize(self.h))

@@ -154,6 +154,7 @@ int mf_create(const mf_config* cfg, mf_context** out) {
        cudaMalloc(&ctx->d_Twc, sizeof(float) * 16) == cudaSuccess &&
        cudaMalloc(&ctx->d_frames, sizeof(InstFrame) * MAX_INSTANCES) == cudaSuccess &&
        cudaMalloc(&ctx->d_status, sizeof(int)) == cudaSuccess &&
+       cudaMallocHost(&ctx->gn_timeout, sizeof(int)) == cudaSuccess &&
        cudaMalloc(&ctx->d_reserved, sizeof(unsigned long long) * MAX_INSTANCES) == cudaSuccess &&
        cudaMalloc(&ctx->d_inst_label, sizeof(int) * MAX_INSTANCES) == cudaSuccess &&
        cudaMalloc(&ctx->d_visit, sizeof(int) * cap) == cudaSuccess &&
@@ -192,6 +193,7 @@ int mf_create(const mf_config* cfg, mf_context** out) {
   cudaMemsetAsync(P.active, 0, cap, ctx->stream);
   cudaMemsetAsync(P.count, 0, sizeof(int), ctx->stream);
   cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream);
+  *ctx->gn_timeout = 0;
   cudaMemsetAsync(ctx->d_vertex, 0, sizeof(F3) * WH, ctx->stream);
   cudaMemsetAsync(ctx->d_normal, 0, sizeof(F3) * WH, ctx->stream);
   cudaMemsetAsync(ctx->d_label, 0, sizeof(int) * WH, ctx->stream);
@@ -231,6 +233,7 @@ int mf_destroy(mf_context* ctx) {
                 ctx->d_render, ctx->d_render_small, ctx->d_rayhit, ctx->d_raytf,
                 ctx->d_mc_tris, ctx->d_mesh};
   for (void* p : ps) if (p) cudaFree(p);
+  if (ctx->gn_timeout) cudaFreeHost(ctx->gn_timeout);
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->side) cudaStreamDestroy(ctx->side);
   if (ctx->ev_start) cudaEventDestroy(ctx->ev_start);
@@ -249,6 +252,7 @@ int mf_status(mf_context* ctx, int* flags) {
   MF_CUDA(cudaMemcpyAsync(&v, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   MF_CUDA(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
   MF_CUDA(cudaStreamSynchronize(ctx->stream));
+  *ctx->gn_timeout = 0;
   *flags = v;
   return MF_OK;
 }
@@ -262,7 +266,7 @@ int mf_get_stream(mf_context* ctx, void** stream) {
 int mf_synchronize(mf_context* ctx) {
   if (check(ctx)) return MF_E_ARG;
   MF_CUDA(cudaStreamSynchronize(ctx->stream));
-  return MF_OK;
+  return track_waited(ctx);
 }
 
 int mf_instance_add(mf_context* ctx, int size, float dim, const float T_w_o[16], int label,
@@ -319,7 +323,7 @@ int mf_instance_get_pose(mf_context* ctx, int id, float T[16]) {
   if (id < 0 || id >= (int)ctx->inst.size()) return MF_E_NOT_FOUND;
   MF_CUDA(cudaMemcpyAsync(T, ctx->d_Two + 16 * id, 64, cudaMemcpyDeviceToHost, ctx->stream));
   MF_CUDA(cudaStreamSynchronize(ctx->stream));
-  return MF_OK;
+  return track_waited(ctx);
 }
 
 int mf_set_camera_pose(mf_context* ctx, const float T[16]) {
@@ -335,7 +339,7 @@ int mf_get_camera_pose(mf_context* ctx, float T[16]) {
   if (check(ctx) || !T) return MF_E_ARG;
   MF_CUDA(cudaMemcpyAsync(T, ctx->d_Twc, 64, cudaMemcpyDeviceToHost, ctx->stream));
   MF_CUDA(cudaStreamSynchronize(ctx->stream));
-  return MF_OK;
+  return track_waited(ctx);
 }
 
 int mf_frame_upload(mf_context* ctx, const float* depth, const uint8_t* rgb,
@@ -621,7 +625,7 @@ int mf_get_poses(mf_context* ctx, float* T_w_c, float* T_w_o) {
     MF_CUDA(cudaMemcpyAsync(T_w_o, ctx->d_Two, 64 * ctx->inst.size(), cudaMemcpyDeviceToHost,
                             ctx->stream));
   MF_CUDA(cudaStreamSynchronize(ctx->stream));
-  return MF_OK;
+  return track_waited(ctx);
 }
 
 int mf_frame_stats(mf_context* ctx, long long* out, int n) {
@@ -774,6 +778,15 @@ int mf_debug_gn_step(mf_context* ctx, int n, const double* state, const double* 
     return MF_E_ARG;
   if (n == 0) return MF_OK;
   return gn_step_check(ctx, n, state, sums, out_device, out_host);
+}
+
+int mf_debug_gn_wait(mf_context* ctx, unsigned polls) {
+  if (check(ctx)) return MF_E_ARG;
+  if (ctx->gn_polls != polls) {
+    ctx->gn_polls = polls;
+    ++ctx->tune.gen;  // captured frame graphs are rebuilt
+  }
+  return MF_OK;
 }
 
 int mf_camera_cost(mf_context* ctx, const float* T_live, double* out, float* d_grad_tsdf) {
@@ -951,6 +964,7 @@ int mf_save_poses(mf_context* ctx, const char* prefix, int frame) {
     MF_CUDA(cudaMemcpyAsync(T.data() + 16, ctx->d_Two, 64 * (size_t)n, cudaMemcpyDeviceToHost,
                             ctx->stream));
   MF_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (int rc = track_waited(ctx)) return rc;
   for (int i = 0; i < n; ++i) {
     Instance& in = ctx->inst[i];
     const bool cam = in.label == 0;

@@ -81,6 +81,8 @@ struct Context {
   float* d_Twc = nullptr;           // 16, camera pose
   InstFrame* d_frames = nullptr;    // MAX_INSTANCES
   int* d_status = nullptr;          // OR of Status flags
+  int* gn_timeout = nullptr;        // pinned host word, set by a GN launch that gave up waiting
+  unsigned gn_polls = 1u << 21;     // polls of a GN launch's wait before it gives up (1 s)
   unsigned long long* d_reserved = nullptr;  // MAX_INSTANCES reference list capacities
   int* d_inst_label = nullptr;      // MAX_INSTANCES instance labels
   int* d_scratch_i = nullptr;       // small device scratch (export slot lists)
@@ -184,6 +186,9 @@ void track_free(Context* ctx);
 // which writes them whole
 int track_preprocess(Context* ctx, bool clear_mask = true);
 int track_set_ref(Context* ctx);
+// After a synchronisation: MF_E_TIMEOUT if a GN launch since the last mf_status
+// gave up waiting for its own CTAs (its poses are not written then).
+int track_waited(Context* ctx);
 int track_camera(Context* ctx, uint32_t moving, int retrack = 0);
 int track_objects(Context* ctx, const IdList& ids);
 // the same in phases, for a frame that runs the pose-independent parts on

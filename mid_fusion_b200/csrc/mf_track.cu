@@ -1472,7 +1472,9 @@ struct GNLoop {
   uint8_t* lives;    // objects: the tiles with a sum, 2 x slots x max_tiles
   unsigned* bar;     // barrier arrivals by problem slot
   int slots;         // problem slots (the context's instance capacity)
+  unsigned polls;    // of a wait before it gives up
   int* status;
+  int* timeout;      // Context::gn_timeout
   float* poses;      // camera: T_w_c; objects: the volume poses
 };
 
@@ -1556,13 +1558,15 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   return v;
 }
 
-// Waits until `target` CTAs have arrived at `bar`.  Bounded: after GN_BAR_SPINS
-// polls it sets MF_STATUS_GN_TIMEOUT and returns 1, and the CTA returns.
-constexpr unsigned GN_BAR_SPINS = 1u << 21;   // polls, 32 ns apart after the first 64: about 1 s
-__device__ __forceinline__ int gn_wait(const unsigned* bar, unsigned target, int* status) {
+// Waits until `target` CTAs have arrived at `bar`.  Bounded: after `polls` polls
+// (32 ns apart after the first 64: about 1 s) it sets MF_STATUS_GN_TIMEOUT and
+// the host's word, which calls that read poses look at, and returns 1; the CTA
+// returns then.
+__device__ __forceinline__ int gn_wait(const unsigned* bar, unsigned target, const GNLoop& g) {
   for (unsigned spins = 0; ld_acquire_u32(bar) < target; ++spins) {
-    if (spins >= GN_BAR_SPINS) {
-      atomicOr(status, MF_STATUS_GN_TIMEOUT);
+    if (spins >= g.polls) {
+      atomicOr(g.status, MF_STATUS_GN_TIMEOUT);
+      *(volatile int*)g.timeout = 1;
       return 1;
     }
     if (spins > 64) __nanosleep(32);
@@ -1619,7 +1623,7 @@ gn_camera_kernel(GNArgs a, GNLoop g) {
         if (lane == 0) {
           atomicAdd(g.bar, 1u);
           target += gridDim.x;
-          sm.flag = gn_wait(g.bar, target, g.status);
+          sm.flag = gn_wait(g.bar, target, g);
         }
       }
       __syncthreads();
@@ -1924,7 +1928,7 @@ gn_objects_kernel(GNArgs a, GNLoop g, IdList slots, const float* __restrict__ Tw
           __threadfence();
           atomicAdd(bar, 1u);
           target += size;
-          sm.flag = gn_wait(bar, target, g.status);
+          sm.flag = gn_wait(bar, target, g);
         }
         __syncthreads();
         if (sm.flag) return;
@@ -2278,6 +2282,12 @@ static int tile_depth_range(Context* ctx) {
   return MF_OK;
 }
 
+int track_waited(Context* ctx) {
+  if (!*(volatile int*)ctx->gn_timeout) return MF_OK;
+  ctx->last_error = "a Gauss-Newton launch gave up waiting for its CTAs (mf_status clears this)";
+  return MF_E_TIMEOUT;
+}
+
 // The camera's GN launch: the whole loop, or with `only` >= 0 one evaluation
 // of that level whose sums land in the problem's state (plain mode).
 static int launch_gn_camera(Context* ctx, const GNArgs& a, int only) {
@@ -2287,7 +2297,9 @@ static int launch_gn_camera(Context* ctx, const GNArgs& a, int only) {
   g.only = only;
   g.rows = T.d_gnrows;
   g.bar = T.d_gnbar;
+  g.polls = ctx->gn_polls;
   g.status = ctx->d_status;
+  g.timeout = ctx->gn_timeout;
   g.poses = ctx->d_Twc;
   int rows = 1;
   for (int L = 0; L < T.levels; ++L) {
@@ -2328,7 +2340,9 @@ static int launch_gn_objects(Context* ctx, const GNArgs& a, const IdList& slots,
   g.lives = T.d_objlive;
   g.slots = ctx->cfg.max_instances;
   g.bar = T.d_gnbar;
+  g.polls = ctx->gn_polls;
   g.status = ctx->d_status;
+  g.timeout = ctx->gn_timeout;
   g.poses = ctx->d_Two;
   for (int L = 0; L < T.levels; ++L) g.iters[L] = ctx->cfg.gn_iterations[L];
   const int ctas = std::min(T.obj_blocks, GO_CTAS * slots.n);
@@ -2379,6 +2393,7 @@ static int gn_host(Context* ctx, int slot) {
       MF_CUDA(cudaMemcpyAsync(S.sums[L], sums_ptr(T, slot, L), sizeof(double) * 32,
                               cudaMemcpyDeviceToHost, ctx->stream));
       MF_CUDA(cudaStreamSynchronize(ctx->stream));
+      if (int rc = track_waited(ctx)) return rc;
       gn_step(S, S.sums[L], L);
     }
   }
@@ -2492,6 +2507,7 @@ int track_info(Context* ctx, int slot, int* iters, double* sums, double* T64) {
   MF_CUDA(cudaMemcpyAsync(&S, ctx->track->d_state + slot, sizeof(GNState),
                           cudaMemcpyDeviceToHost, ctx->stream));
   MF_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (int rc = track_waited(ctx)) return rc;
   for (int l = 0; l < MAX_PYR; ++l) {
     if (iters) iters[l] = S.iters[l];
     if (sums) for (int i = 0; i < 32; ++i) sums[32 * l + i] = S.sums[l][i];
@@ -3292,6 +3308,7 @@ int motion_residuals(Context* ctx, float threshold, float moved, float* ratio,
   MF_CUDA(cudaMemcpyAsync(Tr, T.d_Twc_prev, 64, cudaMemcpyDeviceToHost, ctx->stream));
   MF_CUDA(cudaMemsetAsync(T.d_mcount, 0, sizeof(int) * 64, ctx->stream));
   MF_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (int rc = track_waited(ctx)) return rc;
   const mf_config& c = ctx->cfg;
   const F4 k{c.k[0], c.k[1], c.k[2], c.k[3]};
   MotionArgs a;
@@ -3359,6 +3376,7 @@ int object_residuals(Context* ctx, int i, float threshold, int8_t* d_rows, float
   float Tr[16];
   MF_CUDA(cudaMemcpyAsync(Tr, T->d_Twc_prev, 64, cudaMemcpyDeviceToHost, ctx->stream));
   MF_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (int rc = track_waited(ctx)) return rc;
   const mf_config& c = ctx->cfg;
   const F4 k{c.k[0], c.k[1], c.k[2], c.k[3]};
   MotionArgs a;
@@ -3472,6 +3490,7 @@ int track_results(Context* ctx, int slot, int8_t* d_out, float* d_err, float* po
     MF_CUDA(cudaMemcpyAsync(pose_eval, &ctx->track->d_state[slot].evalTf, sizeof(M4),
                             cudaMemcpyDeviceToHost, ctx->stream));
     MF_CUDA(cudaStreamSynchronize(ctx->stream));
+    return track_waited(ctx);
   }
   return MF_OK;
 }
