@@ -187,16 +187,13 @@ def run_ours(args, rank, world, local_rank):
     # device-resident inputs
     d_depth, d_rgb, d_lab = to_device(frames)
 
-    def run(batched, record_poses=True, scene=None, inputs=None, tune=None, persistent=None,
-            overlap=None):
+    def run(batched, record_poses=True, scene=None, inputs=None, tune=None, overlap=None):
         """Frames through mf_process_frame_device; device time per frame after
         1 + warmup untimed frames.  tune="auto": mf_autotune on the last
         warm-up frame (outside the timed region; its report lands in
         tuned[id(ctx)]); a dict {stage: variant}: those launch shapes from the
         start."""
         ctx = make_ctx(batched, scene)
-        if persistent is not None:
-            ctx.set_gn_persistent(persistent)
         if overlap is not None:
             ctx.set_overlap(overlap)
         if isinstance(tune, dict):
@@ -241,8 +238,10 @@ def run_ours(args, rank, world, local_rank):
         import ctypes
         Tc = np.zeros(16, np.float32)
         To = np.zeros(16 * ctx.n_instances, np.float32)
-        ctx.lib.mf_get_poses(ctx.h, Tc.ctypes.data_as(ctypes.c_void_p),
-                             To.ctypes.data_as(ctypes.c_void_p))
+        rc = ctx.lib.mf_get_poses(ctx.h, Tc.ctypes.data_as(ctypes.c_void_p),
+                                  To.ctypes.data_as(ctypes.c_void_p))
+        if rc != 0:
+            raise RuntimeError(f"mf_get_poses failed: {rc}")
         return Tc.reshape(4, 4), To.reshape(-1, 4, 4)
 
     def shapes(ctx):
@@ -266,20 +265,11 @@ def run_ours(args, rank, world, local_rank):
                     status=(st_b, 0), clocks=sampler.summary(), h2d=0, d2h=0,
                     ms_b=1e3 * total_b / max(len(t_b), 1), stats=stats, prof=prof, n_inst=len(s.instances),
                     tune=tuned.get(id(ctx_b)))
-    # ---- the batched GN as one cooperative launch per pyramid level instead
-    # of one launch per iteration (same poses bit for bit)
+    # ---- the background's integration in order instead of overlapped with
+    # object tracking (mf_set_overlap(ctx, 0); same poses bit for bit)
     gn_modes = None
     if world == 1 and not args.profile:
-        ctx_q, t_q, poses_q, st_q = run(True, tune=tune_b, persistent=True)
-        same = all(np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
-                   for a, b in zip(poses_b, poses_q))
-        gn_modes = {"default": {"ms_per_step": round(1e3 * total_b / len(t_b), 4)},
-                    "set_gn_persistent": {"ms_per_step": round(1e3 * sum(t_q) / len(t_q), 4),
-                                             "status_flags": st_q},
-                    "same_poses": bool(same)}
-        ctx_q.close()
-        # the background's integration in order instead of overlapped with
-        # object tracking (mf_set_overlap(ctx, 0))
+        gn_modes = {"default": {"ms_per_step": round(1e3 * total_b / len(t_b), 4)}}
         ctx_o, t_o, poses_o, st_o = run(True, tune=tune_b, overlap=0)
         same = all(np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
                    for a, b in zip(poses_b, poses_o))
@@ -304,9 +294,6 @@ def run_ours(args, rank, world, local_rank):
         su = scene_for(rank, n_uneven, "uneven")
         ins = to_device(rendered["uneven"])
         cub, tub, pub, stub = run(True, scene=su, inputs=ins, tune=auto)
-        cuq, tuq, puq, stuq = run(True, scene=su, inputs=ins, tune=shapes(cub), persistent=True,
-                                  record_poses=False)
-        cuq.close()
         cup, tup, pup, stup = run(False, scene=su, inputs=ins, tune=shapes(cub))
         du = 0.0
         for (cb, ob), (cp, op) in zip(pub, pup):
@@ -318,7 +305,6 @@ def run_ours(args, rank, world, local_rank):
                   "ms_batched": round(1e3 * ub / len(tub), 4),
                   "ms_plain": round(1e3 * up / len(tup), 4),
                   "batched_over_plain": round(up / ub, 3), "pose_diff_batched_vs_plain_m": du,
-                  "ms_batched_persistent_gn": round(1e3 * sum(tuq) / len(tuq), 4),
                   "autotune": tuned.get(id(cub)), "status_flags": [stub, stup]}
         for c in (cub, cup):
             c.close()

@@ -546,7 +546,7 @@ int mf_set_graphs(mf_context* ctx, int enable);
 /* No counterpart in the reference.  Kept for callers: it used to choose
  * between one launch per GN iteration (0) and one per pyramid level (1).
  * Batched GN is now one launch for all levels and iterations of a stage in
- * either setting, with the same poses bit for bit. */
+ * either setting, with the same poses bit for bit; the call does nothing. */
 int mf_set_gn_persistent(mf_context* ctx, int enable);
 /* No counterpart in the reference.  Batched frames with objects: the
  * background's allocation and integration (which need only the camera pose)

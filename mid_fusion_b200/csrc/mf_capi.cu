@@ -664,14 +664,7 @@ int mf_set_graphs(mf_context* ctx, int enable) {
   return MF_OK;
 }
 
-int mf_set_gn_persistent(mf_context* ctx, int enable) {
-  if (check(ctx)) return MF_E_ARG;
-  if (ctx->gn_persistent != (enable != 0)) {
-    ctx->gn_persistent = enable != 0;
-    ++ctx->tune.gen;  // captured frame graphs are rebuilt
-  }
-  return MF_OK;
-}
+int mf_set_gn_persistent(mf_context* ctx, int) { return check(ctx) ? MF_E_ARG : MF_OK; }
 
 int mf_set_overlap(mf_context* ctx, int ctas) {
   if (check(ctx) || ctas > 65535) return MF_E_ARG;

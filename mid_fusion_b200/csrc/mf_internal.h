@@ -121,7 +121,6 @@ struct Context {
   float ray_epsilon = 0.f;          // ray iterator direction epsilon (first volume)
   void* graphs = nullptr;           // captured frame graphs (mf_pipeline.cu)
   bool use_graphs = true;
-  bool gn_persistent = false;       // mf_set_gn_persistent's last argument (selects nothing)
   // batched frames: the background's allocation and integration run on a
   // low-priority side stream while the objects are tracked (overlap_ctas:
   // CTAs of that integration launch, < 0 the launch shape's own grid;
