@@ -2483,9 +2483,6 @@ int track_eval(Context* ctx, int slot, int L, const float* pose16, double* sums)
   S.ticket = 0;
   MF_CUDA(cudaMemcpyAsync(T.d_state + slot, &S, sizeof(GNState), cudaMemcpyHostToDevice,
                           ctx->stream));
-  IdList one;
-  one.n = 1;
-  one.v[0] = slot;
   const GNArgs a = make_args(ctx);
   const int tiles = div_up((long long)T.pyr.w[L] * T.pyr.h[L], GN_THREADS * gn_pix(L));
   if (S.kind == 1)
@@ -2507,9 +2504,6 @@ int track_eval(Context* ctx, int slot, int L, const float* pose16, double* sums)
 int profile_gn(Context* ctx, int reps, double* us, double* bytes) {
   if (!ctx->track) return MF_E_STATE;
   TrackState& T = *ctx->track;
-  IdList one;
-  one.n = 1;
-  one.v[0] = 0;
   GNState S;
   MF_CUDA(cudaMemcpyAsync(&S, T.d_state, sizeof(GNState), cudaMemcpyDeviceToHost, ctx->stream));
   MF_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -2517,7 +2511,6 @@ int profile_gn(Context* ctx, int reps, double* us, double* bytes) {
   S.ticket = 0;
   MF_CUDA(cudaMemcpyAsync(T.d_state, &S, sizeof(GNState), cudaMemcpyHostToDevice, ctx->stream));
   const GNArgs a = make_args(ctx);
-  const int tiles = div_up((long long)T.pyr.w[0] * T.pyr.h[0], GN_THREADS * gn_pix(0));
   auto launch = [&]() -> int {
     MF_CUDA(cudaMemsetAsync(T.d_gnbar, 0, sizeof(unsigned), ctx->stream));
     return launch_gn_camera(ctx, a, 0);
