@@ -226,7 +226,7 @@ def run_ours(args, rank, world, local_rank):
             if record_poses:
                 poses.append(ctx_poses(ctx))
         st = ctx.status()
-        if batched and scene is None:
+        if batched and scene is None and not stats:   # the timed region's own run
             stats.update(ctx.frame_stats())
         return ctx, times, poses, st
 
@@ -264,7 +264,8 @@ def run_ours(args, rank, world, local_rank):
         return dict(total_b=total_b, total_p=total_b, total_e=total_b, dpos=0.0, gt_err=0.0,
                     status=(st_b, 0), clocks=sampler.summary(), h2d=0, d2h=0,
                     ms_b=1e3 * total_b / max(len(t_b), 1), stats=stats, prof=prof, n_inst=len(s.instances),
-                    tune=tuned.get(id(ctx_b)))
+                    tune=tuned.get(id(ctx_b)),
+                    ray_shape=capi.tune_describe(capi.TUNE_RAYCAST, tune_b[capi.TUNE_RAYCAST]))
     # ---- the background's integration in order instead of overlapped with
     # object tracking (mf_set_overlap(ctx, 0); same poses bit for bit)
     gn_modes = None
@@ -488,7 +489,8 @@ def run_ours(args, rank, world, local_rank):
                 ms_b=1e3 * total_b / max(len(t_b), 1), stats=stats, prof=prof, cpu=cpu,
                 pose_check=pose_check,
                 n_inst=len(s.instances), uneven=uneven, adjoint=adjoint, motion=motion, room=room,
-                tune=tuned.get(id(ctx_b)), gn_modes=gn_modes)
+                tune=tuned.get(id(ctx_b)), gn_modes=gn_modes,
+                ray_shape=capi.tune_describe(capi.TUNE_RAYCAST, tune_b[capi.TUNE_RAYCAST]))
 
 
 def run_motion(ctx, frames, poses, n, dev, torch):
@@ -849,6 +851,9 @@ def main():
                 "traffic": traffic_from_profiles("gn_camera_kernel_640x480.md")}
     ai = gbs(prof["integrate_bytes"], prof["integrate_us"])
     ar = gbs(prof["raycast_bytes"], prof["raycast_us"])
+    # the raycast in the context's shape
+    ray, ray_file = (("raycast_hits_kernel + raycast_fold_kernel", "raycast_hits_kernel")
+                     if "phased" in r["ray_shape"] else ("raycast_objects_kernel",) * 2)
     others = {
         "integrate_blocks_kernel": {"achieved": round(ai, 1), "unit": "GB/s",
                                     "frac": round(ai / hbm, 4),
@@ -856,11 +861,11 @@ def main():
                                     "algorithmic_bytes_per_launch": int(prof["integrate_bytes"]),
                                     "traffic": traffic_from_profiles(
                                         "integrate_blocks_kernel_640x480.md")},
-        "raycast (raycast_hits_kernel + raycast_fold_kernel)": {
+        f"raycast ({ray})": {
             "achieved": round(ar, 1), "unit": "GB/s", "frac": round(ar / hbm, 4),
             "us_per_launch": round(prof["raycast_us"], 2),
             "algorithmic_bytes_per_launch": int(prof["raycast_bytes"]),
-            "traffic": traffic_from_profiles("raycast_hits_kernel_640x480.md")},
+            "traffic": traffic_from_profiles(ray_file + "_640x480.md")},
     }
     per_frame = (r["stats"] or {}).get("graph_kernels", 0) + 1  # graph + rgb conversion
     launches = per_frame * args.steps
