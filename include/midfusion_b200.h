@@ -72,8 +72,9 @@ int mf_create(const mf_config* cfg, mf_context** out);
 int mf_destroy(mf_context* ctx);
 const char* mf_last_error(const mf_context* ctx);
 /* Pending device status flags (MF_STATUS_*), cleared by the call.
- * After MF_STATUS_GN_TIMEOUT a pose is the one before its tracking.  Until this
- * call clears the flag, the calls that read poses or tracking results
+ * After MF_STATUS_GN_TIMEOUT a pose is the one before its tracking, and what the
+ * same mf_process_frame* call integrated and raycast used it.  Until this call
+ * clears the flag, the calls that read poses or tracking results
  * (mf_get_camera_pose, mf_instance_get_pose, mf_get_poses, mf_save_poses,
  * mf_track_info, mf_track_results with a pose, mf_motion_residuals,
  * mf_object_residuals, mf_process_frame_motion, tracking without `batched`) and
